@@ -53,7 +53,7 @@ __global__ void publish_queue_kernel(SegQueue* q, int count, const int* count_de
 }
 
 struct Plan {
-  int bq = 128, S = 1;
+  int bq = 64, S = 1;
   std::vector<SegItem> items;
   uint64_t hash = 0;
 };
@@ -281,17 +281,14 @@ mann_status knn_graph_batched_device(Context* ctx, cudaStream_t s, const mann_kn
   Bufs b;
   if (tuned == st.tuned.end()) {
     // measure every candidate once on this call's data (each run writes the
-    // full result): tile heights (64-row tiles for k+1 > 32) x point splits
-    static const int cand32[][2] = {{128, 1}, {64, 1}, {128, 2}, {64, 2}, {128, 4}};
-    static const int cand64[][2] = {{64, 1}, {32, 1}, {64, 2}, {64, 4}};
-    const int ncand = sh.kk > 32 ? 4 : 5;
+    // full result): tile heights x point splits
+    static const int cand[][2] = {{64, 1}, {32, 1}, {64, 2}, {64, 4}};
     float best = 1e30f;
-    std::pair<int, int> pick{sh.kk > 32 ? 64 : 128, 1};
+    std::pair<int, int> pick{64, 1};
     cudaEvent_t e0, e1;
     MANN_CUDA_TRY(cudaEventCreate(&e0));
     MANN_CUDA_TRY(cudaEventCreate(&e1));
-    for (int ci = 0; ci < ncand; ++ci) {
-      const int* c = sh.kk > 32 ? cand64[ci] : cand32[ci];
+    for (const int(&c)[2] : cand) {
       make_plan(offs, nsets, c[0], c[1], &pl);
       MANN_TRY(prepare(ctx, s, sh, offs, pl, &b, st));
       cudaEventRecord(e0, s);

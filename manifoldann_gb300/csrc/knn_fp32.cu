@@ -2,14 +2,13 @@
 //
 // Replaces the per-query scan of src/indices/bruteforce.jl:59-65 (one
 // Distances.jl evaluation per point, then partialsortperm) and the batch loop
-// of src/ann_index.jl:91-98.  One CTA owns BQ queries and a contiguous split
-// of the points; it walks the split in tiles of 128 points, computes the
-// BQ x 128 distance tile in registers (difference form, one fused
-// multiply-add per dimension in order 0..d-1 -- bit-identical to the oracle's
-// sequential sum), stages it in shared memory and folds it into per-row
-// sorted top-k lists that live in the registers of the warp owning the row.
-// Splits are merged by a second kernel.  Order: (distance, id) as
-// partialsortperm (bruteforce.jl:65).
+// of src/ann_index.jl:91-98.  A CTA owns a block of queries and walks tiles of
+// 128 points: it computes the tile's distances in registers (difference form,
+// one fused multiply-add per dimension in order 0..d-1 -- bit-identical to the
+// oracle's sequential sum) and folds those below a row's k-th best into the
+// row's sorted top-k list in shared memory.  The (query block, tile) units are
+// shared out evenly over the CTAs; a row's partial lists are merged by a
+// second kernel.  Order: (distance, id) as partialsortperm (bruteforce.jl:65).
 #include <algorithm>
 
 #include "kernels.cuh"
@@ -23,6 +22,8 @@ namespace {
 constexpr int K1_THREADS = 256;
 constexpr int K1_BN = 128;  // points per tile
 constexpr int K1_DK = 16;   // dimensions per shared-memory stage
+constexpr int K1_QCAP = 32;  // candidates a row's queue holds
+constexpr int K1_DRAIN = 8;  // ... and the number at which it is merged into the row's list
 constexpr unsigned FULL = 0xFFFFFFFFu;
 using wl::list_get;
 using wl::list_insert;
@@ -157,35 +158,151 @@ struct StageLoader {
   }
 };
 
+// Shared-memory footprint of one CTA of the tile kernels: the sorted list of
+// every row, its queue of admitted candidates and their count, the row's
+// threshold (two words for Euclidean), and the two staged slices.
+template <int BQ, int KW>
+__host__ __device__ constexpr size_t k1_smem_bytes() {
+  return sizeof(uint64_t) * BQ * (32 * KW + K1_QCAP) + sizeof(uint32_t) * 4 * BQ +
+         sizeof(float) * 2 * K1_DK * ((BQ + 4) + (K1_BN + 4));
+}
+
+// CTAs per SM that the tile kernels are compiled for.  The tile phase is
+// bound by the FP32 pipe and the fold by latency, so a second and third CTA
+// fill the pipe while one folds: three where the lists leave room (k <= 32), else two.
+template <int BQ, int KW>
+__host__ __device__ constexpr int k1_ctas() {
+  return KW == 1 ? 3 : 2;
+}
+
+// v[j] for a lane-varying j in [0, N), N a power of two: a select tree on the bits of j
+template <int N>
+__device__ __forceinline__ float select_tree(const float (&v)[N], int j) {
+  float t[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) t[i] = v[i];
+#pragma unroll
+  for (int w = N / 2, bit = 1; w >= 1; w >>= 1, bit <<= 1) {
+#pragma unroll
+    for (int i = 0; i < w; ++i) t[i] = (j & bit) ? t[2 * i + 1] : t[2 * i];
+  }
+  return t[0];
+}
+
+// One compare-exchange stage of a warp bitonic network (lane holds one key).
+__device__ __forceinline__ uint64_t cmpex(uint64_t v, int j, bool keep_min) {
+  const uint64_t o = __shfl_xor_sync(FULL, (unsigned long long)v, j);
+  return keep_min == (o < v) ? o : v;
+}
+
+// The cnt <= 32 queued candidates of a row into its sorted list of 32 KW
+// entries.  KW = 1: the candidates are sorted across the lanes (16-wide when
+// that holds them) and merged in one bitonic step -- reverse, lane-wise
+// minimum, five half-cleaners -- whatever their number; longer lists take
+// them one by one.
+template <int KW>
+__device__ __forceinline__ void k1_drain_row(uint64_t* __restrict__ list, const uint64_t* __restrict__ queue, int cnt,
+                                             int k, int lane, uint64_t& kth) {
+  uint64_t c = lane < cnt ? queue[lane] : KEY_NONE;
+  if constexpr (KW == 1) {
+    uint64_t L = list[lane];
+#pragma unroll
+    for (int w = 2; w <= 16; w <<= 1)
+#pragma unroll
+      for (int j = w >> 1; j > 0; j >>= 1) c = cmpex(c, j, ((lane & j) == 0) == ((lane & w) == 0));
+    if (cnt > 16) {  // the halves are sorted up and down: merge them
+#pragma unroll
+      for (int j = 16; j > 0; j >>= 1) c = cmpex(c, j, (lane & j) == 0);
+    }
+    const uint64_t r = __shfl_sync(FULL, (unsigned long long)c, 31 - lane);
+    L = r < L ? r : L;
+#pragma unroll
+    for (int j = 16; j > 0; j >>= 1) L = cmpex(L, j, (lane & j) == 0);
+    list[lane] = L;
+    kth = __shfl_sync(FULL, (unsigned long long)L, k - 1);
+  } else {
+    uint64_t L[KW];
+#pragma unroll
+    for (int s = 0; s < KW; ++s) L[s] = list[s * 32 + lane];
+    uint64_t thr = list_get<KW>(L, k - 1);
+    for (int e = 0; e < cnt; ++e) {
+      const uint64_t cnd = __shfl_sync(FULL, (unsigned long long)c, e);
+      if (cnd < thr) {
+        list_insert<KW>(L, cnd, lane);
+        thr = list_get<KW>(L, k - 1);
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < KW; ++s) list[s * 32 + lane] = L[s];
+    kth = thr;
+  }
+}
+
 // One CTA's work: queries [q0, min(q0 + BQ, nq)) against points [nb0, nb1);
 // the sorted list of query row gq goes to dst + gq * dst_stride.
+//
+// Tile phase: BQ x 128 distances in registers, TQ x 8 per thread, bound by
+// the FP32 pipe (one sub and one fma per dimension and pair, two pairs per
+// f32x2 instruction).  The global loads of the next 16-dimension slice -- of
+// the next tile after a tile's last -- are in flight during the current one.
+//
+// Fold: distances are never staged.  Every distance is compared in its
+// register with the row's k-th best so far (as raw bits: distances are not
+// negative, and NaN sorts last); the few that pass go to the row's queue in
+// shared memory, and the warp that owns the row merges the queue into the
+// row's list once it holds K1_DRAIN candidates.  A queue that runs full ends
+// the round: its rows are merged, and the candidates left are tested again.
+// Points come in ascending id order, so in a tile's first round a distance
+// equal to the k-th belongs to a later id and is refused (strict test; the
+// threshold holds earlier tiles only); later rounds of the tile admit equals
+// and the merge orders them by id.
+//
+// Measured on one GB300 against the former kernel (128-row tiles, one CTA per
+// SM, distances staged in shared memory, one warp-wide insertion per
+// candidate, a grid of whole query blocks): 1,000 x 10,000 x 64, k = 10:
+// 291 -> 133 us; self graph of 20,011 x 100, k = 15: 7.69 -> 3.23 ms (25 of
+// the 40 T lane-operations/s of the FP32 pipe); 10,000 x 60,000 x 784:
+// 55.1 -> 31.9 ms (29.5 T); graphs of 24 clouds, 32 dimensions, k = 15:
+// 29.4 -> 22.7 ms (26 T).
 template <int METRIC, int BQ, int KW, bool VEC>
 __device__ __forceinline__ void k1_body(const float* __restrict__ base, int64_t nb0, int64_t nb1,
                                         const float* __restrict__ qs, const int32_t* __restrict__ qrows,
                                         int64_t q0, int64_t nq, int d, const float* __restrict__ qnorm,
                                         const float* __restrict__ bnorm, int k, uint64_t* __restrict__ dst0,
-                                        int64_t dst_stride, float* smem) {
+                                        int64_t dst_stride, uint64_t* smem) {
   constexpr int TQ = BQ / 16;
   constexpr int TN = 8;
   constexpr int RPW = BQ / 8;
   constexpr int QSTR = BQ + 4;
   constexpr int BSTR = K1_BN + 4;
-  float* Qs = smem;                   // [2][DK][QSTR]
-  float* Bs = Qs + 2 * K1_DK * QSTR;  // [2][DK][BSTR]
-  float* Dt = Bs + 2 * K1_DK * BSTR;  // [BQ][BSTR]
+  constexpr uint32_t ALL = 0xFFFFFFFFu;
+  uint64_t* lists = smem;                                        // [BQ][32 KW]
+  uint64_t* queues = lists + BQ * 32 * KW;                       // [BQ][QCAP]
+  float* Qs = reinterpret_cast<float*>(queues + BQ * K1_QCAP);   // [2][DK][QSTR]
+  float* Bs = Qs + 2 * K1_DK * QSTR;                             // [2][DK][BSTR]
+  uint32_t* thr = reinterpret_cast<uint32_t*>(Bs + 2 * K1_DK * BSTR);  // [BQ] bits of the k-th distance (ALL: none)
+  uint32_t* thr_sq = thr + BQ;                                   // [BQ] Euclidean: bits no passing square exceeds
+  int* qcnt = reinterpret_cast<int*>(thr_sq + BQ);               // [BQ]
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ty = tid >> 4, tx = tid & 15;
   const int nchunks = (d + K1_DK - 1) / K1_DK;
 
-  uint64_t L[RPW][KW];
-#pragma unroll
-  for (int r = 0; r < RPW; ++r)
-#pragma unroll
-    for (int s = 0; s < KW; ++s) L[r][s] = KEY_NONE;
+  for (int e = tid; e < BQ * 32 * KW; e += K1_THREADS) lists[e] = KEY_NONE;
+  for (int e = tid; e < BQ; e += K1_THREADS) {
+    thr[e] = ALL;
+    thr_sq[e] = ALL;
+    qcnt[e] = 0;
+  }
 
   StageLoader<BQ, VEC> qload;
   StageLoader<K1_BN, VEC> bload;
+  qload.load(qs, qrows, q0, nq, d, 0, tid);
+  bload.load(base, nullptr, nb0, min(nb1, nb0 + K1_BN), d, 0, tid);
+  qload.store(Qs, QSTR, tid);
+  bload.store(Bs, BSTR, tid);
+  __syncthreads();
+  int buf = 0;
 
   for (int64_t t0 = nb0; t0 < nb1; t0 += K1_BN) {
     const int64_t tend = min(nb1, t0 + K1_BN);
@@ -196,39 +313,40 @@ __device__ __forceinline__ void k1_body(const float* __restrict__ base, int64_t 
 #pragma unroll
       for (int j = 0; j < TN / 2; ++j) acc2[i][j] = 0ull;
 
-    qload.load(qs, qrows, q0, nq, d, 0, tid);
-    bload.load(base, nullptr, t0, tend, d, 0, tid);
-    qload.store(Qs, QSTR, tid);
-    bload.store(Bs, BSTR, tid);
-    __syncthreads();
-
     for (int c = 0; c < nchunks; ++c) {
-      const int buf = c & 1;
-      const bool more = (c + 1) < nchunks;
+      const bool last = c + 1 == nchunks;
+      const bool more = !last || tend < nb1;
       if (more) {
-        qload.load(qs, qrows, q0, nq, d, (c + 1) * K1_DK, tid);
-        bload.load(base, nullptr, t0, tend, d, (c + 1) * K1_DK, tid);
+        const int64_t tn = last ? tend : t0;
+        const int c0 = last ? 0 : (c + 1) * K1_DK;
+        qload.load(qs, qrows, q0, nq, d, c0, tid);
+        bload.load(base, nullptr, tn, min(nb1, tn + K1_BN), d, c0, tid);
       }
       const float* qsb = Qs + buf * K1_DK * QSTR;
       const float* bsb = Bs + buf * K1_DK * BSTR;
+      const int kend = min(K1_DK, d - c * K1_DK);  // dimensions past d hold zeros on both sides
 #pragma unroll
-      for (int kk = 0; kk < K1_DK; ++kk) {
-        float qv[TQ], bv[TN];
-        load_q_frag<TQ>(qsb + kk * QSTR, ty, qv);
-        load_b_frag(bsb + kk * BSTR, tx, bv);
-        uint64_t b2[TN / 2];
+      for (int k4 = 0; k4 < K1_DK; k4 += 4) {
+        if (k4 >= kend) break;
 #pragma unroll
-        for (int j = 0; j < TN / 2; ++j) b2[j] = f2::pack(bv[2 * j], bv[2 * j + 1]);
+        for (int kk = k4; kk < k4 + 4; ++kk) {
+          float qv[TQ], bv[TN];
+          load_q_frag<TQ>(qsb + kk * QSTR, ty, qv);
+          load_b_frag(bsb + kk * BSTR, tx, bv);
+          uint64_t b2[TN / 2];
 #pragma unroll
-        for (int i = 0; i < TQ; ++i) {
-          const uint64_t q2 = f2::pack(qv[i], qv[i]);
+          for (int j = 0; j < TN / 2; ++j) b2[j] = f2::pack(bv[2 * j], bv[2 * j + 1]);
 #pragma unroll
-          for (int j = 0; j < TN / 2; ++j) {
-            if constexpr (METRIC == MANN_METRIC_COSINE) {
-              acc2[i][j] = f2::fma(q2, b2[j], acc2[i][j]);
-            } else {
-              const uint64_t t = f2::sub(q2, b2[j]);
-              acc2[i][j] = f2::fma(t, t, acc2[i][j]);
+          for (int i = 0; i < TQ; ++i) {
+            const uint64_t q2 = f2::pack(qv[i], qv[i]);
+#pragma unroll
+            for (int j = 0; j < TN / 2; ++j) {
+              if constexpr (METRIC == MANN_METRIC_COSINE) {
+                acc2[i][j] = f2::fma(q2, b2[j], acc2[i][j]);
+              } else {
+                const uint64_t t = f2::sub(q2, b2[j]);
+                acc2[i][j] = f2::fma(t, t, acc2[i][j]);
+              }
             }
           }
         }
@@ -238,118 +356,140 @@ __device__ __forceinline__ void k1_body(const float* __restrict__ base, int64_t 
         bload.store(Bs + (buf ^ 1) * K1_DK * BSTR, BSTR, tid);
       }
       __syncthreads();
+      buf ^= 1;
     }
 
-    float acc[TQ][TN];
+    float acc[TQ * TN];  // element i * 8 + j: row tile_row(ty, i), column tile_col(tx, j)
 #pragma unroll
     for (int i = 0; i < TQ; ++i)
 #pragma unroll
-      for (int j = 0; j < TN / 2; ++j) f2::unpack(acc2[i][j], acc[i][2 * j], acc[i][2 * j + 1]);
-    // finish the metric and stage the tile
+      for (int j = 0; j < TN / 2; ++j) f2::unpack(acc2[i][j], acc[i * TN + 2 * j], acc[i * TN + 2 * j + 1]);
+    if constexpr (METRIC == MANN_METRIC_COSINE) {
 #pragma unroll
-    for (int i = 0; i < TQ; ++i) {
-      const int r = tile_row<TQ>(ty, i);
-      float qn = 0.f;
-      if constexpr (METRIC == MANN_METRIC_COSINE) {
-        const int64_t gq = q0 + r;
-        qn = (gq < nq) ? qnorm[qrows ? qrows[gq] : gq] : 1.0f;
-      }
+      for (int i = 0; i < TQ; ++i) {
+        const int64_t gq = q0 + tile_row<TQ>(ty, i);
+        const float qn = (gq < nq) ? qnorm[qrows ? qrows[gq] : gq] : 1.0f;
 #pragma unroll
-      for (int j = 0; j < TN; ++j) {
-        float v = acc[i][j];
-        if constexpr (METRIC == MANN_METRIC_EUCLIDEAN) {
-          v = __fsqrt_rn(v);
-        } else if constexpr (METRIC == MANN_METRIC_COSINE) {
+        for (int j = 0; j < TN; ++j) {
           const int64_t gb = t0 + tile_col(tx, j);
           const float bn = (gb < tend) ? bnorm[gb] : 1.0f;
           const float den = __fmul_rn(__fsqrt_rn(qn), __fsqrt_rn(bn));
-          v = __fsub_rn(1.0f, __fdiv_rn(v, den));
+          float v = __fsub_rn(1.0f, __fdiv_rn(acc[i * TN + j], den));
           if (v < 0.0f) v = 0.0f;
+          acc[i * TN + j] = v;
         }
-        acc[i][j] = v;
-      }
-      float* drow = Dt + r * BSTR;
-      *reinterpret_cast<float4*>(drow + tx * 4) =
-          make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-      *reinterpret_cast<float4*>(drow + 64 + tx * 4) =
-          make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]);
-    }
-    __syncthreads();
-
-    // fold the tile into the per-row lists (warp `warp` owns RPW rows)
-#pragma unroll
-    for (int r = 0; r < RPW; ++r) {
-      const int row = warp * RPW + r;
-      const float* drow = Dt + row * BSTR;
-      uint64_t thr = list_get<KW>(L[r], k - 1);
-      // keys are built only for distances at or below the threshold's (the
-      // exact key order decides); a list that is not full, or whose threshold
-      // is NaN, takes every key through the exact comparison
-      const float thr_f = thr == KEY_NONE ? 0.0f : key_dist(thr);
-      const bool exact = thr == KEY_NONE || !(thr_f == thr_f);
-      uint64_t key[4];
-      unsigned pend = 0;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int col = lane + 32 * j;
-        const int64_t gid = t0 + col;
-        const float dv = drow[col];
-        key[j] = KEY_NONE;
-        if (gid < tend && (exact || dv <= thr_f)) {
-          key[j] = make_key(dv, (uint32_t)gid);
-          if (key[j] < thr) pend |= 1u << j;
-        }
-      }
-      for (;;) {
-        const unsigned any = __ballot_sync(FULL, pend != 0);
-        if (!any) break;
-        const int src = __ffs(any) - 1;
-        uint64_t mine = KEY_NONE;
-        if (pend) {
-          const int j = __ffs(pend) - 1;
-          mine = (j == 0) ? key[0] : (j == 1) ? key[1] : (j == 2) ? key[2] : key[3];
-        }
-        const uint64_t cnd = __shfl_sync(FULL, mine, src);
-        if (lane == src) pend &= pend - 1;
-        if (cnd < thr) {
-          list_insert<KW>(L[r], cnd, lane);
-          thr = list_get<KW>(L[r], k - 1);
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (!(key[j] < thr)) pend &= ~(1u << j);
       }
     }
-    __syncthreads();
+    // candidates of this thread: one bit per element
+    const bool partial_tile = tend - t0 < K1_BN;
+    uint32_t pend = 0;
+#pragma unroll
+    for (int i = 0; i < TQ; ++i) {
+      const int r = tile_row<TQ>(ty, i);
+      const uint32_t lim = METRIC == MANN_METRIC_EUCLIDEAN ? thr_sq[r] : thr[r];
+      uint32_t m = 0;
+#pragma unroll
+      for (int j = 0; j < TN; ++j) m |= (__float_as_uint(acc[i * TN + j]) < lim ? 1u : 0u) << j;
+      if (q0 + r >= nq) m = 0;
+      pend |= m << (i * TN);
+    }
+    if (partial_tile) {
+      uint32_t cm = 0;
+#pragma unroll
+      for (int j = 0; j < TN; ++j) cm |= (t0 + tile_col(tx, j) < tend ? 1u : 0u) << j;
+#pragma unroll
+      for (int i = 1; i < TQ; ++i) cm |= (cm & 0xFFu) << (i * TN);
+      pend &= cm;
+    }
+    for (bool first = true;; first = false) {
+      uint32_t todo = pend;
+      while (todo) {
+        const int e = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const int r = tile_row<TQ>(ty, e >> 3);
+        float v = select_tree<TQ * TN>(acc, e);
+        if constexpr (METRIC == MANN_METRIC_EUCLIDEAN) v = __fsqrt_rn(v);
+        const uint32_t lim = thr[r], vb = __float_as_uint(v);
+        if (first ? vb < lim : vb <= lim) {
+          const int pos = atomicAdd(&qcnt[r], 1);
+          if (pos >= K1_QCAP) continue;  // full: tested again in the next round
+          queues[r * K1_QCAP + pos] = make_key(v, (uint32_t)(t0 + tile_col(tx, e & 7)));
+        }
+        pend &= ~(1u << e);
+      }
+      const bool again = __syncthreads_or(pend != 0);
+      // merge the queues of this warp's rows: all that hold K1_DRAIN
+      // candidates, and in the last round of the last tile every one
+      const int least = tend < nb1 || again ? K1_DRAIN : 1;
+      for (int r = warp * RPW; r < warp * RPW + RPW; ++r) {
+        const int cnt = min(qcnt[r], K1_QCAP);
+        if (cnt < least) continue;  // warp-uniform
+        uint64_t kth;
+        k1_drain_row<KW>(lists + r * 32 * KW, queues + r * K1_QCAP, cnt, k, lane, kth);
+        __syncwarp();
+        if (lane == 0) {
+          qcnt[r] = 0;
+          if (kth != KEY_NONE) {
+            const float t = key_dist(kth);
+            thr[r] = __float_as_uint(t);
+            // sqrt(v) < t needs v < t^2 (1 + 2^-21): a square at or past that
+            // bound has a larger root however both round
+            if constexpr (METRIC == MANN_METRIC_EUCLIDEAN)
+              thr_sq[r] = __float_as_uint(__fadd_ru(__fmul_ru(__fmul_ru(t, t), 1.0000005f), 1e-44f));
+          }
+        }
+      }
+      if (!again) break;
+      __syncthreads();
+    }
   }
-
-  // write this split's lists
-#pragma unroll
-  for (int r = 0; r < RPW; ++r) {
-    const int64_t gq = q0 + warp * RPW + r;
-    if (gq >= nq) continue;
+  // write this split's lists (each warp its own rows)
+  for (int r = warp * RPW; r < warp * RPW + RPW; ++r) {
+    const int64_t gq = q0 + r;
+    if (gq >= nq) break;
     uint64_t* dst = dst0 + gq * dst_stride;
-#pragma unroll
-    for (int s = 0; s < KW; ++s) {
-      const int e = s * 32 + lane;
-      if (e < k) dst[e] = L[r][s];
-    }
+    for (int e = lane; e < k; e += 32) dst[e] = lists[r * 32 * KW + e];
   }
 }
 
+// How the tile kernel's CTAs share the (query block, point tile) units.
+// Unit u is tile u % tiles of query block u / tiles.
+//   splits == 0: CTA c takes units [c per, (c + 1) per) -- an equal share of
+//     the whole work, whatever the block and tile counts; a query block's
+//     lists go to consecutive slots, one per CTA that touches it.
+//   splits > 0: CTA c takes split c % splits (tiles_per tiles) of query block
+//     c / splits.
+struct K1Walk {
+  int64_t total, per;
+  int tiles, splits, tiles_per;
+  int slots;  // lists per query row
+};
+
 template <int METRIC, int BQ, int KW, bool VEC>
-__global__ void __launch_bounds__(K1_THREADS, 1)
+__global__ void __launch_bounds__(K1_THREADS, k1_ctas<BQ, KW>())
     k1_tile_topk(const float* __restrict__ base, int64_t n, const float* __restrict__ qs,
                  const int32_t* __restrict__ qrows, int64_t nq, int d,
-                 const float* __restrict__ qnorm, const float* __restrict__ bnorm, int k,
-                 int64_t split_len, int nsplit, uint64_t* __restrict__ partial) {
-  extern __shared__ float4 k1_smem[];
-  const int split = blockIdx.y;
-  const int64_t nb0 = (int64_t)split * split_len;
-  const int64_t nb1 = min(n, nb0 + split_len);
-  k1_body<METRIC, BQ, KW, VEC>(base, nb0, nb1, qs, qrows, (int64_t)blockIdx.x * BQ, nq, d, qnorm, bnorm, k,
-                               partial + (int64_t)split * k, (int64_t)nsplit * k,
-                               reinterpret_cast<float*>(k1_smem));
+                 const float* __restrict__ qnorm, const float* __restrict__ bnorm, int k, K1Walk w,
+                 uint64_t* __restrict__ partial) {
+  extern __shared__ __align__(16) uint64_t k1_smem[];
+  int64_t u = (int64_t)blockIdx.x * w.per, uend = min(w.total, u + w.per);
+  if (w.splits > 0) {
+    const int64_t qb = blockIdx.x / w.splits;
+    const int t0 = (int)(blockIdx.x % w.splits) * w.tiles_per;
+    u = qb * w.tiles + t0;
+    uend = qb * w.tiles + min(w.tiles, t0 + w.tiles_per);
+  }
+  while (u < uend) {
+    const int64_t qb = u / w.tiles;
+    const int t0 = (int)(u - qb * w.tiles);
+    const int t1 = (int)min((int64_t)w.tiles, t0 + (uend - u));
+    const int slot = w.splits > 0 ? (int)(blockIdx.x % w.splits)
+                                  : (int)((int64_t)blockIdx.x - qb * w.tiles / w.per);
+    k1_body<METRIC, BQ, KW, VEC>(base, (int64_t)t0 * K1_BN, min(n, (int64_t)t1 * K1_BN), qs, qrows, qb * BQ, nq, d,
+                                 qnorm, bnorm, k, partial + (int64_t)slot * k, (int64_t)w.slots * k, k1_smem);
+    u += t1 - t0;
+    __syncthreads();  // the next block's set-up overwrites the lists
+  }
 }
 
 // Segmented persistent form over a device work queue: the work items of many
@@ -363,11 +503,11 @@ __global__ void __launch_bounds__(K1_THREADS, 1)
 // bounded by `wait_cycles`, after which the CTA records MANN_ETIMEOUT in
 // q->status and returns without touching any list.
 template <int METRIC, int BQ, int KW, bool VEC>
-__global__ void __launch_bounds__(K1_THREADS, 2)
+__global__ void __launch_bounds__(K1_THREADS, k1_ctas<BQ, KW>())
     k1_persistent(const float* __restrict__ data, const SegItem* __restrict__ items, SegQueue* q, unsigned epoch,
                   long long wait_cycles, int d, int k, int nsplit, uint64_t* __restrict__ partial,
                   const int32_t* __restrict__ qrows) {
-  extern __shared__ float4 k1_smem[];
+  extern __shared__ __align__(16) uint64_t k1_smem[];
   __shared__ int s_item;
   __shared__ int s_count;
   if (threadIdx.x == 0) {
@@ -397,8 +537,7 @@ __global__ void __launch_bounds__(K1_THREADS, 2)
     if (idx < 0) break;
     const SegItem it = items[idx];
     k1_body<METRIC, BQ, KW, VEC>(data, it.nb0, it.nb1, data, qrows, it.q0, it.qend, d, nullptr, nullptr, k,
-                                 partial + (int64_t)it.split * k, (int64_t)nsplit * k,
-                                 reinterpret_cast<float*>(k1_smem));
+                                 partial + (int64_t)it.split * k, (int64_t)nsplit * k, k1_smem);
     __syncthreads();  // s_item is rewritten only after every thread read it
   }
 }
@@ -663,14 +802,21 @@ mann_status launch_few_m(int grid, const float* base, int64_t n, const float* qs
   return MANN_OK;
 }
 
-// Merge nsplit sorted lists of k keys per query into one sorted list of k.
-// One warp per query; lane s walks list s (and s+32, ...).
-__global__ void merge_lists_kernel(const uint64_t* __restrict__ partial, int64_t nq, int nsplit,
-                                   int k, uint64_t* __restrict__ out) {
+// Merge up to `slots` sorted lists of k keys per query into one sorted list
+// of k.  One warp per query; lane s walks list s (and s+32, ...).  A balanced
+// walk of the tile kernel (w.per > 0, bq rows per block) wrote only the slots
+// of the CTAs that its query block met.
+__global__ void merge_lists_kernel(const uint64_t* __restrict__ partial, int64_t nq, int slots,
+                                   int k, uint64_t* __restrict__ out, int64_t tiles, int64_t per, int bq) {
   const int lane = threadIdx.x & 31;
   const int64_t q = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (q >= nq) return;
-  const uint64_t* src = partial + q * (int64_t)nsplit * k;
+  const uint64_t* src = partial + q * (int64_t)slots * k;
+  int nsplit = slots;
+  if (per > 0) {
+    const int64_t qb = q / bq;
+    nsplit = (int)(((qb + 1) * tiles - 1) / per - qb * tiles / per) + 1;
+  }
   constexpr int MAXL = 8;  // lists per lane (nsplit <= 256)
   int head[MAXL];
   uint64_t cur[MAXL];
@@ -723,18 +869,44 @@ __global__ void finish_kernel(const uint64_t* __restrict__ keys, int64_t nq, int
   }
 }
 
+// query rows per CTA of the tile kernel
+int k1_rows(int64_t nq, int k) { return nq > 32 && k <= 128 ? 64 : 32; }
+
+// The tile kernel's walk.  splits > 0: that many splits per query block.
+// splits == 0: an equal share of the units for every CTA that the device
+// holds at once -- a grid of whole query blocks leaves a nearly empty last
+// wave (20,011 rows: 313 blocks on 456 places) or, with few blocks, idle SMs
+// -- unless there are so many query blocks that whole ones balance to within
+// an eighth, which needs no merge.
+K1Walk k1_walk(int num_sms, int64_t n, int64_t nq, int k, int splits) {
+  const int bq = k1_rows(nq, k);
+  const int64_t qblocks = ceil_div(nq, bq);
+  K1Walk w{};
+  w.tiles = (int)ceil_div(n, K1_BN);
+  w.total = qblocks * w.tiles;
+  const int64_t places = (int64_t)num_sms * (k <= 32 ? k1_ctas<64, 1>() : k1_ctas<64, 2>());
+  if (splits == 0 && qblocks >= 8 * places) splits = 1;
+  if (splits > 0) {
+    w.tiles_per = (int)ceil_div(w.tiles, splits);
+    w.splits = (int)ceil_div(w.tiles, w.tiles_per);
+    w.slots = w.splits;
+    return w;
+  }
+  w.per = std::max(ceil_div(w.total, places), ceil_div(w.tiles, 96));  // at most 97 lists per row
+  w.slots = w.per % w.tiles == 0 ? 1 : (w.tiles % w.per == 0 ? (int)(w.tiles / w.per) : (int)((w.tiles - 2) / w.per) + 2);
+  return w;
+}
+
 template <int METRIC, int BQ, int KW, bool VEC>
 mann_status launch_k1(Context* ctx, const float* base, int64_t n, const float* qs, const int32_t* rows,
-                      int64_t nq, int d, const float* qn, const float* bn, int k,
-                      int64_t split_len, int nsplit, uint64_t* partial, cudaStream_t s) {
-  constexpr int QSTR = BQ + 4, BSTR = K1_BN + 4;
-  const size_t smem = sizeof(float) * (2 * K1_DK * QSTR + 2 * K1_DK * BSTR + BQ * BSTR);
+                      int64_t nq, int d, const float* qn, const float* bn, int k, const K1Walk& w, uint64_t* partial,
+                      cudaStream_t s) {
+  constexpr size_t smem = k1_smem_bytes<BQ, KW>();
   auto kern = k1_tile_topk<METRIC, BQ, KW, VEC>;
   MANN_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  dim3 grid((unsigned)ceil_div(nq, BQ), (unsigned)nsplit);
+  const int64_t grid = w.splits > 0 ? ceil_div(nq, BQ) * w.splits : ceil_div(w.total, w.per);
   ctx->time_begin(s);
-  kern<<<grid, K1_THREADS, smem, s>>>(base, n, qs, rows, nq, d, qn, bn, k, split_len, nsplit,
-                                      partial);
+  kern<<<(unsigned)grid, K1_THREADS, smem, s>>>(base, n, qs, rows, nq, d, qn, bn, k, w, partial);
   ctx->time_end(s);
   MANN_CHECK_LAUNCH();
   return MANN_OK;
@@ -742,26 +914,28 @@ mann_status launch_k1(Context* ctx, const float* base, int64_t n, const float* q
 
 template <int METRIC, bool VEC>
 mann_status dispatch_k1(Context* ctx, int k, const float* base, int64_t n, const float* qs, const int32_t* rows,
-                        int64_t nq, int d, const float* qn, const float* bn, int64_t split_len,
-                        int nsplit, uint64_t* partial, cudaStream_t s) {
-  if (nq <= 32) {  // a handful of queries (e.g. rows re-run by the exact scan): narrow tiles
-    if (k <= 32)
-      return launch_k1<METRIC, 32, 1, VEC>(ctx, base, n, qs, rows, nq, d, qn, bn, k, split_len,
-                                           nsplit, partial, s);
-    return launch_k1<METRIC, 32, 8, VEC>(ctx, base, n, qs, rows, nq, d, qn, bn, k, split_len,
-                                         nsplit, partial, s);
-  }
-  if (k <= 32)
-    return launch_k1<METRIC, 128, 1, VEC>(ctx, base, n, qs, rows, nq, d, qn, bn, k, split_len, nsplit,
-                                          partial, s);
-  if (k <= 64)
-    return launch_k1<METRIC, 128, 2, VEC>(ctx, base, n, qs, rows, nq, d, qn, bn, k, split_len, nsplit,
-                                          partial, s);
-  if (k <= 128)
-    return launch_k1<METRIC, 64, 4, VEC>(ctx, base, n, qs, rows, nq, d, qn, bn, k, split_len, nsplit,
-                                         partial, s);
-  return launch_k1<METRIC, 32, 8, VEC>(ctx, base, n, qs, rows, nq, d, qn, bn, k, split_len, nsplit,
-                                       partial, s);
+                        int64_t nq, int d, const float* qn, const float* bn, const K1Walk& w, uint64_t* partial,
+                        cudaStream_t s) {
+  if (k1_rows(nq, k) == 32)
+    return launch_k1<METRIC, 32, 8, VEC>(ctx, base, n, qs, rows, nq, d, qn, bn, k, w, partial, s);
+  if (k <= 32) return launch_k1<METRIC, 64, 1, VEC>(ctx, base, n, qs, rows, nq, d, qn, bn, k, w, partial, s);
+  if (k <= 64) return launch_k1<METRIC, 64, 2, VEC>(ctx, base, n, qs, rows, nq, d, qn, bn, k, w, partial, s);
+  return launch_k1<METRIC, 64, 4, VEC>(ctx, base, n, qs, rows, nq, d, qn, bn, k, w, partial, s);
+}
+
+// The tile kernel for any metric and alignment.
+mann_status run_k1(Context* ctx, int metric, int k, const float* base, int64_t n, const float* qs, const int32_t* rows,
+                   int64_t nq, int d, const float* qn, const float* bn, const K1Walk& w, uint64_t* partial,
+                   cudaStream_t s) {
+  const bool vec = (d % 4 == 0) && ((reinterpret_cast<uintptr_t>(base) & 15) == 0) &&
+                   ((reinterpret_cast<uintptr_t>(qs) & 15) == 0);
+#define K1_METRIC(M)                                                                                    \
+  return vec ? dispatch_k1<M, true>(ctx, k, base, n, qs, rows, nq, d, qn, bn, w, partial, s)            \
+             : dispatch_k1<M, false>(ctx, k, base, n, qs, rows, nq, d, qn, bn, w, partial, s)
+  if (metric == MANN_METRIC_EUCLIDEAN) K1_METRIC(MANN_METRIC_EUCLIDEAN);
+  if (metric == MANN_METRIC_SQEUCLIDEAN) K1_METRIC(MANN_METRIC_SQEUCLIDEAN);
+  K1_METRIC(MANN_METRIC_COSINE);
+#undef K1_METRIC
 }
 
 }  // namespace
@@ -770,8 +944,7 @@ template <int METRIC, int BQ, int KW, bool VEC>
 static mann_status launch_pers_t(int num_sms, const float* data, const SegItem* items, SegQueue* q, unsigned epoch,
                                  long long wait_cycles, int d, int k, int nsplit, uint64_t* partial,
                                  const int32_t* qrows, cudaStream_t s) {
-  constexpr int QSTR = BQ + 4, BSTR = K1_BN + 4;
-  const size_t smem = sizeof(float) * (2 * K1_DK * QSTR + 2 * K1_DK * BSTR + BQ * BSTR);
+  constexpr size_t smem = k1_smem_bytes<BQ, KW>();
   auto kern = k1_persistent<METRIC, BQ, KW, VEC>;
   MANN_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per_sm = 0;
@@ -797,18 +970,16 @@ mann_status launch_k1_persistent(int num_sms, const float* data, const SegItem* 
       if (bq == 32) PERS_CASE(MANN_METRIC_EUCLIDEAN, 32, 2);
       PERS_CASE(MANN_METRIC_EUCLIDEAN, 64, 2);
     }
-    if (bq == 64) PERS_CASE(MANN_METRIC_EUCLIDEAN, 64, 1);
     if (bq == 32) PERS_CASE(MANN_METRIC_EUCLIDEAN, 32, 1);
-    PERS_CASE(MANN_METRIC_EUCLIDEAN, 128, 1);
+    PERS_CASE(MANN_METRIC_EUCLIDEAN, 64, 1);
   }
   if (metric == MANN_METRIC_SQEUCLIDEAN) {
     if (k > 32) {
       if (bq == 32) PERS_CASE(MANN_METRIC_SQEUCLIDEAN, 32, 2);
       PERS_CASE(MANN_METRIC_SQEUCLIDEAN, 64, 2);
     }
-    if (bq == 64) PERS_CASE(MANN_METRIC_SQEUCLIDEAN, 64, 1);
     if (bq == 32) PERS_CASE(MANN_METRIC_SQEUCLIDEAN, 32, 1);
-    PERS_CASE(MANN_METRIC_SQEUCLIDEAN, 128, 1);
+    PERS_CASE(MANN_METRIC_SQEUCLIDEAN, 64, 1);
   }
 #undef PERS_CASE
   return fail(MANN_EINVAL_ARG, "batched graphs: Euclidean or SqEuclidean");
@@ -818,7 +989,7 @@ mann_status launch_merge_lists(const uint64_t* partial, int64_t nq, int nsplit, 
                                cudaStream_t s) {
   if (nq <= 0) return MANN_OK;
   if (nsplit > 128) return fail(MANN_EINVAL_ARG, "at most 128 lists per query can be merged");
-  merge_lists_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, s>>>(partial, nq, nsplit, k, out);
+  merge_lists_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, s>>>(partial, nq, nsplit, k, out, 0, 0, 1);
   MANN_CHECK_LAUNCH();
   return MANN_OK;
 }
@@ -876,54 +1047,23 @@ mann_status knn_fp32_keys(Context* ctx, cudaStream_t s, const float* base, int64
     }
     uint64_t* keys = nullptr;
     MANN_TRY(ctx->scratch_t(slot_keys, (size_t)nq * kk, &keys));
-    merge_lists_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, s>>>(partial, nq, grid, kk, keys);
+    merge_lists_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, s>>>(partial, nq, grid, kk, keys, 0, 0, 1);
     MANN_CHECK_LAUNCH();
     *out_keys = keys;
     return MANN_OK;
   }
-  const int bq = nq <= 32 ? 32 : (kk <= 64 ? 128 : (kk <= 128 ? 64 : 32));
-  const int64_t qblocks = ceil_div(nq, bq);
-  const int64_t tiles = ceil_div(n, K1_BN);
-  // Split the points so that the grid covers the SMs at least once.
-  int64_t want = std::max<int64_t>(1, ceil_div(ctx->num_sms, qblocks));
-  want = std::min<int64_t>(want, std::min<int64_t>(tiles, 128));
-  const int64_t tiles_per = ceil_div(tiles, want);
-  const int nsplit = (int)ceil_div(tiles, tiles_per);
-  const int64_t split_len = tiles_per * K1_BN;
-
+  const K1Walk w = k1_walk(ctx->num_sms, n, nq, kk, 0);
   uint64_t* partial = nullptr;
-  MANN_TRY(ctx->scratch_t(slot_partial, (size_t)nq * nsplit * kk, &partial));
-  const bool vec = (d % 4 == 0) && ((reinterpret_cast<uintptr_t>(base) & 15) == 0) &&
-                   ((reinterpret_cast<uintptr_t>(qs) & 15) == 0);
-  mann_status st;
-  switch (metric) {
-    case MANN_METRIC_EUCLIDEAN:
-      st = vec ? dispatch_k1<MANN_METRIC_EUCLIDEAN, true>(ctx, kk, base, n, qs, rows, nq, d, qn, bn,
-                                                          split_len, nsplit, partial, s)
-               : dispatch_k1<MANN_METRIC_EUCLIDEAN, false>(ctx, kk, base, n, qs, rows, nq, d, qn, bn,
-                                                           split_len, nsplit, partial, s);
-      break;
-    case MANN_METRIC_SQEUCLIDEAN:
-      st = vec ? dispatch_k1<MANN_METRIC_SQEUCLIDEAN, true>(ctx, kk, base, n, qs, rows, nq, d, qn, bn,
-                                                            split_len, nsplit, partial, s)
-               : dispatch_k1<MANN_METRIC_SQEUCLIDEAN, false>(ctx, kk, base, n, qs, rows, nq, d, qn,
-                                                             bn, split_len, nsplit, partial, s);
-      break;
-    default:
-      st = vec ? dispatch_k1<MANN_METRIC_COSINE, true>(ctx, kk, base, n, qs, rows, nq, d, qn, bn,
-                                                       split_len, nsplit, partial, s)
-               : dispatch_k1<MANN_METRIC_COSINE, false>(ctx, kk, base, n, qs, rows, nq, d, qn, bn,
-                                                        split_len, nsplit, partial, s);
-      break;
-  }
-  MANN_TRY(st);
-  if (nsplit == 1) {
+  MANN_TRY(ctx->scratch_t(slot_partial, (size_t)nq * w.slots * kk, &partial));
+  MANN_TRY(run_k1(ctx, metric, kk, base, n, qs, rows, nq, d, qn, bn, w, partial, s));
+  if (w.slots == 1) {
     *out_keys = partial;
     return MANN_OK;
   }
   uint64_t* keys = nullptr;
   MANN_TRY(ctx->scratch_t(slot_keys, (size_t)nq * kk, &keys));
-  merge_lists_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, s>>>(partial, nq, nsplit, kk, keys);
+  merge_lists_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, s>>>(partial, nq, w.slots, kk, keys, w.tiles, w.per,
+                                                               k1_rows(nq, kk));
   MANN_CHECK_LAUNCH();
   *out_keys = keys;
   return MANN_OK;
@@ -934,7 +1074,7 @@ mann_status knn_fp32_keys(Context* ctx, cudaStream_t s, const float* base, int64
 namespace mann {
 
 // Plan of the FP32 form for (n, nq, kk) on a device with num_sms SMs, as
-// knn_fp32_keys makes it: a few rows (nq <= FEW_Q, kk <= 64) go to the
+// knn_fp32_keys_on makes it: a few rows (nq <= FEW_Q, kk <= 64) go to the
 // few-row kernel with `*nsplit_out` = its grid of point slices; otherwise the
 // tile kernel with `*nsplit_out` point splits.  `*words_out` = the uint64
 // words of scratch (per-split lists, then merged lists when there is more
@@ -992,33 +1132,10 @@ mann_status knn_fp32_keys_on(int num_sms, cudaStream_t s, const float* base, int
         break;
     }
   } else {
-    const int64_t tiles = ceil_div(n, K1_BN);
-    const int64_t tiles_per = ceil_div(tiles, nsplit);
-    const int64_t split_len = tiles_per * K1_BN;
     Context plain;  // carries the SM count; no timing, no scratch
     plain.num_sms = num_sms;
-    const bool vec = (d % 4 == 0) && ((reinterpret_cast<uintptr_t>(base) & 15) == 0) &&
-                     ((reinterpret_cast<uintptr_t>(qs) & 15) == 0);
-    switch (metric) {
-      case MANN_METRIC_EUCLIDEAN:
-        st = vec ? dispatch_k1<MANN_METRIC_EUCLIDEAN, true>(&plain, kk, base, n, qs, nullptr, nq, d, qn,
-                                                            bn, split_len, nsplit, partial, s)
-                 : dispatch_k1<MANN_METRIC_EUCLIDEAN, false>(&plain, kk, base, n, qs, nullptr, nq, d,
-                                                             qn, bn, split_len, nsplit, partial, s);
-        break;
-      case MANN_METRIC_SQEUCLIDEAN:
-        st = vec ? dispatch_k1<MANN_METRIC_SQEUCLIDEAN, true>(&plain, kk, base, n, qs, nullptr, nq, d,
-                                                              qn, bn, split_len, nsplit, partial, s)
-                 : dispatch_k1<MANN_METRIC_SQEUCLIDEAN, false>(&plain, kk, base, n, qs, nullptr, nq, d,
-                                                               qn, bn, split_len, nsplit, partial, s);
-        break;
-      default:
-        st = vec ? dispatch_k1<MANN_METRIC_COSINE, true>(&plain, kk, base, n, qs, nullptr, nq, d, qn,
-                                                         bn, split_len, nsplit, partial, s)
-                 : dispatch_k1<MANN_METRIC_COSINE, false>(&plain, kk, base, n, qs, nullptr, nq, d, qn,
-                                                          bn, split_len, nsplit, partial, s);
-        break;
-    }
+    st = run_k1(&plain, metric, kk, base, n, qs, nullptr, nq, d, qn, bn, k1_walk(num_sms, n, nq, kk, nsplit), partial,
+                s);
   }
   MANN_TRY(st);
   if (nsplit == 1) {
@@ -1026,7 +1143,7 @@ mann_status knn_fp32_keys_on(int num_sms, cudaStream_t s, const float* base, int
     return MANN_OK;
   }
   uint64_t* keys = partial + (size_t)nq * nsplit * kk;
-  merge_lists_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, s>>>(partial, nq, nsplit, kk, keys);
+  merge_lists_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, s>>>(partial, nq, nsplit, kk, keys, 0, 0, 1);
   MANN_CHECK_LAUNCH();
   *out_keys = keys;
   return MANN_OK;
