@@ -100,77 +100,311 @@ __global__ void gather_rows_kernel(const float* __restrict__ X, int d, const int
 }
 
 // ------------------------------------------------------------------ k-means++
-__global__ void fill_inf_kernel(float* __restrict__ v, int64_t n) {
-  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < n) v[j] = __int_as_float(0x7F800000);
-}
+// A step draws the next centroid: every point's smallest squared distance to
+// the centroids chosen so far is brought up to date with the last one, the
+// distances are summed in PP_CHUNK-point blocks and over the blocks, and the
+// running sum is searched for u * total -- all sums in FP64, in point order.
+//
+// One launch per step: a CTA updates PP_PTS points, the last CTA of a block
+// sums the block, and the last block's CTA searches (tickets below).  FP64
+// additions are slow and a chain of them slower still (one thread per 1024
+// additions took 110 us per step, as did the one-thread search), so sums are
+// made in 64-bit integers, in parallel, whenever that is exact: with every
+// term a multiple of 2^L and the total at most 2^53 units, each partial sum is
+// a double, so the ordered FP64 sum rounds nowhere and equals the integer one.
+// Where the terms' range does not allow it, one thread adds in order.
+// Measured (262,144 x 128, 1,024 centroids): 265 -> 50 us per step; the row
+// reads (134 MB per step) are what is left.
+constexpr int PP_PTS = 128;  // points (and threads) per CTA
+constexpr int PP_DC = 64;    // dimensions staged at a time
+constexpr int PP_STR = PP_DC + 4;
+constexpr long long PP_EXACT = 1ll << 53;
+static_assert(PP_CHUNK % PP_PTS == 0, "a CTA belongs to one block of points");
 
-// min D^2 of every point against the centroid X[idx[i-1]] (FP32 difference
-// form, dimensions in order).  Block of 128 points staged 32 dims at a time.
-__global__ void __launch_bounds__(128) pp_update_kernel(const float* __restrict__ X, int64_t n, int d,
-                                                        const int64_t* __restrict__ idx, int i,
-                                                        float* __restrict__ mind) {
-  __shared__ float xs[32][129];
-  __shared__ float cs[32];
-  const int64_t j0 = (int64_t)blockIdx.x * 128;
-  const int64_t j = j0 + threadIdx.x;
-  const float* c = X + idx[i - 1] * d;
-  float s = 0.0f;
-  for (int c0 = 0; c0 < d; c0 += 32) {
-    for (int e = threadIdx.x; e < 128 * 32; e += 128) {
-      const int r = e >> 5, cc = e & 31;
-      xs[cc][r] = (j0 + r < n && c0 + cc < d) ? X[(j0 + r) * d + c0 + cc] : 0.0f;
-    }
-    if (threadIdx.x < 32) cs[threadIdx.x] = (c0 + threadIdx.x < d) ? c[c0 + threadIdx.x] : 0.0f;
-    __syncthreads();
-    const int lim = min(32, d - c0);
-    for (int cc = 0; cc < lim; ++cc) {
-      const float t = __fsub_rn(xs[cc][threadIdx.x], cs[cc]);
-      s = __fmaf_rn(t, t, s);
-    }
-    __syncthreads();
+// v = mant * 2^exp2 with an odd mantissa (or 0); false for inf and NaN
+__device__ __forceinline__ bool pp_split(double v, long long& mant, int& exp2) {
+  const long long bits = __double_as_longlong(v);
+  const int e = (int)((bits >> 52) & 0x7FF);
+  mant = (bits & 0xFFFFFFFFFFFFFll) | (e ? (1ll << 52) : 0ll);
+  exp2 = (e ? e : 1) - 1075;
+  if (mant) {
+    const int tz = __ffsll(mant) - 1;
+    mant >>= tz;
+    exp2 += tz;
   }
-  if (j < n && s < mind[j]) mind[j] = s;
+  return e != 0x7FF && bits >= 0;
+}
+// 2^e as a double, -1022 <= e <= 1023
+__device__ __forceinline__ double pp_pow2(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
+
+// terms in units of 2^low, or -1 past 2^53
+__device__ __forceinline__ long long pp_units(long long mant, int exp2, int low) {
+  if (mant == 0) return 0;
+  const int sh = exp2 - low;
+  if (sh > 52 || mant > (PP_EXACT >> sh)) return -1;
+  return mant << sh;
 }
 
-__global__ void pp_block_sums_kernel(const float* __restrict__ mind, int64_t n,
-                                     double* __restrict__ bsum) {
-  const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t nb = (n + PP_CHUNK - 1) / PP_CHUNK;
-  if (b >= nb) return;
-  double s = 0.0;
-  const int64_t e = min(n, (b + 1) * PP_CHUNK);
-  for (int64_t j = b * PP_CHUNK; j < e; ++j) s += (double)mind[j];
-  bsum[b] = s;
+__device__ __forceinline__ int pp_block_min(int v, int* red) {
+  for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = red[0];
+  for (int w = 1; w < PP_PTS / 32; ++w) v = min(v, red[w]);
+  return v;
 }
 
-// searchsortedfirst(cumsum(mind), u * total) with the blocked running sums
-__global__ void pp_pick_kernel(const float* __restrict__ mind, int64_t n,
-                               const double* __restrict__ bsum, const double* __restrict__ u, int i,
-                               int64_t* __restrict__ idx) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const int64_t nb = (n + PP_CHUNK - 1) / PP_CHUNK;
-  double total = 0.0;
-  for (int64_t b = 0; b < nb; ++b) total += bsum[b];
-  const double thr = u[i] * total;
-  double acc = 0.0;
-  int64_t pick = n - 1;
-  for (int64_t b = 0; b < nb; ++b) {
-    if (acc + bsum[b] >= thr) {
-      const int64_t e = min(n, (b + 1) * PP_CHUNK);
-      double a2 = acc;
-      for (int64_t j = b * PP_CHUNK; j < e; ++j) {
-        a2 += (double)mind[j];
-        if (a2 >= thr) {
-          pick = j;
-          break;
+// exclusive prefix of v over the block; the total in `total`
+__device__ __forceinline__ long long pp_block_scan(long long v, long long* red, long long& total) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  long long inc = v;
+  for (int o = 1; o < 32; o <<= 1) {
+    const long long x = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += x;
+  }
+  __syncthreads();
+  if (lane == 31) red[w] = inc;
+  __syncthreads();
+  long long base = 0;
+  total = 0;
+  for (int i = 0; i < PP_PTS / 32; ++i) {
+    if (i < w) base += red[i];
+    total += red[i];
+  }
+  return base + inc - v;
+}
+
+// The ordered running sum acc, acc + x(0), ... of `count` terms >= 0, each
+// thread holding a contiguous run [i0, i1) of them: the total (in `total`), and
+// through `visit(i, partial sum before i, partial sum through i)` every partial
+// sum of the thread's run, when all of them are exact in FP64; false otherwise.
+template <typename Term, typename Visit>
+__device__ bool pp_exact_sum(double acc, int64_t i0, int64_t i1, Term term, int* redi, long long* redl, double& total,
+                             Visit visit) {
+  constexpr int NO_LOW = 1 << 20;
+  int low = NO_LOW;
+  bool ok = true;
+  auto part = [&](double v, long long& m, int& e) {
+    ok &= pp_split(v, m, e);
+    if (m) low = min(low, e);
+  };
+  long long m;
+  int e;
+  part(acc, m, e);
+  for (int64_t i = i0; i < i1; ++i) part(term(i), m, e);
+  low = pp_block_min(ok ? low : -NO_LOW, redi);
+  if (low == -NO_LOW) return false;
+  if (low == NO_LOW) low = 0;  // every term is zero
+  if (low < -1000) return false;
+  pp_split(acc, m, e);
+  const long long a0 = pp_units(m, e, low);
+  long long mine = 0;
+  ok = a0 >= 0;
+  for (int64_t i = i0; i < i1 && ok; ++i) {
+    pp_split(term(i), m, e);
+    const long long u = pp_units(m, e, low);
+    mine += u;
+    ok = u >= 0 && mine <= PP_EXACT;
+  }
+  if (!__syncthreads_and(ok)) return false;
+  long long sum;
+  long long run = a0 + pp_block_scan(mine, redl, sum);
+  if (a0 + sum > PP_EXACT) return false;  // at most 129 * 2^53: no overflow
+  const double unit = pp_pow2(low);
+  total = (double)(a0 + sum) * unit;
+  for (int64_t i = i0; i < i1; ++i) {
+    pp_split(term(i), m, e);
+    const long long next = run + pp_units(m, e, low);
+    visit(i, (double)run * unit, (double)next * unit);
+    run = next;
+  }
+  return true;
+}
+
+struct PpArgs {
+  const float* X;
+  int64_t n;
+  int d;
+  int i;              // the centroid to choose; idx[0 .. i) are chosen
+  int vec;            // rows are 16-byte aligned
+  const double* u;    // draws
+  int64_t* idx;
+  float* mind;        // [n]
+  double* bsum;       // [blocks]
+  unsigned* tickets;  // [blocks + 1], zero between steps
+};
+
+__global__ void __launch_bounds__(PP_PTS) pp_step_kernel(PpArgs a) {
+  extern __shared__ __align__(16) float pp_tile[];  // [PP_PTS][PP_STR], then the block's values
+  __shared__ float cs[PP_DC];
+  __shared__ int redi[PP_PTS / 32];
+  __shared__ long long redl[PP_PTS / 32];
+  __shared__ int s_last;
+  __shared__ long long s_pick;
+  __shared__ double s_acc;
+  const int t = threadIdx.x;
+  const int64_t n = a.n;
+  const int d = a.d;
+  const int64_t j0 = (int64_t)blockIdx.x * PP_PTS;
+  const int64_t j = j0 + t;
+  const float* c = a.X + a.idx[a.i - 1] * d;
+
+  // squared distances in the FP32 form (dimension order), rows staged with
+  // every load of a slice in flight; columns past d are zero on both sides
+  float s = 0.0f;
+  const int rows = (int)min((int64_t)PP_PTS, n - j0);
+  for (int c0 = 0; c0 < d; c0 += PP_DC) {
+    const int cw = min(PP_DC, d - c0);
+    __syncthreads();
+    if (a.vec) {
+      const int q = cw >> 2;
+      for (int e = t; e < PP_PTS * (PP_DC / 4); e += PP_PTS) {
+        const int r = e / (PP_DC / 4), cc = e % (PP_DC / 4);
+        float* dst = pp_tile + r * PP_STR + cc * 4;
+        if (r < rows && cc < q) {
+          const uint32_t sa = (uint32_t)__cvta_generic_to_shared(dst);
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sa), "l"(a.X + (j0 + r) * d + c0 + cc * 4)
+                       : "memory");
+        } else {
+          *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
         }
       }
-      break;
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    } else {
+      for (int e = t; e < PP_PTS * PP_DC; e += PP_PTS) {
+        const int r = e / PP_DC, cc = e % PP_DC;
+        pp_tile[r * PP_STR + cc] = (r < rows && cc < cw) ? __ldg(a.X + (j0 + r) * d + c0 + cc) : 0.0f;
+      }
     }
-    acc += bsum[b];
+    if (t < PP_DC) cs[t] = t < cw ? __ldg(c + c0 + t) : 0.0f;
+    __syncthreads();
+    const float* row = pp_tile + t * PP_STR;
+#pragma unroll 4
+    for (int cc = 0; cc < cw; cc += 4) {
+      const float4 x = *reinterpret_cast<const float4*>(row + cc);
+      float v = __fsub_rn(x.x, cs[cc]);
+      s = __fmaf_rn(v, v, s);
+      v = __fsub_rn(x.y, cs[cc + 1]);
+      s = __fmaf_rn(v, v, s);
+      v = __fsub_rn(x.z, cs[cc + 2]);
+      s = __fmaf_rn(v, v, s);
+      v = __fsub_rn(x.w, cs[cc + 3]);
+      s = __fmaf_rn(v, v, s);
+    }
   }
-  idx[i] = pick;
+  if (j < n) {
+    const float old = a.i == 1 ? __int_as_float(0x7F800000) : a.mind[j];
+    a.mind[j] = s < old ? s : old;
+  }
+
+  // the last CTA of the block of points sums it
+  const int64_t nb = (n + PP_CHUNK - 1) / PP_CHUNK;
+  const int64_t blk = j0 / PP_CHUNK;
+  const int64_t b0 = blk * PP_CHUNK;
+  const int len = (int)min((int64_t)PP_CHUNK, n - b0);
+  __threadfence();
+  __syncthreads();
+  if (t == 0) {
+    const unsigned turn = (unsigned)((len + PP_PTS - 1) / PP_PTS);
+    s_last = atomicAdd(&a.tickets[blk], 1u) + 1u == turn;
+    if (s_last) a.tickets[blk] = 0u;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  float* vals = pp_tile;
+  constexpr int PER = PP_CHUNK / PP_PTS;
+  auto load_block = [&](int64_t first, int count) {
+    __syncthreads();
+    for (int e = t; e < count; e += PP_PTS) vals[e] = __ldcg(a.mind + first + e);
+    __syncthreads();
+  };
+  auto value = [&](int64_t e) { return (double)vals[e]; };
+  load_block(b0, len);
+  double total = 0.0;
+  if (!pp_exact_sum(0.0, min(len, t * PER), min(len, (t + 1) * PER), value, redi, redl, total,
+                    [](int64_t, double, double) {})) {
+    total = 0.0;
+    if (t == 0)
+      for (int e = 0; e < len; ++e) total += (double)vals[e];
+  }
+  if (t == 0) {
+    a.bsum[blk] = total;
+    __threadfence();
+    s_last = atomicAdd(&a.tickets[nb], 1u) + 1u == (unsigned)nb;
+    if (s_last) a.tickets[nb] = 0u;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+
+  // searchsortedfirst(cumsum(mind), u * total) with the blocked running sums
+  if (t == 0) {
+    s_pick = nb;
+    s_acc = 0.0;
+  }
+  __syncthreads();
+  const int64_t per = (nb + PP_PTS - 1) / PP_PTS;
+  const int64_t i0 = min(nb, t * per), i1 = min(nb, (t + 1) * per);
+  auto block_sum = [&](int64_t b) { return __ldcg(a.bsum + b); };
+  bool exact = pp_exact_sum(0.0, i0, i1, block_sum, redi, redl, total, [](int64_t, double, double) {});
+  double thr = a.u[a.i] * total;
+  if (exact) {
+    double unused;
+    pp_exact_sum(0.0, i0, i1, block_sum, redi, redl, unused, [&](int64_t b, double, double through) {
+      if (through >= thr) atomicMin(&s_pick, (long long)b);
+    });
+    __syncthreads();
+    const int64_t pb = s_pick;
+    pp_exact_sum(0.0, i0, i1, block_sum, redi, redl, unused, [&](int64_t b, double before, double) {
+      if (b == pb) s_acc = before;
+    });
+  } else if (t == 0) {
+    total = 0.0;
+    for (int64_t b = 0; b < nb; ++b) total += __ldcg(a.bsum + b);
+    thr = a.u[a.i] * total;
+    double acc = 0.0;
+    for (int64_t b = 0; b < nb; ++b) {
+      if (acc + __ldcg(a.bsum + b) >= thr) {
+        s_pick = b;
+        break;
+      }
+      acc += __ldcg(a.bsum + b);
+    }
+    s_acc = acc;
+    redl[0] = __double_as_longlong(thr);
+  }
+  __syncthreads();
+  if (!exact) thr = __longlong_as_double(redl[0]);
+  const int64_t pb = s_pick;
+  const double acc = s_acc;
+  if (pb >= nb) {
+    if (t == 0) a.idx[a.i] = n - 1;
+    return;
+  }
+  const int64_t f0 = pb * PP_CHUNK;
+  const int flen = (int)min((int64_t)PP_CHUNK, n - f0);
+  load_block(f0, flen);
+  if (t == 0) s_pick = n - 1;
+  __syncthreads();
+  if (!pp_exact_sum(acc, min(flen, t * PER), min(flen, (t + 1) * PER), value, redi, redl, total,
+                    [&](int64_t e, double, double through) {
+                      if (through >= thr) atomicMin(&s_pick, (long long)(f0 + e));
+                    }) &&
+      t == 0) {
+    double a2 = acc;
+    for (int e = 0; e < flen; ++e) {
+      a2 += (double)vals[e];
+      if (a2 >= thr) {
+        s_pick = f0 + e;
+        break;
+      }
+    }
+  }
+  __syncthreads();
+  if (t == 0) a.idx[a.i] = s_pick;
 }
 
 // ------------------------------------------------------------------ M-step
@@ -435,22 +669,20 @@ mann_status kmeans_assign_device(Context* ctx, cudaStream_t s, const float* X, i
 mann_status kmeanspp_device(Context* ctx, cudaStream_t s, const float* X, int64_t n, int d, int k,
                             int64_t first, const double* u_host, int64_t* idx_dev) {
   float* mind = nullptr;
-  double* bsum = nullptr;
-  double* u = nullptr;
+  double *bsum = nullptr, *u = nullptr;
+  unsigned* tickets = nullptr;
   const int64_t nb = ceil_div(n, PP_CHUNK);
   MANN_TRY(ctx->scratch_t(SLOT_KM_A, (size_t)n, &mind));
-  MANN_TRY(ctx->scratch_t(SLOT_KM_B, (size_t)nb, &bsum));
+  MANN_TRY(ctx->scratch_t(SLOT_KM_B, (size_t)nb * 2 + 1, &bsum));
+  tickets = reinterpret_cast<unsigned*>(bsum + nb);
   MANN_TRY(ctx->scratch_t(SLOT_KM_C, (size_t)k, &u));
   MANN_CUDA_TRY(cudaMemcpyAsync(u, u_host, sizeof(double) * k, cudaMemcpyHostToDevice, s));
   MANN_CUDA_TRY(cudaMemcpyAsync(idx_dev, &first, sizeof(int64_t), cudaMemcpyHostToDevice, s));
-  fill_inf_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, s>>>(mind, n);
-  MANN_CHECK_LAUNCH();
-  for (int i = 1; i < k; ++i) {
-    pp_update_kernel<<<(unsigned)ceil_div(n, 128), 128, 0, s>>>(X, n, d, idx_dev, i, mind);
-    MANN_CHECK_LAUNCH();
-    pp_block_sums_kernel<<<(unsigned)ceil_div(nb, 128), 128, 0, s>>>(mind, n, bsum);
-    MANN_CHECK_LAUNCH();
-    pp_pick_kernel<<<1, 32, 0, s>>>(mind, n, bsum, u, i, idx_dev);
+  MANN_CUDA_TRY(cudaMemsetAsync(tickets, 0, sizeof(unsigned) * (nb + 1), s));
+  PpArgs a{X, n, d, 0, (d % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0) ? 1 : 0, u, idx_dev, mind, bsum,
+           tickets};
+  for (a.i = 1; a.i < k; ++a.i) {
+    pp_step_kernel<<<(unsigned)ceil_div(n, PP_PTS), PP_PTS, sizeof(float) * PP_PTS * PP_STR, s>>>(a);
     MANN_CHECK_LAUNCH();
   }
   return MANN_OK;
