@@ -22,6 +22,11 @@ __device__ __forceinline__ uint64_t sub(uint64_t a, uint64_t b) {
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
+__device__ __forceinline__ uint64_t mul(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
 // a * b + c per lane, one rounding
 __device__ __forceinline__ uint64_t fma(uint64_t a, uint64_t b, uint64_t c) {
   uint64_t r;
