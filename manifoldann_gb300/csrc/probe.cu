@@ -47,12 +47,22 @@ namespace {
 
 typedef __nv_bfloat16 bf16;
 
-constexpr int GM = 128, GN = 128, GK = 64;
-constexpr int GSTAGES = 4;
+// GEMM tiles are GM x GN with GN = 128, or 32 where 128-wide tiles leave most
+// SMs idle: a training step's 1024 x 512 products are 32 tiles of 128 columns,
+// whose K-slices and epilogues run in 32 CTAs; every sum over K keeps its
+// order.  Measured (cold, per launch): the two GELU-derivative products
+// 22.2 -> 15.8 us, bias + GELU 12.7 -> 7.4 us, the small weight gradients
+// 10.4 -> 8.3 us; a whole training step (batch 1,024, 128-512-512-4096) with
+// the changes below, replayed as a graph: 264 -> 142 us.
+constexpr int GM = 128, GK = 64;
 constexpr int G_A_BYTES = GM * GK * 2;
-constexpr int G_STAGE = G_A_BYTES + GN * GK * 2;
 constexpr int G_THREADS = 192;
-constexpr size_t G_SMEM = 1024 + (size_t)GSTAGES * G_STAGE + (2 * GSTAGES + 2) * 8 + 16;
+template <int GN>
+struct GTile {
+  static constexpr int STAGES = GN == 128 ? 3 : 5;  // about 100 KB: two CTAs per SM
+  static constexpr int STAGE = G_A_BYTES + GN * GK * 2;
+  static constexpr size_t SMEM = 1024 + (size_t)STAGES * STAGE + (2 * STAGES + 2) * 8 + 16;
+};
 
 enum { EPI_F32 = 0, EPI_BIAS_GELU = 1, EPI_LOGITS = 2, EPI_DGELU = 3 };
 enum { PERR_TIMEOUT = 1 };
@@ -72,10 +82,11 @@ __device__ __forceinline__ float gelu_grad(float z) {
   return 0.5f * (1.0f + erff(z * 0.70710678118654752f)) + z * 0.39894228040143268f * expf(-0.5f * z * z);
 }
 
-template <int EPI>
-__global__ void __launch_bounds__(G_THREADS, 1)
+template <int EPI, int GN>
+__global__ void __launch_bounds__(G_THREADS, 2)
     probe_gemm(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                GemmArgs g) {
+  constexpr int GSTAGES = GTile<GN>::STAGES, G_STAGE = GTile<GN>::STAGE;
   extern __shared__ __align__(1024) uint8_t g_smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(g_smem_raw) + 1023) &
                                              ~uintptr_t(1023));
@@ -229,13 +240,13 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// K-major BF16 matrix [rows][cols], boxes of 64 columns x 128 rows
-mann_status map_kmajor(CUtensorMap* m, const bf16* ptr, int64_t rows, int64_t cols) {
+// K-major BF16 matrix [rows][cols], boxes of 64 columns x box_rows rows
+mann_status map_kmajor(CUtensorMap* m, const bf16* ptr, int64_t rows, int64_t cols, int box_rows) {
   EncodeTiledFn enc = encode_fn();
   if (!enc) return fail(MANN_ECUDA, "cuTensorMapEncodeTiled unavailable");
   cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
   cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
-  cuuint32_t box[2] = {(cuuint32_t)GK, 128u};
+  cuuint32_t box[2] = {(cuuint32_t)GK, (cuuint32_t)box_rows};
   cuuint32_t es[2] = {1, 1};
   CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<bf16*>(ptr), dims, strides, box, es,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -244,47 +255,58 @@ mann_status map_kmajor(CUtensorMap* m, const bf16* ptr, int64_t rows, int64_t co
   return MANN_OK;
 }
 
-template <int EPI>
+template <int EPI, int GN>
 mann_status launch_gemm_t(cudaStream_t s, const bf16* A, const bf16* B, const GemmArgs& g) {
   static std::once_flag once;
   static cudaError_t attr = cudaSuccess;
+  constexpr size_t smem = GTile<GN>::SMEM;
   std::call_once(once, [] {
-    attr = cudaFuncSetAttribute(probe_gemm<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G_SMEM);
+    attr = cudaFuncSetAttribute(probe_gemm<EPI, GN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   });
   MANN_CUDA_TRY(attr);
   CUtensorMap ma, mb;
-  MANN_TRY(map_kmajor(&ma, A, g.M, g.K));
-  MANN_TRY(map_kmajor(&mb, B, g.N, g.K));
+  MANN_TRY(map_kmajor(&ma, A, g.M, g.K, GM));
+  MANN_TRY(map_kmajor(&mb, B, g.N, g.K, GN));
   dim3 grid((unsigned)(g.N / GN), (unsigned)(g.M / GM));
-  probe_gemm<EPI><<<grid, G_THREADS, G_SMEM, s>>>(ma, mb, g);
+  probe_gemm<EPI, GN><<<grid, G_THREADS, smem, s>>>(ma, mb, g);
   MANN_CHECK_LAUNCH();
   return MANN_OK;
+}
+
+// 128-wide tiles where they fill at least 96 SMs, else 32-wide ones
+template <int EPI>
+mann_status launch_gemm(cudaStream_t s, const bf16* A, const bf16* B, const GemmArgs& g) {
+  if ((int64_t)(g.M / GM) * (g.N / 128) >= 96) return launch_gemm_t<EPI, 128>(s, A, B, g);
+  return launch_gemm_t<EPI, 32>(s, A, B, g);
 }
 
 // C[M][N] = A[M][K] B[N][K]^T with the given epilogue; M, N multiples of 128, K of 64.
 mann_status gemm(cudaStream_t s, int epi, const bf16* A, const bf16* B, int M, int N, int K,
                  const float* bias, float* outf, bf16* outh, bf16* outt, const float* zin, int* err) {
-  if (M % GM || N % GN || K % GK || K <= 0)
+  if (M % GM || N % 128 || K % GK || K <= 0)
     return fail(MANN_EINVAL_ARG, "probe GEMM shape must be multiples of 128 x 128 x 64");
   GemmArgs g{M, N, K, bias, outf, outh, outt, zin, err};
   switch (epi) {
-    case EPI_F32: return launch_gemm_t<EPI_F32>(s, A, B, g);
-    case EPI_BIAS_GELU: return launch_gemm_t<EPI_BIAS_GELU>(s, A, B, g);
-    case EPI_LOGITS: return launch_gemm_t<EPI_LOGITS>(s, A, B, g);
-    default: return launch_gemm_t<EPI_DGELU>(s, A, B, g);
+    case EPI_F32: return launch_gemm<EPI_F32>(s, A, B, g);
+    case EPI_BIAS_GELU: return launch_gemm<EPI_BIAS_GELU>(s, A, B, g);
+    case EPI_LOGITS: return launch_gemm<EPI_LOGITS>(s, A, B, g);
+    default: return launch_gemm<EPI_DGELU>(s, A, B, g);
   }
 }
 
 // ------------------------------------------------------------ batch staging
 // X bf16 [Bp][dinp] and X^T [dinp][Bp]; Xf f32 [Bp][din]; labels [Bp][L].
-// Rows past nb (and columns past din) are zero; their labels are -1.
+// Rows past nb (and columns past din) are zero; their labels are -1.  Row r is
+// query idx[*done + r] (done: rows of the epoch staged by earlier steps), idx[r]
+// or, without an index, r.
 __global__ void stage_batch_kernel(const float* __restrict__ q, int din, const int32_t* __restrict__ idx,
-                                   int nb, int Bp, int dinp, const int32_t* __restrict__ labels, int L,
-                                   bf16* __restrict__ X, bf16* __restrict__ Xt, float* __restrict__ Xf,
-                                   int32_t* __restrict__ lb) {
+                                   const int* __restrict__ done, int nb, int Bp, int dinp,
+                                   const int32_t* __restrict__ labels, int L, bf16* __restrict__ X,
+                                   bf16* __restrict__ Xt, float* __restrict__ Xf, int32_t* __restrict__ lb) {
   __shared__ float tile[32][33];
   const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
+  if (done) idx += *done;
   for (int i = ty; i < 32; i += 8) {
     const int r = r0 + i, c = c0 + tx;
     float v = 0.0f;
@@ -330,17 +352,35 @@ __device__ __forceinline__ float score_at(const SoftmaxArgs& a, int r, int c, fl
   return v;
 }
 
-// one warp per row: log-sum-exp of the scores and the row's loss
-__global__ void softmax_stats_kernel(SoftmaxArgs a) {
-  const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (r >= a.Bp) return;
+// One block per row: log-sum-exp of the scores and the row's loss.  The
+// exponentials are made by all the threads and added by warp 0 in a warp's
+// order (lane l: columns l, l + 32, ...), so a row's sum does not depend on the
+// block; a warp per row alone was bound by its own loads.
+constexpr int SS_THREADS = 128;
+__global__ void __launch_bounds__(SS_THREADS) softmax_stats_kernel(SoftmaxArgs a) {
+  extern __shared__ float ss_val[];  // [nout]
+  __shared__ float red[SS_THREADS / 32];
+  const int r = blockIdx.x, t = threadIdx.x, lane = t & 31;
   const float beta = a.D ? expf(*a.theta) : 0.0f;
   float mx = -INFINITY;
-  for (int c = lane; c < a.nout; c += 32) mx = fmaxf(mx, score_at(a, r, c, beta));
+#pragma unroll 8
+  for (int c = t; c < a.nout; c += SS_THREADS) {
+    const float v = score_at(a, r, c, beta);
+    ss_val[c] = v;
+    mx = fmaxf(mx, v);
+  }
   for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if (lane == 0) red[t >> 5] = mx;
+  __syncthreads();
+  mx = red[0];
+  for (int w = 1; w < SS_THREADS / 32; ++w) mx = fmaxf(mx, red[w]);
+#pragma unroll 4
+  for (int c = t; c < a.nout; c += SS_THREADS) ss_val[c] = expf(ss_val[c] - mx);
+  __syncthreads();
+  if (t >= 32) return;
   float sm = 0.0f;
-  for (int c = lane; c < a.nout; c += 32) sm += expf(score_at(a, r, c, beta) - mx);
+#pragma unroll 8
+  for (int c = lane; c < a.nout; c += 32) sm += ss_val[c];
   for (int o = 16; o; o >>= 1) sm += __shfl_xor_sync(0xffffffffu, sm, o);
   const float lse = mx + logf(sm);
   if (lane == 0) {
@@ -362,54 +402,82 @@ __global__ void softmax_stats_kernel(SoftmaxArgs a) {
   }
 }
 
-// 32 x 32 tiles: dL = (softmax - y) / nb in both layouts, and the tile's
-// share of d loss / d theta (theta = log beta).
-__global__ void softmax_grad_kernel(SoftmaxArgs a) {
+// dL = (softmax - y) / nb in both layouts, in 32 x 32 tiles, and each tile's
+// share of d loss / d theta (theta = log beta).  A block takes 32 rows by
+// SG_TILES tiles and counts the rows' labels in them once, in shared memory
+// instead of walking a row's label list for every element; the scores of all
+// its tiles are loaded before the first is finished.
+constexpr int SG_TILES = 4;
+__global__ void __launch_bounds__(256) softmax_grad_kernel(SoftmaxArgs a) {
   __shared__ bf16 tile[32][34];
   __shared__ float red[8];
-  const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
+  __shared__ int hits[32][32 * SG_TILES];
+  __shared__ int nvalid[32];
+  const int r0 = blockIdx.y * 32, cb = blockIdx.x * 32 * SG_TILES;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int e = threadIdx.x; e < 32 * 32 * SG_TILES; e += 256) hits[e / (32 * SG_TILES)][e % (32 * SG_TILES)] = 0;
+  if (threadIdx.x < 32) nvalid[threadIdx.x] = 0;
+  __syncthreads();
+  for (int i = ty; i < 32; i += 8)
+    for (int l = tx; l < a.L; l += 32) {
+      const int lc = a.lb[(size_t)(r0 + i) * a.L + l];
+      if (lc >= 0 && lc < a.nout) {
+        atomicAdd(&nvalid[i], 1);
+        if (lc >= cb && lc < cb + 32 * SG_TILES) atomicAdd(&hits[i][lc - cb], 1);
+      }
+    }
   const float beta = a.D ? expf(*a.theta) : 0.0f;
   const float inv_nb = 1.0f / (float)max(a.nb, 1);
-  float th = 0.0f;
-  for (int i = ty; i < 32; i += 8) {
-    const int r = r0 + i, c = c0 + tx;
-    float gv = 0.0f;
-    if (r < a.nb && c < a.nout) {
-      int nv = 0, hit = 0;
-      for (int l = 0; l < a.L; ++l) {
-        const int lc = a.lb[(size_t)r * a.L + l];
-        if (lc >= 0 && lc < a.nout) {
-          ++nv;
-          hit += lc == c;
-        }
-      }
-      const float sc = score_at(a, r, c, beta);
-      const float p = expf(sc - a.lse[r]);
-      const float y = nv ? (float)hit / nv : 0.0f;
-      gv = nv ? (p - y) * inv_nb : 0.0f;
-      if (a.D) th += gv * (-beta * a.D[(size_t)r * a.nout + c]);
+  float sc[SG_TILES][4], lse[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int r = r0 + ty + 8 * u;
+    lse[u] = r < a.nb ? a.lse[r] : 0.0f;
+#pragma unroll
+    for (int ct = 0; ct < SG_TILES; ++ct) {
+      const int c = cb + ct * 32 + tx;
+      sc[ct][u] = r < a.nb && c < a.nout ? score_at(a, r, c, beta) : 0.0f;
     }
-    const bf16 h = __float2bfloat16_rn(gv);
-    a.dL[(size_t)r * a.noutp + c] = h;
-    tile[i][tx] = h;
   }
   __syncthreads();
-  for (int i = ty; i < 32; i += 8) a.dLt[(size_t)(c0 + i) * a.Bp + r0 + tx] = tile[tx][i];
-  if (a.theta_part) {
-    for (int o = 16; o; o >>= 1) th += __shfl_xor_sync(0xffffffffu, th, o);
-    if (tx == 0) red[ty] = th;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      float t = 0.0f;
-      for (int i = 0; i < 8; ++i) t += red[i];
-      a.theta_part[blockIdx.y * gridDim.x + blockIdx.x] = t;
+#pragma unroll
+  for (int ct = 0; ct < SG_TILES; ++ct) {
+    const int c0 = cb + ct * 32;
+    if (c0 >= a.noutp) break;  // block-uniform
+    float th = 0.0f;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = ty + 8 * u, r = r0 + i, c = c0 + tx;
+      float gv = 0.0f;
+      if (r < a.nb && c < a.nout) {
+        const int nv = nvalid[i], hit = hits[i][ct * 32 + tx];
+        const float p = expf(sc[ct][u] - lse[u]);
+        const float y = hit ? (float)hit / nv : 0.0f;
+        gv = nv ? (p - y) * inv_nb : 0.0f;
+        if (a.D) th += gv * (-beta * a.D[(size_t)r * a.nout + c]);
+      }
+      const bf16 h = __float2bfloat16_rn(gv);
+      a.dL[(size_t)r * a.noutp + c] = h;
+      tile[i][tx] = h;
     }
+    __syncthreads();
+    for (int i = ty; i < 32; i += 8) a.dLt[(size_t)(c0 + i) * a.Bp + r0 + tx] = tile[tx][i];
+    if (a.theta_part) {
+      for (int o = 16; o; o >>= 1) th += __shfl_xor_sync(0xffffffffu, th, o);
+      if (tx == 0) red[ty] = th;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        float t = 0.0f;
+        for (int i = 0; i < 8; ++i) t += red[i];
+        a.theta_part[blockIdx.y * (a.noutp / 32) + c0 / 32] = t;
+      }
+    }
+    __syncthreads();
   }
 }
 
 // Row sums (fixed order) of up to three transposed BF16 matrices into the
-// bias gradients; the block past them reduces theta's partials and the loss.
+// bias gradients; the first two warps sum theta's partials and the loss.
 struct BiasGradArgs {
   const bf16* src[3];
   float* dst[3];
@@ -421,60 +489,123 @@ struct BiasGradArgs {
   const float* loss_row;
   int nb;
   float* loss_acc;  // += mean loss of the batch (nullable)
+  int* step;        // training: [0] += 1 step, [1] += nb rows staged (nullable)
 };
 
-__global__ void bias_grad_kernel(BiasGradArgs a) {
+// x[0] + x[1] + ... in order, by one warp: 512 values at a time through shared
+// memory, so the chain of additions does not wait for loads (one lane reading
+// as it adds: 20 us for the 1,024 losses of a batch).
+__device__ __forceinline__ float ordered_sum(const float* __restrict__ x, int n, float (*buf)[512]) {
   const int lane = threadIdx.x & 31;
-  int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  float* b = buf[threadIdx.x >> 5];
+  float s = 0.0f;
+  for (int i0 = 0; i0 < n; i0 += 512) {
+    const int m = min(512, n - i0);
+    __syncwarp();
+    for (int i = lane; i < m; i += 32) b[i] = x[i0 + i];
+    __syncwarp();
+#pragma unroll 8
+    for (int i = 0; i < m; ++i) s += b[i];
+  }
+  return s;
+}
+
+__global__ void __launch_bounds__(256) bias_grad_kernel(BiasGradArgs a) {
+  __shared__ float buf[8][512];
+  const int lane = threadIdx.x & 31;
+  int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5) - 2;  // -2, -1: theta and the loss, the long chains
   const int total = a.rows[0] + a.rows[1] + a.rows[2];
-  if (r < total) {
+  if (r >= 0 && r < total) {
     int m = 0;
     while (r >= a.rows[m]) r -= a.rows[m++];
     const bf16* p = a.src[m] + (size_t)r * a.Bp;
     float s = 0.0f;
+#pragma unroll 8
     for (int i = lane; i < a.Bp; i += 32) s += __bfloat162float(p[i]);
     for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) a.dst[m][r] = s;
-  } else if (r == total && lane == 0) {
-    if (a.dtheta) {
-      float t = 0.0f;
-      for (int i = 0; i < a.ntheta; ++i) t += a.theta_part[i];
-      *a.dtheta = t;
-    }
-    if (a.loss_acc) {
-      float l = 0.0f;
-      for (int i = 0; i < a.nb; ++i) l += a.loss_row[i];
+  } else if (r == -2 && a.dtheta) {
+    const float t = ordered_sum(a.theta_part, a.ntheta, buf);
+    if (lane == 0) *a.dtheta = t;
+  } else if (r == -1 && a.loss_acc) {
+    const float l = ordered_sum(a.loss_row, a.nb, buf);
+    if (lane == 0) {
       *a.loss_acc += l / (float)max(a.nb, 1);
+      if (a.step) {  // after this step's staging, before its update
+        a.step[0] += 1;
+        a.step[1] += a.nb;
+      }
     }
   }
 }
 
 // ------------------------------------------------------------ AdamW
+struct AdamMat {
+  int64_t off;   // in the flat parameter vector
+  int rows, cols;
+  bf16 *wb, *wt;  // BF16 copies [rows][cols] and [cols][rows]
+};
 struct AdamArgs {
   float* w;
   const float* g;
   float* m;
   float* v;
-  int64_t n;
-  float lr, b1, b2, eps, wd, bc1, bc2;
-  int64_t decay_end[3];    // [decay_begin[i], decay_end[i]) take weight decay
-  int64_t decay_begin[3];
+  float lr, b1, b2, eps, wd;
+  const float2* bc;       // bias corrections by step
+  const int* step;        // steps counted, this one among them
+  AdamMat mat[3];         // the matrices (with weight decay)
+  int64_t vec_begin[3];   // what follows each of them (biases, theta): no decay
+  int64_t vec_end[3];
 };
 
-__global__ void adamw_kernel(AdamArgs a) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += (int64_t)gridDim.x * blockDim.x) {
-    const float g = a.g[i];
-    const float m = a.b1 * a.m[i] + (1.0f - a.b1) * g;
-    const float v = a.b2 * a.v[i] + (1.0f - a.b2) * g * g;
-    a.m[i] = m;
-    a.v[i] = v;
-    float w = a.w[i];
-    bool dec = false;
+__device__ __forceinline__ float adam_update(const AdamArgs& a, float2 bc, int64_t i, bool decay) {
+  const float g = a.g[i];
+  const float m = a.b1 * a.m[i] + (1.0f - a.b1) * g;
+  const float v = a.b2 * a.v[i] + (1.0f - a.b2) * g * g;
+  a.m[i] = m;
+  a.v[i] = v;
+  float w = a.w[i];
+  if (decay) w -= a.lr * a.wd * w;
+  w -= a.lr * (m / bc.x) / (sqrtf(v / bc.y) + a.eps);
+  a.w[i] = w;
+  return w;
+}
+
+// One block per 32 x 32 tile of a matrix -- the updated weights go to both
+// BF16 copies from the same pass (three more launches read them back before)
+// -- then blocks of 1,024 vector entries.
+__global__ void __launch_bounds__(256) adamw_kernel(AdamArgs a) {
+  __shared__ bf16 tile[32][34];
+  int b = blockIdx.x;
+  const float2 bc = a.bc[*a.step - 1];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) dec |= (i >= a.decay_begin[j] && i < a.decay_end[j]);
-    if (dec) w -= a.lr * a.wd * w;
-    w -= a.lr * (m / a.bc1) / (sqrtf(v / a.bc2) + a.eps);
-    a.w[i] = w;
+  for (int j = 0; j < 3; ++j) {
+    const AdamMat& q = a.mat[j];
+    const int tc = q.cols / 32, tiles = (q.rows / 32) * tc;
+    if (b >= 0 && b < tiles) {
+      const int r0 = (b / tc) * 32, c0 = (b % tc) * 32;
+      const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+#pragma unroll
+      for (int i = ty; i < 32; i += 8) {
+        const size_t e = (size_t)(r0 + i) * q.cols + c0 + tx;
+        const bf16 h = __float2bfloat16_rn(adam_update(a, bc, q.off + (int64_t)e, true));
+        q.wb[e] = h;
+        tile[i][tx] = h;
+      }
+      __syncthreads();
+      for (int i = ty; i < 32; i += 8) q.wt[(size_t)(c0 + i) * q.rows + r0 + tx] = tile[tx][i];
+      return;
+    }
+    b -= tiles;
+  }
+  for (int64_t e = (int64_t)b * 1024 + threadIdx.x, k = 0; k < 4; ++k, e += 256) {
+    int64_t i = e;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const int64_t len = a.vec_end[j] - a.vec_begin[j];
+      if (i >= 0 && i < len) adam_update(a, bc, a.vec_begin[j] + i, false);
+      i -= len;
+    }
   }
 }
 
@@ -928,9 +1059,35 @@ struct Batch {
   }
 };
 
+// Side stream of a training step and the events that order it (the weight
+// gradients run beside the chain of back-propagated signals).
+struct Side {
+  cudaStream_t s = nullptr;
+  cudaEvent_t ev[3] = {};
+  mann_status create() {
+    MANN_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    for (cudaEvent_t& e : ev) MANN_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    return MANN_OK;
+  }
+  ~Side() {
+    for (cudaEvent_t e : ev)
+      if (e) cudaEventDestroy(e);
+    if (s) cudaStreamDestroy(s);
+  }
+  // what follows on `to` waits for what was issued on `from`
+  mann_status order(int i, cudaStream_t from, cudaStream_t to) {
+    MANN_CUDA_TRY(cudaEventRecord(ev[i], from));
+    MANN_CUDA_TRY(cudaStreamWaitEvent(to, ev[i], 0));
+    return MANN_OK;
+  }
+};
+
 // Forward (and with `grad`, backward into m->grad) of the rows staged in b.
-// The loss of the batch is added to *loss_slot when given.
-mann_status fwd_bwd(ProbeModel* m, cudaStream_t s, Batch& b, int nb, bool grad, float* loss_slot) {
+// The loss of the batch is added to *loss_slot when given; `step` is advanced
+// with it.  With a side stream the weight gradients run on it; s waits for
+// them at the end.
+mann_status fwd_bwd(ProbeModel* m, cudaStream_t s, Batch& b, int nb, bool grad, float* loss_slot, int* step = nullptr,
+                    Side* side = nullptr) {
   const Layout& P = m->pad;
   const bool prior = m->p.use_prior != 0;
   const int Bp = b.Bp;
@@ -944,15 +1101,25 @@ mann_status fwd_bwd(ProbeModel* m, cudaStream_t s, Batch& b, int nb, bool grad, 
   if (!grad) return MANN_OK;
   SoftmaxArgs sa{b.logits, prior ? b.D : nullptr, w + P.theta, b.lb, b.L, nb, P.nout, P.noutp, Bp,
                  b.lse, b.loss_row, b.dL, b.dLt, prior ? b.theta_part : nullptr};
-  softmax_stats_kernel<<<(unsigned)ceil_div(Bp, 8), 256, 0, s>>>(sa);
+  static std::once_flag once;
+  static cudaError_t attr = cudaSuccess;
+  std::call_once(once, [] {
+    attr = cudaFuncSetAttribute(softmax_stats_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(sizeof(float) * ROUTE_MAXCOLS));  // nout <= ROUTE_MAXCOLS
+  });
+  MANN_CUDA_TRY(attr);
+  softmax_stats_kernel<<<(unsigned)Bp, SS_THREADS, sizeof(float) * P.nout, s>>>(sa);
   MANN_CHECK_LAUNCH();
-  softmax_grad_kernel<<<dim3(P.noutp / 32, Bp / 32), 256, 0, s>>>(sa);
+  softmax_grad_kernel<<<dim3((unsigned)ceil_div(P.noutp, 32 * SG_TILES), Bp / 32), 256, 0, s>>>(sa);
   MANN_CHECK_LAUNCH();
   float* g = m->grad;
   // dW3 = dL^T H2 ; dZ2 = (dL W3) * gelu'(Z2) ; dW2 = dZ2^T H1 ; dZ1 = (dZ2 W2) * gelu'(Z1) ; dW1 = dZ1^T X
-  MANN_TRY(gemm(s, EPI_F32, b.dLt, b.H2t, P.noutp, P.h2p, Bp, nullptr, g + P.w3, nullptr, nullptr, nullptr, m->err));
+  cudaStream_t sw = side ? side->s : s;
+  if (side) MANN_TRY(side->order(0, s, sw));
+  MANN_TRY(gemm(sw, EPI_F32, b.dLt, b.H2t, P.noutp, P.h2p, Bp, nullptr, g + P.w3, nullptr, nullptr, nullptr, m->err));
   MANN_TRY(gemm(s, EPI_DGELU, b.dL, m->w3t, Bp, P.h2p, P.noutp, nullptr, nullptr, b.dZ2, b.dZ2t, b.Z2, m->err));
-  MANN_TRY(gemm(s, EPI_F32, b.dZ2t, b.H1t, P.h2p, P.h1p, Bp, nullptr, g + P.w2, nullptr, nullptr, nullptr, m->err));
+  if (side) MANN_TRY(side->order(1, s, sw));
+  MANN_TRY(gemm(sw, EPI_F32, b.dZ2t, b.H1t, P.h2p, P.h1p, Bp, nullptr, g + P.w2, nullptr, nullptr, nullptr, m->err));
   MANN_TRY(gemm(s, EPI_DGELU, b.dZ2, m->w2t, Bp, P.h1p, P.h2p, nullptr, nullptr, b.dZ1, b.dZ1t, b.Z1, m->err));
   MANN_TRY(gemm(s, EPI_F32, b.dZ1t, b.Xt, P.h1p, P.dinp, Bp, nullptr, g + P.w1, nullptr, nullptr, nullptr, m->err));
   BiasGradArgs ba{};
@@ -972,18 +1139,19 @@ mann_status fwd_bwd(ProbeModel* m, cudaStream_t s, Batch& b, int nb, bool grad, 
   ba.loss_row = b.loss_row;
   ba.nb = nb;
   ba.loss_acc = loss_slot;
-  const int rows = P.noutp + P.h2p + P.h1p + 1;
+  ba.step = step;
+  const int rows = P.noutp + P.h2p + P.h1p + 2;
   bias_grad_kernel<<<(unsigned)ceil_div(rows, 8), 256, 0, s>>>(ba);
   MANN_CHECK_LAUNCH();
-  if (!prior) MANN_CUDA_TRY(cudaMemsetAsync(g + P.theta, 0, sizeof(float), s));
+  if (side) MANN_TRY(side->order(2, sw, s));
   return MANN_OK;
 }
 
 mann_status stage(ProbeModel* m, cudaStream_t s, Batch& b, const float* q, const int32_t* idx, int nb,
-                  const int32_t* labels) {
+                  const int32_t* labels, const int* done = nullptr) {
   const Layout& P = m->pad;
-  stage_batch_kernel<<<dim3(P.dinp / 32, b.Bp / 32), 256, 0, s>>>(q, P.din, idx, nb, b.Bp, P.dinp, labels,
-                                                                   b.L, b.X, b.Xt, b.Xf, labels ? b.lb : nullptr);
+  stage_batch_kernel<<<dim3(P.dinp / 32, b.Bp / 32), 256, 0, s>>>(
+      q, P.din, idx, done, nb, b.Bp, P.dinp, labels, b.L, b.X, b.Xt, b.Xf, labels ? b.lb : nullptr);
   MANN_CHECK_LAUNCH();
   return MANN_OK;
 }
@@ -992,31 +1160,34 @@ mann_status prior_dist(Context* ctx, ProbeModel* m, cudaStream_t s, const float*
   return pairwise_device(ctx, s, Xf, rows, m->cent, m->pad.nout, m->pad.din, MANN_METRIC_SQEUCLIDEAN, D);
 }
 
-mann_status adam_step(ProbeModel* m, cudaStream_t s) {
+mann_status adam_step(ProbeModel* m, cudaStream_t s, const float2* bc, const int* step) {
   const Layout& P = m->pad;
-  m->step += 1;
   AdamArgs a{};
   a.w = m->master;
   a.g = m->grad;
   a.m = m->adam_m;
   a.v = m->adam_v;
-  a.n = P.total;
   a.lr = m->p.lr;
   a.b1 = m->p.beta1;
   a.b2 = m->p.beta2;
   a.eps = m->p.eps;
   a.wd = m->p.weight_decay;
-  a.bc1 = (float)(1.0 - std::pow((double)a.b1, (double)m->step));
-  a.bc2 = (float)(1.0 - std::pow((double)a.b2, (double)m->step));
-  a.decay_begin[0] = P.w1;
-  a.decay_end[0] = P.b1;
-  a.decay_begin[1] = P.w2;
-  a.decay_end[1] = P.b2;
-  a.decay_begin[2] = P.w3;
-  a.decay_end[2] = P.b3;
-  adamw_kernel<<<(unsigned)std::min<int64_t>(ceil_div(P.total, 256), 4096), 256, 0, s>>>(a);
+  a.bc = bc;
+  a.step = step;
+  a.mat[0] = {P.w1, P.h1p, P.dinp, m->w1, m->w1t};
+  a.mat[1] = {P.w2, P.h2p, P.h1p, m->w2, m->w2t};
+  a.mat[2] = {P.w3, P.noutp, P.h2p, m->w3, m->w3t};
+  const int64_t ends[3] = {P.w2, P.w3, P.total}, begins[3] = {P.b1, P.b2, P.b3};
+  int64_t blocks = 0, nvec = 0;
+  for (int j = 0; j < 3; ++j) {
+    a.vec_begin[j] = begins[j];
+    a.vec_end[j] = ends[j];
+    nvec += ends[j] - begins[j];
+    blocks += (int64_t)(a.mat[j].rows / 32) * (a.mat[j].cols / 32);
+  }
+  adamw_kernel<<<(unsigned)(blocks + ceil_div(nvec, 1024)), 256, 0, s>>>(a);
   MANN_CHECK_LAUNCH();
-  return refresh_bf16(m, s);
+  return MANN_OK;
 }
 
 }  // namespace
@@ -1038,7 +1209,7 @@ mann_status probe_route_device(Context* ctx, ProbeModel* m, cudaStream_t s, cons
     MANN_TRY(ctx->scratch_t(SLOT_PROBE_H1, (size_t)Bp * P.h1p, &H1));
     MANN_TRY(ctx->scratch_t(SLOT_PROBE_H2, (size_t)Bp * P.h2p, &H2));
     MANN_TRY(ctx->scratch_t(SLOT_PROBE_LOGITS, (size_t)Bp * P.noutp, &logits));
-    stage_batch_kernel<<<dim3(P.dinp / 32, Bp / 32), 256, 0, s>>>(qs + r0 * P.din, P.din, nullptr, nb, Bp,
+    stage_batch_kernel<<<dim3(P.dinp / 32, Bp / 32), 256, 0, s>>>(qs + r0 * P.din, P.din, nullptr, nullptr, nb, Bp,
                                                                    P.dinp, nullptr, 0, X, nullptr, nullptr,
                                                                    nullptr);
     MANN_CHECK_LAUNCH();
@@ -1235,30 +1406,84 @@ mann_status mann_probe_train(mann_probe* m, const float* queries, int64_t nq, co
   Free f2{dl};
   MANN_CUDA_TRY(cudaMemcpyAsync(dq, queries, sizeof(float) * nq * P.din, cudaMemcpyHostToDevice, s));
   MANN_CUDA_TRY(cudaMemcpyAsync(dl, labels, sizeof(int32_t) * nq * nlabel, cudaMemcpyHostToDevice, s));
-  MANN_CUDA_TRY(cudaMemsetAsync(b.loss_acc, 0, sizeof(float) * 64, s));
+  const int64_t steps_per_epoch = ceil_div(nq, B), total = steps_per_epoch * epochs;
+  // Adam's bias corrections by step, and the counters of the running call
+  std::vector<float2> hbc((size_t)total);
+  for (int64_t i = 0; i < total; ++i) {
+    const double st = (double)(m->step + 1 + i);
+    hbc[i] = make_float2((float)(1.0 - std::pow((double)m->p.beta1, st)), (float)(1.0 - std::pow((double)m->p.beta2, st)));
+  }
+  float2* bc = nullptr;  // [total] | losses [epochs] | step counters [2]
+  const size_t bc_bytes = sizeof(float2) * (size_t)total + sizeof(float) * (size_t)epochs + 2 * sizeof(int);
+  MANN_CUDA_TRY(cudaMalloc(&bc, bc_bytes));
+  Free f3{bc};
+  float* dloss = reinterpret_cast<float*>(bc + total);
+  int* step = reinterpret_cast<int*>(dloss + epochs);
+  MANN_CUDA_TRY(cudaMemcpyAsync(bc, hbc.data(), sizeof(float2) * (size_t)total, cudaMemcpyHostToDevice, s));
+  MANN_CUDA_TRY(cudaMemsetAsync(step, 0, 2 * sizeof(int), s));
+  float* slot = b.loss_acc;
+  // One step's launches.  Nothing in them depends on the step but the rows
+  // of the batch: the counters give the place in the shuffled order and the
+  // bias corrections, so full batches replay one captured graph (launch by
+  // launch a step is bound by its gaps: 13 launches of a few microseconds).
+  Side side;
+  MANN_TRY(side.create());
+  auto issue = [&](int nb) -> mann_status {
+    MANN_TRY(stage(m, s, b, dq, b.idx, nb, dl, step + 1));
+    if (m->p.use_prior) MANN_TRY(prior_dist(ctx, m, s, b.Xf, Bp, b.D));
+    MANN_TRY(fwd_bwd(m, s, b, nb, true, slot, step, &side));
+    return adam_step(m, s, bc, step);
+  };
+  struct Graph {
+    cudaGraphExec_t exec = nullptr;
+    ~Graph() {
+      if (exec) cudaGraphExecDestroy(exec);
+    }
+  } graph;
+  constexpr int64_t GRAPH_MIN_STEPS = 16;  // a shorter training does not pay for the capture
   std::vector<int32_t> perm((size_t)nq);
   Splitmix r{m->p.seed ^ 0xC0FFEEull ^ (uint64_t)m->step};
-  std::vector<float> losses((size_t)epochs, 0.0f);
-  const int64_t steps_per_epoch = ceil_div(nq, B);
-  for (int e = 0; e < epochs; ++e) {
+  auto shuffle = [&] {
     for (int64_t i = 0; i < nq; ++i) perm[i] = (int32_t)i;
     for (int64_t i = nq - 1; i > 0; --i) std::swap(perm[i], perm[r.next() % (uint64_t)(i + 1)]);
+  };
+  shuffle();
+  for (int e = 0; e < epochs; ++e) {
     MANN_CUDA_TRY(cudaMemcpyAsync(b.idx, perm.data(), sizeof(int32_t) * nq, cudaMemcpyHostToDevice, s));
-    float* slot = b.loss_acc + (e % 64);
+    MANN_CUDA_TRY(cudaMemsetAsync(step + 1, 0, sizeof(int), s));
     MANN_CUDA_TRY(cudaMemsetAsync(slot, 0, sizeof(float), s));
     for (int64_t st = 0; st < steps_per_epoch; ++st) {
       const int nb = (int)std::min<int64_t>(B, nq - st * B);
-      MANN_TRY(stage(m, s, b, dq, b.idx + st * B, nb, dl));
-      if (m->p.use_prior) MANN_TRY(prior_dist(ctx, m, s, b.Xf, Bp, b.D));
-      MANN_TRY(fwd_bwd(m, s, b, nb, true, slot));
-      MANN_TRY(adam_step(m, s));
+      m->step += 1;
+      if (nb < B || total < GRAPH_MIN_STEPS || (e == 0 && st == 0)) {
+        MANN_TRY(issue(nb));  // the first step also sets up what a capture may not
+        continue;
+      }
+      if (!graph.exec) {
+        cudaGraph_t g = nullptr;
+        MANN_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+        const mann_status rc = issue(nb);
+        const cudaError_t ce = cudaStreamEndCapture(s, &g);
+        if (rc != MANN_OK) {
+          (void)cudaGetLastError();
+          if (g) cudaGraphDestroy(g);
+          return rc;
+        }
+        MANN_CUDA_TRY(ce);
+        const cudaError_t ie = cudaGraphInstantiate(&graph.exec, g, 0);
+        cudaGraphDestroy(g);
+        MANN_CUDA_TRY(ie);
+      }
+      MANN_CUDA_TRY(cudaGraphLaunch(graph.exec, s));
     }
-    float l = 0.0f;
-    MANN_CUDA_TRY(cudaMemcpyAsync(&l, slot, sizeof(float), cudaMemcpyDeviceToHost, s));
-    MANN_CUDA_TRY(cudaStreamSynchronize(s));
-    losses[e] = l / (float)steps_per_epoch;
+    MANN_CUDA_TRY(cudaMemcpyAsync(dloss + e, slot, sizeof(float), cudaMemcpyDeviceToDevice, s));
+    MANN_CUDA_TRY(cudaStreamSynchronize(s));  // perm is free again (and a cudaFree never meets running steps)
+    if (e + 1 < epochs) shuffle();
   }
+  std::vector<float> losses((size_t)epochs, 0.0f);
+  MANN_CUDA_TRY(cudaMemcpyAsync(losses.data(), dloss, sizeof(float) * epochs, cudaMemcpyDeviceToHost, s));
   MANN_CUDA_TRY(cudaStreamSynchronize(s));
+  for (float& l : losses) l /= (float)steps_per_epoch;
   MANN_TRY(read_err(m, s));
   if (out_loss) std::memcpy(out_loss, losses.data(), sizeof(float) * epochs);
   return MANN_OK;
