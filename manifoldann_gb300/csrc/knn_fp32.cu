@@ -22,6 +22,7 @@ namespace {
 constexpr int K1_THREADS = 256;
 constexpr int K1_BN = 128;  // points per tile
 constexpr int K1_DK = 16;   // dimensions per shared-memory stage
+constexpr uint32_t K1_NAN = 0x7FFFFFFFu;  // every NaN distance in the threshold tests
 constexpr int K1_QCAP = 32;  // candidates a row's queue holds
 constexpr int K1_DRAIN = 8;  // ... and the number at which it is merged into the row's list
 constexpr unsigned FULL = 0xFFFFFFFFu;
@@ -409,7 +410,7 @@ __device__ __forceinline__ void k1_body(const float* __restrict__ base, int64_t 
         const int r = tile_row<TQ>(ty, e >> 3);
         float v = select_tree<TQ * TN>(acc, e);
         if constexpr (METRIC == MANN_METRIC_EUCLIDEAN) v = __fsqrt_rn(v);
-        const uint32_t lim = thr[r], vb = __float_as_uint(v);
+        const uint32_t lim = thr[r], vb = v == v ? __float_as_uint(v) : K1_NAN;
         if (first ? vb < lim : vb <= lim) {
           const int pos = atomicAdd(&qcnt[r], 1);
           if (pos >= K1_QCAP) continue;  // full: tested again in the next round
@@ -431,7 +432,7 @@ __device__ __forceinline__ void k1_body(const float* __restrict__ base, int64_t 
           qcnt[r] = 0;
           if (kth != KEY_NONE) {
             const float t = key_dist(kth);
-            thr[r] = __float_as_uint(t);
+            thr[r] = t == t ? __float_as_uint(t) : K1_NAN;
             // sqrt(v) < t needs v < t^2 (1 + 2^-21): a square at or past that
             // bound has a larger root however both round
             if constexpr (METRIC == MANN_METRIC_EUCLIDEAN)

@@ -65,3 +65,12 @@ def test_not_a_number_sorts_last(gpu_lib, orc):
     base = rng.standard_normal((700, 5)).astype(np.float32)
     base[rng.choice(700, 650, replace=False), 2] = np.nan
     check(orc, base, rng.standard_normal((90, 5)).astype(np.float32), 64, 0)
+
+
+@pytest.mark.parametrize("k", [5, 32, 42, 64, 100])
+def test_rows_of_nothing_but_nan_take_the_lowest_ids(gpu_lib, orc, k):
+    # a zero query has a NaN cosine to every point: more equal candidates than a queue holds
+    rng = np.random.default_rng(8)
+    q = rng.standard_normal((70, 9)).astype(np.float32)
+    q[::3] = 0.0
+    check(orc, rng.standard_normal((700, 9)).astype(np.float32), q, k, 2)
