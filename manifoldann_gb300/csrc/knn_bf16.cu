@@ -70,10 +70,20 @@ struct Stg {
 
 constexpr int AUG = 24;                              // norm-fold columns read after a BF16 row's main part
 constexpr int LIST = 32;                             // candidates kept per query row
-constexpr int SEED_SAMPLE = 2048;                    // points sampled by the seed pass
-constexpr int SEED_DEPTH = 5;                        // the seed is the 5th smallest (chunk minimum)
+constexpr int SEED_SAMPLE = 2048;                    // most points sampled by the seed pass
+// densest sample: every 8th point (below 16 SEED_SAMPLE points; without a seed
+// the 10,000 x 4,096 x 128 routing of an inverted file, all admissions, took
+// 375 us, with one and two epilogue sets 120)
+constexpr int SEED_STRIDE = 8;
+constexpr int SEED_MIN_SAMPLE = 256;                 // fewer sampled points: no seed pass
+constexpr int SEED_KEEP = 12;                        // smallest half-chunk minima kept (the seed is one of them)
 constexpr int KREQ_MAX_BF16 = 24;                    // largest k (k+1 for graphs) of this form
-constexpr int SEG_SEED_STRIDE = 32;                  // many point sets: the seed pass samples every 32nd point
+// Many point sets: the seed pass samples every 8th point of each set.  With the
+// rank that so dense a sample allows the main pass admits a third fewer points
+// than with the 5th minimum of every 32nd (graphs of 24 clouds of 2k-50k points
+// in 32-d, with the items cut by cost and the views read ahead: main pass 12.9
+// -> 6.2 ms, seed pass 0.18 -> 0.39 ms)
+constexpr int SEG_SEED_STRIDE = 8;
 constexpr uint32_t TMEM_COLS = 2 * BN;               // double-buffered accumulator
 // Bands and CTA pairs are built but not selected: on one GB300 the
 // phase-aligned single-band walk beat 48 MB bands (1M x 128: 8.2 vs 11.8 ms;
@@ -116,36 +126,55 @@ __global__ void scale_rows_kernel(const float* __restrict__ x, int64_t n, int d,
 
 // Column means over an evenly spaced sample of rows (rows <= CENTRE_ROWS).
 // Any centre keeps the distances unchanged; a good one shrinks the BF16
-// values and their rounding.  Block (32 columns x 32 row groups): FP32
-// partial sums per thread, FP64 across groups.  With row norms (cosine) each
-// sampled row is scaled by one reciprocal, computed once per block: the
-// centre only needs to be near the unit rows' mean, not their exact bits.
+// values and their rounding.  Block (32 columns x 32 row groups) of one of
+// CENTRE_PARTS shares of the rows: FP32 partial sums per thread, FP64 across
+// groups; the last share's block of a column group adds the shares in order
+// (one share per column group left most SMs idle: 18 us at 784 columns).  With
+// row norms (cosine) each sampled row is scaled by one reciprocal, computed
+// once per block: the centre only needs to be near the unit rows' mean, not
+// their exact bits.
 constexpr int CENTRE_ROWS = 4096;
-__global__ void centre_sample_kernel(const float* __restrict__ x, int64_t n, int d, int64_t stride,
-                                     int64_t rows, float* __restrict__ mu, const float* __restrict__ rnorm) {
+constexpr int CENTRE_PARTS = 8;
+__global__ void __launch_bounds__(1024)
+    centre_sample_kernel(const float* __restrict__ x, int64_t n, int d, int64_t stride, int64_t rows,
+                         double* __restrict__ shares, unsigned* __restrict__ tickets, float* __restrict__ mu,
+                         const float* __restrict__ rnorm) {
   __shared__ double part[32][33];
-  __shared__ float inv[CENTRE_ROWS];
+  __shared__ float inv[CENTRE_ROWS / CENTRE_PARTS + 1];
+  __shared__ int last;
   const int cl = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + cl;
+  const int64_t r0 = rows * blockIdx.y / CENTRE_PARTS, r1 = rows * (blockIdx.y + 1) / CENTRE_PARTS;
   if (rnorm) {
-    for (int64_t i = threadIdx.x; i < rows; i += blockDim.x) {
+    for (int64_t i = r0 + threadIdx.x; i < r1; i += blockDim.x) {
       const float nr = __fsqrt_rn(rnorm[i * stride]);
-      inv[i] = nr > 0.0f ? 1.0f / nr : 0.0f;
+      inv[i - r0] = nr > 0.0f ? 1.0f / nr : 0.0f;
     }
     __syncthreads();
   }
   float s = 0.0f;
   if (c < d)
-    for (int64_t i = g; i < rows; i += 32) {
-      const float xv = x[(i * stride) * d + c];
-      s += rnorm ? xv * inv[i] : xv;
+#pragma unroll 8
+    for (int64_t i = r0 + g; i < r1; i += 32) {
+      const float xv = __ldg(x + (i * stride) * d + c);
+      s += rnorm ? xv * inv[i - r0] : xv;
     }
   part[g][cl] = (double)s;
   __syncthreads();
-  if (g == 0 && c < d) {
+  if (g == 0) {
     double t = 0.0;
     for (int i = 0; i < 32; ++i) t += part[i][cl];
-    mu[c] = (float)(t / (double)rows);
+    if (c < d) shares[(size_t)blockIdx.y * d + c] = t;
+    __threadfence();
+    __syncwarp();
+    if (cl == 0) last = atomicAdd(&tickets[blockIdx.x], 1u) + 1u == CENTRE_PARTS;
+    __syncwarp();
+    if (last && c < d) {
+      __threadfence();
+      t = 0.0;
+      for (int i = 0; i < CENTRE_PARTS; ++i) t += __ldcg(shares + (size_t)i * d + c);
+      mu[c] = (float)(t / (double)rows);
+    }
   }
 }
 
@@ -161,73 +190,111 @@ __device__ __forceinline__ void scale_candidate(int i, float m, float* sc, float
   else { *sc = 1.0f; *mc = rintf(m); }
 }
 
-// per candidate: sum over sampled rows of ||cv - bf16(cv)||^2 / ||cv||^2; the
-// first candidate also records the sampled max |x - mu| (float bits, integer
-// max) in score[NUM_SCALES] for the FP16 form's scale
-__global__ void scale_probe_kernel(const float* __restrict__ x, int64_t n, int d,
-                                   const float* __restrict__ mu, int64_t stride,
-                                   double* __restrict__ score, const float* __restrict__ rnorm) {
-  const int lane = threadIdx.x & 31;
-  const int64_t row = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * stride;
-  const int cand = blockIdx.y;
-  if (row >= n) return;
-  float rr = 0.0f, cc = 0.0f, mx = 0.0f;  // a heuristic score: FP32 is plenty
-  float inv = 1.0f;  // unit rows: one reciprocal of the row's norm (a heuristic needs no exact division)
-  if (rnorm) {
-    const float nr = __fsqrt_rn(rnorm[row]);
-    inv = nr > 0.0f ? 1.0f / nr : 0.0f;
-  }
-  for (int c = lane; c < d; c += 32) {
-    float sc, mc;
-    scale_candidate(cand, mu[c], &sc, &mc);
-    const float cv = __fmul_rn(sc, __fsub_rn(x[row * d + c] * inv, mc));
-    const float bv = __bfloat162float(__float2bfloat16_rn(cv));
-    rr = __fmaf_rn(cv - bv, cv - bv, rr);
-    cc = __fmaf_rn(cv, cv, cc);
-    mx = fmaxf(mx, fabsf(cv));
+// Per candidate: the sum over the sampled rows (a warp per row) of ||cv -
+// bf16(cv)||^2 / ||cv||^2, and the sampled max |x - mu| (float bits, integer
+// max) in score[NUM_SCALES] for the FP16 form's scale.  The last block picks
+// the candidate with the smallest residual (moving off the plain mean only for
+// a clear win), replaces mu by its centre, publishes its scale and clears the
+// rows' bounds that the conversion will fill.
+struct ScaleOut {
+  float* mu;
+  float* scale;
+  int* inexact;
+  float* f16_scale;
+  BaseMax* bmax;
+  double* score;      // [NUM_SCALES + 1], zero
+  unsigned* ticket;   // zero
+  int64_t nrows;      // sampled rows
+};
+__global__ void __launch_bounds__(256)
+    scale_probe_kernel(const float* __restrict__ x, int64_t n, int d, int64_t stride, const float* __restrict__ rnorm,
+                       ScaleOut o) {
+  __shared__ float wsum[8][NUM_SCALES + 1];
+  __shared__ int last, best;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t row = ((int64_t)blockIdx.x * 8 + w) * stride;
+  float rr[NUM_SCALES] = {}, cc[NUM_SCALES] = {}, mx = 0.0f;  // a heuristic score: FP32 is plenty
+  if (row < n) {
+    float inv = 1.0f;  // unit rows: one reciprocal of the row's norm (a heuristic needs no exact division)
+    if (rnorm) {
+      const float nr = __fsqrt_rn(rnorm[row]);
+      inv = nr > 0.0f ? 1.0f / nr : 0.0f;
+    }
+#pragma unroll 4
+    for (int c = lane; c < d; c += 32) {
+      const float xv = __ldg(x + row * d + c) * inv, m = o.mu[c];
+#pragma unroll
+      for (int i = 0; i < NUM_SCALES; ++i) {
+        float sc, mc;
+        scale_candidate(i, m, &sc, &mc);
+        const float cv = __fmul_rn(sc, __fsub_rn(xv, mc));
+        const float bv = __bfloat162float(__float2bfloat16_rn(cv));
+        rr[i] = __fmaf_rn(cv - bv, cv - bv, rr[i]);
+        cc[i] = __fmaf_rn(cv, cv, cc[i]);
+        if (i == 0) mx = fmaxf(mx, fabsf(cv));
+      }
+    }
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    rr += __shfl_xor_sync(FULL, rr, o);
-    cc += __shfl_xor_sync(FULL, cc, o);
-    mx = fmaxf(mx, __shfl_xor_sync(FULL, mx, o));
+  for (int s = 16; s > 0; s >>= 1) {
+#pragma unroll
+    for (int i = 0; i < NUM_SCALES; ++i) {
+      rr[i] += __shfl_xor_sync(FULL, rr[i], s);
+      cc[i] += __shfl_xor_sync(FULL, cc[i], s);
+    }
+    mx = fmaxf(mx, __shfl_xor_sync(FULL, mx, s));
   }
   if (lane == 0) {
-    atomicAdd(&score[cand], cc > 0.0f ? (double)rr / (double)cc : 0.0);
-    if (cand == 0 && mx < 3.0e38f) atomicMax(reinterpret_cast<unsigned*>(&score[NUM_SCALES]), __float_as_uint(mx));
-  }
-}
-
-// pick the candidate with the smallest residual (moving off the plain mean
-// only for a clear win), replace mu by its centre and publish its scale
-__global__ void choose_scale_kernel(const double* __restrict__ score, float* __restrict__ mu, int d,
-                                    float* __restrict__ scale_out, int* __restrict__ inexact, int64_t nrows,
-                                    float* __restrict__ f16_scale_out) {
-  __shared__ int best;
-  if (threadIdx.x == 0) {
-    // FP16 form: the power of two that takes the sampled max |x - mu| into
-    // [2^11, 2^12) -- 16x below FP16's largest value for rows off the sample
-    // (a value that still overflows saturates, and its row's bound says so)
-    const float smax = __uint_as_float(*reinterpret_cast<const unsigned*>(&score[NUM_SCALES]));
-    int e = 0;
-    if (smax > 0.0f) frexpf(smax, &e);  // smax in [2^(e-1), 2^e)
-    *f16_scale_out = ldexpf(1.0f, max(-120, min(120, 12 - e)));
-    int b = 0;
-    for (int i = 1; i < NUM_SCALES; ++i)
-      if (score[i] < 0.25 * score[b]) b = i;
-    best = b;
-    // the mean squared relative residual of the sampled rows: ~2^-18 for data
-    // off any grid, ~1e-14 for grid data that FP32 centring merely blurs
-    *inexact = score[b] > 1e-10 * (double)(nrows > 0 ? nrows : 1) ? 1 : 0;
-    float sc, mc;
-    scale_candidate(b, 0.0f, &sc, &mc);
-    *scale_out = sc;
+#pragma unroll
+    for (int i = 0; i < NUM_SCALES; ++i) wsum[w][i] = cc[i] > 0.0f ? rr[i] / cc[i] : 0.0f;
+    wsum[w][NUM_SCALES] = mx < 3.0e38f ? mx : 0.0f;
   }
   __syncthreads();
+  if (threadIdx.x <= NUM_SCALES) {
+    if (threadIdx.x < NUM_SCALES) {
+      double t = 0.0;
+      for (int i = 0; i < 8; ++i) t += (double)wsum[i][threadIdx.x];
+      atomicAdd(&o.score[threadIdx.x], t);
+    } else {
+      float t = 0.0f;
+      for (int i = 0; i < 8; ++i) t = fmaxf(t, wsum[i][NUM_SCALES]);
+      atomicMax(reinterpret_cast<unsigned*>(&o.score[NUM_SCALES]), __float_as_uint(t));
+    }
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(o.ticket, 1u) + 1u == gridDim.x;
+    if (last) {
+      __threadfence();
+      // FP16 form: the power of two that takes the sampled max |x - mu| into
+      // [2^11, 2^12) -- 16x below FP16's largest value for rows off the sample
+      // (a value that still overflows saturates, and its row's bound says so)
+      const float smax = __uint_as_float(__ldcg(reinterpret_cast<const unsigned*>(&o.score[NUM_SCALES])));
+      int e = 0;
+      if (smax > 0.0f) frexpf(smax, &e);  // smax in [2^(e-1), 2^e)
+      *o.f16_scale = ldexpf(1.0f, max(-120, min(120, 12 - e)));
+      double sc[NUM_SCALES];
+      for (int i = 0; i < NUM_SCALES; ++i) sc[i] = __ldcg(&o.score[i]);
+      int b = 0;
+      for (int i = 1; i < NUM_SCALES; ++i)
+        if (sc[i] < 0.25 * sc[b]) b = i;
+      best = b;
+      // the mean squared relative residual of the sampled rows: ~2^-18 for data
+      // off any grid, ~1e-14 for grid data that FP32 centring merely blurs
+      *o.inexact = sc[b] > 1e-10 * (double)(o.nrows > 0 ? o.nrows : 1) ? 1 : 0;
+      float s0, m0;
+      scale_candidate(b, 0.0f, &s0, &m0);
+      *o.scale = s0;
+      *o.bmax = BaseMax{0u, 0u, 0u, 0u};
+    }
+  }
+  __syncthreads();
+  if (!last) return;
   for (int c = threadIdx.x; c < d; c += blockDim.x) {
     float sc, mc;
-    scale_candidate(best, mu[c], &sc, &mc);
-    mu[c] = mc;
+    scale_candidate(best, o.mu[c], &sc, &mc);
+    o.mu[c] = mc;
   }
 }
 
@@ -471,6 +538,7 @@ struct Walk {
   int nbands;
   int span;       // most CTAs any (band, query block) run touches
   int qrows;      // query rows per query block (BM, or 2 BM for CTA pairs)
+  const int64_t* cuts;  // segmented pass: CTA c holds items [cuts[c], cuts[c + 1])
 };
 
 __host__ __device__ __forceinline__ int band_len(const Walk& w, int b) {
@@ -506,11 +574,13 @@ struct TileItem {
   int64_t q0, qend;   // first row of the block; end of its set's rows
   int64_t t0, tend;   // first point of the tile; end of its set's points
   int64_t run_first;  // first item of this block's run
+  int64_t run_cta;    // the CTA holding it
 };
 
-// a block's run of items: first item and count (segmented merge)
+// a block's run of items: first item and count, and the CTAs that hold them (segmented merge)
 struct RunInfo {
   int64_t first, len;
+  int c0, c1;
 };
 
 struct MainArgs {
@@ -531,7 +601,7 @@ struct MainArgs {
   const float* seed;  // per query: admit only est' below this (NULL = no seed)
   uint64_t* partial;  // [nq][smax][L]
   int* err;
-  int seedmode;       // keep the SEED_DEPTH smallest 32-column chunk minima instead of points
+  int seedmode;       // keep the `depth` (<= SEED_KEEP) smallest minima of 32 (1) or 16 (2) columns, no points
   int f16;            // FP16 main columns: their MMAs read FP16 (the fold step stays BF16)
 };
 
@@ -540,6 +610,7 @@ struct MainArgs {
 struct ItemView {
   int64_t q0, qend, c0, cend, run_first;
   int slot_base;  // band * span (banded walk), 0 (segmented)
+  int run_cta;    // segmented: the CTA holding the run's first item
 };
 
 __device__ __forceinline__ ItemView view_item(const MainArgs& a, int64_t item, int qrows) {
@@ -552,6 +623,7 @@ __device__ __forceinline__ ItemView view_item(const MainArgs& a, int64_t item, i
     v.cend = ti.tend;
     v.run_first = ti.run_first;
     v.slot_base = 0;
+    v.run_cta = (int)ti.run_cta;
   } else {
     int qb, t, band;
     item_pos(a.w, item, qb, t, band);
@@ -561,6 +633,7 @@ __device__ __forceinline__ ItemView view_item(const MainArgs& a, int64_t item, i
     v.cend = a.n;
     v.run_first = run_begin(a.w, band, qb);
     v.slot_base = band * a.w.span;
+    v.run_cta = -1;
   }
   return v;
 }
@@ -822,40 +895,43 @@ __device__ __forceinline__ void epi_chunk(const uint32_t (&v)[32], float nbv, fl
   }
 }
 
-// Seed-pass form of epi_chunk: the row keeps, in registers and sorted, the
-// SEED_DEPTH smallest minima of its 32-column chunks (keyed by the chunk's
-// first column, so each comes from a distinct point).  SEED_DEPTH distinct
-// points lie at or below the SEED_DEPTH-th of them, so it bounds the row's
-// SEED_DEPTH-th smallest est' over the sample from above -- all a seed needs.
+// Seed pass: the row keeps, in registers and sorted, the `rank` smallest
+// minima of its 32-column chunks, or of their 16-column halves (small samples
+// have few chunks).  Each comes from a distinct point, so r distinct points lie
+// at or below the r-th of them: it bounds the row's r-th smallest est' over the
+// sample from above -- all a seed needs.
+__device__ __forceinline__ void seed_keep(float (&top)[SEED_KEEP], float c, int rank) {
+#pragma unroll
+  for (int i = 0; i < SEED_KEEP; ++i) {
+    const float t = fminf(top[i], c);
+    c = fmaxf(top[i], c);
+    top[i] = t;
+    if (i == 5 && rank <= 6) return;  // uniform
+  }
+}
+
 template <bool FP8>
 __device__ __forceinline__ void seed_chunk(const uint32_t (&v)[32], float nbv, float csv, float rs,
-                                           uint64_t (&top)[SEED_DEPTH], uint32_t col0) {
-  float m4[8];
+                                           float (&top)[SEED_KEEP], int rank) {
+  float mn[2];
 #pragma unroll
-  for (int j4 = 0; j4 < 8; ++j4) {
-    float e4[4];
+  for (int h = 0; h < 2; ++h) {
+    float m4[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int j = 4 * j4 + u;
-      const float coef = FP8 ? rs * __shfl_sync(FULL, csv, j) : -2.0f;
-      e4[u] = __fmaf_rn(coef, __uint_as_float(v[j]), __shfl_sync(FULL, nbv, j));
-    }
-    m4[j4] = fminf(fminf(e4[0], e4[1]), fminf(e4[2], e4[3]));
-  }
-  const float mn = fminf(fminf(fminf(m4[0], m4[1]), fminf(m4[2], m4[3])),
-                         fminf(fminf(m4[4], m4[5]), fminf(m4[6], m4[7])));
-  uint64_t c = make_key(mn, col0);
-  if (c < top[SEED_DEPTH - 1]) {
-    top[SEED_DEPTH - 1] = c;
+    for (int j4 = 0; j4 < 4; ++j4) {
+      float e4[4];
 #pragma unroll
-    for (int i = SEED_DEPTH - 1; i > 0; --i) {
-      const uint64_t lo = top[i - 1], hi = top[i];
-      if (hi < lo) {
-        top[i - 1] = hi;
-        top[i] = lo;
+      for (int u = 0; u < 4; ++u) {
+        const int j = 16 * h + 4 * j4 + u;
+        const float coef = FP8 ? rs * __shfl_sync(FULL, csv, j) : -2.0f;
+        e4[u] = __fmaf_rn(coef, __uint_as_float(v[j]), __shfl_sync(FULL, nbv, j));
       }
+      m4[j4] = fminf(fminf(e4[0], e4[1]), fminf(e4[2], e4[3]));
     }
+    mn[h] = fminf(fminf(m4[0], m4[1]), fminf(m4[2], m4[3]));
   }
+  seed_keep(top, mn[0], rank);
+  seed_keep(top, mn[1], rank);
 }
 
 // In the plain-rescan instances, candidates of the norm-folded epilogue wait
@@ -873,10 +949,11 @@ constexpr int ADMIT_Q = 2;
 // the epilogue takes each 16-column half-chunk's largest accumulator from the
 // max-reduction form of the TMEM load
 constexpr bool LD_RED = true;
-// single-matrix passes of at most this many K-stages per tile run the
-// three-stage, two-set instance (their MMA per tile is short against the
-// epilogue's work)
-constexpr int SHORT_K_STAGES = 3;
+// single-matrix passes of at most this many K-stages per tile run two epilogue
+// sets (three stages for long lists): their MMA per tile is short against the
+// epilogue's work (290k x 256 cosine, five stages: main pass 2.25 -> 1.73 ms;
+// thirteen stages, 60k x 784, lose with two sets)
+constexpr int SHORT_K_STAGES = 5;
 // points per work item of the batched form's exact fallback scan
 constexpr int64_t FB_CHUNK = 4096;
 
@@ -962,21 +1039,25 @@ __device__ __forceinline__ void epi_chunk_fold(uint32_t (&v)[32], int nvalid, fl
   }
 }
 
-// Seed-pass form of epi_chunk_fold (the chunk minimum of est = -2 max(acc)).
-__device__ __forceinline__ void seed_chunk_fold(uint32_t (&v)[32], int nvalid, float rmax,
-                                                uint64_t (&top)[SEED_DEPTH], uint32_t col0) {
-  uint64_t c = make_key(-2.0f * chunk_max(v, nvalid, rmax), col0);
-  if (c < top[SEED_DEPTH - 1]) {
-    top[SEED_DEPTH - 1] = c;
+// Seed-pass form of epi_chunk_fold (the half-chunk minima of est = -2 max(acc)).
+__device__ __forceinline__ void seed_chunk_fold(uint32_t (&v)[32], int nvalid, float (&rmax)[2],
+                                                float (&top)[SEED_KEEP], int rank, bool halves) {
+  float m[2] = {rmax[0], rmax[1]};
+  if (!LD_RED || nvalid < 32) {
 #pragma unroll
-    for (int i = SEED_DEPTH - 1; i > 0; --i) {
-      const uint64_t lo = top[i - 1], hi = top[i];
-      if (hi < lo) {
-        top[i - 1] = hi;
-        top[i] = lo;
-      }
+    for (int h = 0; h < 2; ++h) {
+      m[h] = __int_as_float(0xFF800000);  // -inf: est = +inf
+#pragma unroll
+      for (int j = 16 * h; j < 16 * h + 16; ++j)
+        if (j < nvalid) m[h] = fmaxf(m[h], __uint_as_float(v[j]));
     }
   }
+  if (!halves) {
+    seed_keep(top, -2.0f * fmaxf(m[0], m[1]), rank);
+    return;
+  }
+  seed_keep(top, -2.0f * m[0], rank);
+  seed_keep(top, -2.0f * m[1], rank);
 }
 
 // Shared-memory footprint of k2_main<CAP, NSETS>.
@@ -1013,7 +1094,11 @@ static_assert(k2_smem_bytes<false>(24, 2, 3) <= 232448 && k2_smem_bytes<false>(3
 // commits arrive on the stage and accumulator barriers of both CTAs, and both
 // CTAs' epilogue warps release an accumulator on the even CTA's barrier.  The
 // work unit (a walk item) is then one pair tile and `a.w.grid` counts pairs.
-template <int CAP, int NSETS, bool PAIR, bool FP8, bool GROUPED = false, int NST = 0>
+//
+// SEED: the seed pass, whose epilogue keeps minima instead of points (an
+// instance of its own: the two epilogues side by side in one cost the main
+// passes 1 %).
+template <int CAP, int NSETS, bool PAIR, bool FP8, bool GROUPED = false, int NST = 0, bool SEED = false>
 __global__ void __launch_bounds__(64 + 128 * NSETS, 1)
     k2_main(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
             MainArgs a) {
@@ -1038,8 +1123,8 @@ __global__ void __launch_bounds__(64 + 128 * NSETS, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = PAIR ? ptx::cluster_ctarank() : 0u;
   const int cta = PAIR ? (int)ptx::cluster_id_x() : (int)blockIdx.x;  // work unit: pair or CTA
-  const int64_t it0 = chunk_begin(cta, a.w.work, a.w.grid);
-  const int64_t it1 = chunk_begin(cta + 1, a.w.work, a.w.grid);
+  const int64_t it0 = a.w.cuts ? a.w.cuts[cta] : chunk_begin(cta, a.w.work, a.w.grid);
+  const int64_t it1 = a.w.cuts ? a.w.cuts[cta + 1] : chunk_begin(cta + 1, a.w.work, a.w.grid);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -1078,8 +1163,13 @@ __global__ void __launch_bounds__(64 + 128 * NSETS, 1)
       uint32_t it = 0;
       bool ok = true;
       const uint32_t full0 = PAIR ? ptx::mapa(ptx::smem_u32(&full_bar[0]), 0) : 0u;  // even CTA's full_bar[0]
+      // segmented passes (GROUPED instances) read an item's view from memory:
+      // one tile ahead; the banded walk computes it
+      ItemView vn{};
+      if (GROUPED && it1 > it0) vn = view_item(a, walk_item(it0, it1, a.w, 0), QROWS);
       for (int64_t st = 0; st < it1 - it0 && ok; ++st) {
-        const ItemView v = view_item(a, walk_item(it0, it1, a.w, st), QROWS);
+        const ItemView v = GROUPED ? vn : view_item(a, walk_item(it0, it1, a.w, st), QROWS);
+        if (GROUPED && st + 1 < it1 - it0) vn = view_item(a, walk_item(it0, it1, a.w, st + 1), QROWS);
         for (int kb = 0; kb < a.nkb; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
@@ -1193,9 +1283,9 @@ __global__ void __launch_bounds__(64 + 128 * NSETS, 1)
       gmax[g] = 0;
       gidx[g] = 8 * g;
     }
-    uint64_t top[SEED_DEPTH];
+    float top[SEED_KEEP];
 #pragma unroll
-    for (int i = 0; i < SEED_DEPTH; ++i) top[i] = KEY_NONE;
+    for (int i = 0; i < SEED_KEEP; ++i) top[i] = INF;
     int tcount = 0;
     int64_t cur_run = -1, cur_q0 = 0, cur_qend = 0;
     int seg_slot = 0;
@@ -1207,15 +1297,15 @@ __global__ void __launch_bounds__(64 + 128 * NSETS, 1)
     const int64_t row0 = (int64_t)rank * BM;  // this CTA's rows inside a work unit's query block
     const uint32_t tempty0 = PAIR ? ptx::mapa(ptx::smem_u32(&tempty_bar[0]), 0) : 0u;
     auto flush = [&](int64_t q0_, int64_t qend_, int slot_) {
-      if (a.seedmode) {
+      if constexpr (SEED) {
         const int64_t gq = q0_ + row0 + row;
         if (gq < qend_) {
           uint64_t* dst = a.partial + (gq * a.smax + slot_) * LIST;
 #pragma unroll
-          for (int i = 0; i < SEED_DEPTH; ++i) dst[i] = top[i];
+          for (int i = 0; i < SEED_KEEP; ++i) dst[i] = make_key(top[i], (uint32_t)i);
         }
 #pragma unroll
-        for (int i = 0; i < SEED_DEPTH; ++i) top[i] = KEY_NONE;
+        for (int i = 0; i < SEED_KEEP; ++i) top[i] = INF;
         return;
       }
       __syncwarp();
@@ -1247,8 +1337,11 @@ __global__ void __launch_bounds__(64 + 128 * NSETS, 1)
       }
     };
     if (it1 > it0) fetch_norms(0);
+    ItemView vn{};  // as the producer's
+    if (GROUPED && it1 > it0) vn = view_item(a, walk_item(it0, it1, a.w, 0), QROWS);
     for (int64_t st = 0; st < it1 - it0; ++st, ++tcount) {
-      const ItemView v = view_item(a, walk_item(it0, it1, a.w, st), QROWS);
+      const ItemView v = GROUPED ? vn : view_item(a, walk_item(it0, it1, a.w, st), QROWS);
+      if (GROUPED && st + 1 < it1 - it0) vn = view_item(a, walk_item(it0, it1, a.w, st + 1), QROWS);
       if (v.run_first != cur_run) {
         if (cur_run >= 0) {
           // flush the finished segment's lists (every set, even one that saw no candidate)
@@ -1258,7 +1351,8 @@ __global__ void __launch_bounds__(64 + 128 * NSETS, 1)
         cur_run = v.run_first;
         cur_q0 = v.q0;
         cur_qend = v.qend;
-        seg_slot = (v.slot_base + (cta - cta_of(v.run_first, a.w.work, a.w.grid))) * NSETS + set;
+        const int cta0 = v.run_cta >= 0 ? v.run_cta : cta_of(v.run_first, a.w.work, a.w.grid);
+        seg_slot = (v.slot_base + (cta - cta0)) * NSETS + set;
         const int64_t gq = v.q0 + row0 + row;
         seed_key = (a.seed != nullptr && gq < v.qend) ? make_key(a.seed[gq], 0u) : KEY_NONE;
         if constexpr (FP8) rs = gq < v.qend ? __ldg(&a.qscale[gq]) : 0.0f;
@@ -1302,15 +1396,15 @@ __global__ void __launch_bounds__(64 + 128 * NSETS, 1)
         ld_chunk(ch + 1, vb, mb);
         if constexpr (FP8) {
           const float cs_a = pick(csc, ch);
-          if (a.seedmode)
-            seed_chunk<FP8>(va, pick(nbc, ch), cs_a, rs, top, (uint32_t)(col0 + ch * 32));
+          if constexpr (SEED)
+            seed_chunk<FP8>(va, pick(nbc, ch), cs_a, rs, top, a.depth);
           else
             epi_chunk<FP8, GROUPED>(va, pick(nbc, ch), cs_a, rs, mylist, thr_key, thr_est, lslot, nfill,
                            (uint32_t)(col0 + ch * 32), a.depth, gmax, gidx);
         } else {
           const int nva = (int)min((int64_t)32, v.cend - (col0 + ch * 32));
-          if (a.seedmode)
-            seed_chunk_fold(va, nva, fmaxf(ma[0], ma[1]), top, (uint32_t)(col0 + ch * 32));
+          if constexpr (SEED)
+            seed_chunk_fold(va, nva, ma, top, a.depth, a.seedmode == 2);
           else
             epi_chunk_fold<GROUPED>(va, nva, fmaxf(ma[0], ma[1]), mylist, thr_key, thr_est, lslot, nfill,
                                     (uint32_t)(col0 + ch * 32), a.depth, gmax, gidx, dq, dn);
@@ -1330,15 +1424,15 @@ __global__ void __launch_bounds__(64 + 128 * NSETS, 1)
         }
         if constexpr (FP8) {
           const float cs_b = pick(csc, ch + 1);
-          if (a.seedmode)
-            seed_chunk<FP8>(vb, pick(nbc, ch + 1), cs_b, rs, top, (uint32_t)(col0 + (ch + 1) * 32));
+          if constexpr (SEED)
+            seed_chunk<FP8>(vb, pick(nbc, ch + 1), cs_b, rs, top, a.depth);
           else
             epi_chunk<FP8, GROUPED>(vb, pick(nbc, ch + 1), cs_b, rs, mylist, thr_key, thr_est, lslot, nfill,
                            (uint32_t)(col0 + (ch + 1) * 32), a.depth, gmax, gidx);
         } else {
           const int nvb = (int)min((int64_t)32, v.cend - (col0 + (ch + 1) * 32));
-          if (a.seedmode)
-            seed_chunk_fold(vb, nvb, fmaxf(mb[0], mb[1]), top, (uint32_t)(col0 + (ch + 1) * 32));
+          if constexpr (SEED)
+            seed_chunk_fold(vb, nvb, mb, top, a.depth, a.seedmode == 2);
           else
             epi_chunk_fold<GROUPED>(vb, nvb, fmaxf(mb[0], mb[1]), mylist, thr_key, thr_est, lslot, nfill,
                                     (uint32_t)(col0 + (ch + 1) * 32), a.depth, gmax, gidx, dq, dn);
@@ -1383,10 +1477,8 @@ __global__ void k2_merge(const uint64_t* __restrict__ partial, int64_t nq, int s
   if (runs) {
     // segmented pass: the row's block run, slots 0 .. (CTAs of the run) x nsets
     const RunInfo ri = runs[row_run[q]];
-    const int c0 = cta_of(ri.first, w.work, w.grid);
-    const int c1 = cta_of(ri.first + ri.len - 1, w.work, w.grid);
     band_first_slot[0] = 0;
-    band_nslots[0] = (c1 - c0 + 1) * nsets;
+    band_nslots[0] = (ri.c1 - ri.c0 + 1) * nsets;
     nseg = band_nslots[0];
   } else {
     const int qb = (int)(q / w.qrows);
@@ -2492,9 +2584,10 @@ mann_status widen_unresolved(Context* ctx, cudaStream_t s, const float* base, co
     MANN_TRY(ctx->scratch_t(SLOT_TIES_COUNTERS, 4, &counters));
     MANN_TRY(ctx->scratch_t(stage == 0 ? SLOT_TIES_ROWS2 : SLOT_TIES_ROWS3, (size_t)h_unres, &next_rows));
     MANN_CUDA_TRY(cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned long long), s));
-    // batches of at most 32 rows take the few-row scan (one point per thread
-    // across the GPU) when the list fits it; a wider list scans all rows at once
-    const int64_t chunk = kk <= 64 ? 32 : h_unres;
+    // up to a few batches of 32 rows take the few-row scan (one point per thread
+    // across the GPU) when the list fits it; more rows, or a wider list, scan
+    // all rows at once
+    const int64_t chunk = kk <= 64 && h_unres <= 256 ? 32 : h_unres;
     for (int64_t r0 = 0; r0 < h_unres; r0 += chunk) {
       const int64_t nr = std::min<int64_t>(chunk, h_unres - r0);
       uint64_t* fkeys = nullptr;
@@ -2601,10 +2694,10 @@ int h_cta_of(int64_t i, int64_t work, int grid) {
 }
 
 // Launch of one k2_main instance: `units` CTAs, or `units` clusters of two CTAs (PAIR).
-template <int CAP, int NSETS, bool PAIR, bool FP8 = false, bool GROUPED = false, int NST = 0>
+template <int CAP, int NSETS, bool PAIR, bool FP8 = false, bool GROUPED = false, int NST = 0, bool SEED = false>
 mann_status launch_k2(const CUtensorMap& mapA, const CUtensorMap& mapB, const MainArgs& ma, int units, size_t smem,
                       cudaStream_t s) {
-  auto fn = k2_main<CAP, NSETS, PAIR, FP8, GROUPED, NST>;
+  auto fn = k2_main<CAP, NSETS, PAIR, FP8, GROUPED, NST, SEED>;
   MANN_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(PAIR ? 2 * units : units));
@@ -2667,6 +2760,8 @@ struct SegPass {
   const int32_t* row_run = nullptr;
   const RunInfo* runs_host = nullptr;
   int64_t nruns = 0;
+  const int64_t* cuts = nullptr;  // [grid + 1] (device)
+  int grid = 0;                   // CTAs the items are cut for
 };
 
 mann_status run_main_pass(Context* ctx, cudaStream_t s, const CUtensorMap& mapA, const void* bxb, int64_t bstride,
@@ -2687,31 +2782,29 @@ mann_status run_main_pass(Context* ctx, cudaStream_t s, const CUtensorMap& mapA,
   // many-set and seed passes (each set writes its own slot); single-matrix
   // main passes keep one set, whose one list admits about half as many
   // candidates (held-out query pass 0.795 -> 0.789 ms)
-  const int nsets = ((depth <= 16 && (seg || seedmode)) || seg3) ? 2 : 1;
+  const int nsets = ((depth <= 16 && (seg || seedmode || nkb <= SHORT_K_STAGES)) || seg3) ? 2 : 1;
   // CTA pairs (cta_group::2) when there are at least two 128-row query blocks
-  const int pairs = (K2_USE_PAIRS && nq > BM && !seg && !fp8)
+  const int pairs = (K2_USE_PAIRS && nq > BM && !seg && !fp8 && !seedmode)
                         ? (nsets == 2 ? k2_pair_capacity<16, 2>(ctx) : k2_pair_capacity<32, 1>(ctx))
                         : 0;
   const bool pair = pairs >= 1;
   const int qrows = pair ? 2 * BM : BM;
   const int64_t qblocks = ceil_div(nq, qrows);
   const int tiles = (int)ceil_div(n, BN);
-  Walk w;
+  Walk w{};
   if (seg) {
     // one band over the item list in run order; a run is one block's items
     w.tiles = 1;
     w.qblocks = (int)seg->nruns;
     w.qrows = BM;
     w.work = seg->nitems;
-    w.grid = (int)std::min<int64_t>(ctx->num_sms, w.work);
+    w.grid = seg->grid;
+    w.cuts = seg->cuts;
     w.band_tiles = 1;
     w.nbands = 1;
     w.span = 1;
-    for (int64_t r = 0; r < seg->nruns; ++r) {
-      const int c0 = h_cta_of(seg->runs_host[r].first, w.work, w.grid);
-      const int c1 = h_cta_of(seg->runs_host[r].first + seg->runs_host[r].len - 1, w.work, w.grid);
-      w.span = std::max(w.span, c1 - c0 + 1);
-    }
+    for (int64_t r = 0; r < seg->nruns; ++r)
+      w.span = std::max(w.span, seg->runs_host[r].c1 - seg->runs_host[r].c0 + 1);
   } else {
     w.tiles = tiles;
     w.qblocks = (int)qblocks;
@@ -2776,6 +2869,11 @@ mann_status run_main_pass(Context* ctx, cudaStream_t s, const CUtensorMap& mapA,
       MANN_TRY((launch_k2<16, 2, true>(mapA, mapB, ma, w.grid, smem, s)));
     else
       MANN_TRY((launch_k2<32, 1, true>(mapA, mapB, ma, w.grid, smem, s)));
+  } else if (seedmode) {
+    if (fp8)
+      MANN_TRY((launch_k2<16, 2, false, true, false, 0, true>(mapA, mapB, ma, w.grid, smem, s)));
+    else
+      MANN_TRY((launch_k2<16, 2, false, false, false, 0, true>(mapA, mapB, ma, w.grid, smem, s)));
   } else if (fp8) {
     if (nsets == 2)
       MANN_TRY((launch_k2<16, 2, false, true>(mapA, mapB, ma, w.grid, smem, s)));
@@ -2786,7 +2884,7 @@ mann_status run_main_pass(Context* ctx, cudaStream_t s, const CUtensorMap& mapA,
       MANN_TRY((launch_k2<24, 2, false, false, true, 3>(mapA, mapB, ma, w.grid, smem, s)));
     else
       MANN_TRY((launch_k2<32, 2, false, false, true, 3>(mapA, mapB, ma, w.grid, smem, s)));
-  } else if (!seedmode && (seg || depth >= GROUPED_MIN_DEPTH)) {
+  } else if (seg || depth >= GROUPED_MIN_DEPTH) {
     // grouped list maxima where rows admit many candidates: the many-set pass
     // (short per-set scans) and deep lists
     if (nsets == 2)
@@ -3002,34 +3100,38 @@ mann_status bf16_prepare(Context* ctx, cudaStream_t s, const float* base, int64_
   }
 
   // ---- prep
-  double* cpart = nullptr;
+  // scratch: scores and sampled max, tickets (one per 32 columns, one for the
+  // probe), the centre's shares
+  const size_t ntick = (size_t)ceil_div(d, 32) + 1;
+  const size_t nhead = NUM_SCALES + 1 + (ntick + 1) / 2;
+  double* score = nullptr;
   float* mu = nullptr;
-  MANN_TRY(ctx->scratch_t(SLOT_CENTRE, 64, &cpart));
+  MANN_TRY(ctx->scratch_t(SLOT_CENTRE, nhead + (size_t)CENTRE_PARTS * d, &score));
+  unsigned* tickets = reinterpret_cast<unsigned*>(score + NUM_SCALES + 1);
   if (pc)
     mu = pc->misc;
   else
     MANN_TRY(ctx->scratch_t(SLOT_MISC3, (size_t)d + 64, &mu));  // mu | BaseMax | scale
   BaseMax* bmax = reinterpret_cast<BaseMax*>(mu + mu_pad);
-  {
-    const int64_t rows = std::min<int64_t>(n, CENTRE_ROWS);
-    const int64_t stride = n / rows;
-    centre_sample_kernel<<<(unsigned)ceil_div(d, 32), 1024, 0, s>>>(mbase, n, d, stride, rows, mu, rn_b);
-    MANN_CHECK_LAUNCH();
-  }
-  // pick the centre / scale with the smallest BF16 residual on a row sample
-  double* score = cpart;  // probe scores
-  MANN_CUDA_TRY(cudaMemsetAsync(score, 0, (NUM_SCALES + 1) * sizeof(double), s));  // scores | sampled max
-  const int64_t sample_rows = std::min<int64_t>(n, 1024);
-  const int64_t stride = std::max<int64_t>(1, n / sample_rows);
-  dim3 pg((unsigned)ceil_div(ceil_div(n, stride), 8), NUM_SCALES);
-  scale_probe_kernel<<<pg, 256, 0, s>>>(mbase, n, d, mu, stride, score, rn_b);
-  MANN_CHECK_LAUNCH();
   float* scale = reinterpret_cast<float*>(bmax + 1);
   int* inexact = reinterpret_cast<int*>(scale + 1);
   float* f16_scale = reinterpret_cast<float*>(inexact + 1);
-  choose_scale_kernel<<<1, 128, 0, s>>>(score, mu, d, scale, inexact, ceil_div(n, stride), f16_scale);
+  MANN_CUDA_TRY(cudaMemsetAsync(score, 0, nhead * sizeof(double), s));
+  {
+    const int64_t rows = std::min<int64_t>(n, CENTRE_ROWS);
+    const int64_t stride = n / rows;
+    centre_sample_kernel<<<dim3((unsigned)ceil_div(d, 32), CENTRE_PARTS), 1024, 0, s>>>(
+        mbase, n, d, stride, rows, score + nhead, tickets, mu, rn_b);
+    MANN_CHECK_LAUNCH();
+  }
+  // pick the centre / scale with the smallest BF16 residual on a row sample
+  const int64_t sample_rows = std::min<int64_t>(n, 1024);
+  const int64_t stride = std::max<int64_t>(1, n / sample_rows);
+  const int64_t sampled = ceil_div(n, stride);
+  scale_probe_kernel<<<(unsigned)ceil_div(sampled, 8), 256, 0, s>>>(
+      mbase, n, d, stride, rn_b,
+      ScaleOut{mu, scale, inexact, f16_scale, bmax, score, tickets + ntick - 1, sampled});
   MANN_CHECK_LAUNCH();
-  MANN_CUDA_TRY(cudaMemsetAsync(bmax, 0, sizeof(BaseMax), s));
   // Data that BF16 cannot hold exactly (after the best centre and scale) runs
   // in the split form: x~ = hi + lo, three BF16 products per term, bounds ~2^8
   // tighter, so the certificate holds for close neighbours too.
@@ -3124,6 +3226,23 @@ mann_status bf16_prepare(Context* ctx, cudaStream_t s, const float* base, int64_
                      cos_bn, cos_qn, P);
 }
 
+// The rank of the seed among a row's sampled minima.  A row whose certificate
+// reaches past its seed falls back to the exact scan: that takes `rank` of
+// about its kreq + 1 nearest points to be in the sample, each with probability
+// 1 / stride.  The smallest rank that leaves 0.2 such rows per call: one costs
+// ~100 us, a rank more ~4 % of the admissions.
+int seed_rank(int kreq, int64_t stride, int64_t nq) {
+  const int m = kreq + 1;
+  const double most = 0.2 / (double)nq, odds = 1.0 / (double)(stride - 1);
+  double term = std::pow(1.0 - 1.0 / (double)stride, m), tail = 1.0;  // P(i in the sample), P(>= i)
+  for (int i = 0; i < SEED_KEEP; ++i) {
+    if (i >= 2 && tail < most) return i;
+    tail -= term;
+    term *= odds * (double)(m - i) / (double)(i + 1);
+  }
+  return SEED_KEEP;
+}
+
 // The autotuned admission depth (list entries a certificate may need) from
 // the depth histogram of a rerank: the 99.9th percentile + 1, 16 when that
 // is <= 16 (the two-set kernel), the full list when > 0.1 % of rows fell back.
@@ -3179,21 +3298,25 @@ mann_status knn_bf16_keys(Context* ctx, cudaStream_t s, const float* base, int64
   CUtensorMap mapA;
   MANN_TRY(make_map(&mapA, Q.xb, nq, P.width, BM, 1, fp8));
 
-  // ---- seed pass: over an evenly spaced sample of SEED_SAMPLE points, the
-  // SEED_DEPTH-th smallest 32-column chunk minimum of each query (an upper
-  // bound of its SEED_DEPTH-th smallest est' there, roughly its
-  // 5n/SEED_SAMPLE-th neighbour) becomes its admission seed in the main pass,
-  // which spares most insertions.  A seed below the row's k-th estimate
-  // leaves the row uncertified.
+  // ---- seed pass: over an evenly spaced sample of the points, a low-ranked
+  // chunk minimum of each query (an upper bound of its rank-th smallest
+  // est' there, roughly its rank * stride-th neighbour) becomes its admission
+  // seed in the main pass, which spares most insertions.
   float* seed = nullptr;
-  if (n >= 16 * SEED_SAMPLE) {
-    const int64_t bstride = n / SEED_SAMPLE;
+  const int64_t sample = std::min<int64_t>(SEED_SAMPLE, n / SEED_STRIDE);
+  // below 16 SEED_SAMPLE points the pass pays only where the CTAs of the main
+  // pass have a few tiles each
+  const bool enough = n >= 16 * SEED_SAMPLE || ceil_div(nq, BM) * ceil_div(n, BN) >= 2 * (int64_t)ctx->num_sms;
+  if (sample >= SEED_MIN_SAMPLE && enough) {
+    const int64_t bstride = n / sample;
+    const int rank = seed_rank(kreq, bstride, nq);
     uint64_t* slists = nullptr;
-    MANN_TRY(run_main_pass(ctx, s, mapA, B.xb, bstride, Q.info, B.info, B.norms, SEED_SAMPLE, nq, d, P.width, P.mainw, P.augx,
-                           SEED_DEPTH, nullptr, err, SLOT_SEED_PARTIAL, SLOT_SEED_LISTS, false, &slists, 1,
+    MANN_TRY(run_main_pass(ctx, s, mapA, B.xb, bstride, Q.info, B.info, B.norms, sample, nq, d, P.width, P.mainw, P.augx,
+                           rank, nullptr, err, SLOT_SEED_PARTIAL, SLOT_SEED_LISTS, false, &slists,
+                           sample < SEED_SAMPLE ? 2 : 1,
                            nullptr, Q.rscale, B.rscale, P.f16));
     MANN_TRY(ctx->scratch_t(SLOT_SEED, (size_t)nq, &seed));
-    seed_from_lists_kernel<<<(unsigned)ceil_div(nq, 256), 256, 0, s>>>(slists, nq, SEED_DEPTH - 1, seed);
+    seed_from_lists_kernel<<<(unsigned)ceil_div(nq, 256), 256, 0, s>>>(slists, nq, rank - 1, seed);
     MANN_CHECK_LAUNCH();
   }
 
@@ -3317,6 +3440,7 @@ struct SegTables {
   std::vector<TileItem> sitems;
   std::vector<RunInfo> sruns;
   std::vector<int32_t> srow_run;
+  std::vector<int64_t> cuts, scuts;  // CTA ranges of the items
   const void* uploaded = nullptr;  // device items buffer the tables were copied to
   const void* suploaded = nullptr;  // device seed-items buffer
   uint64_t uploaded_hash = 0;
@@ -3331,7 +3455,40 @@ SegTables& seg_tables(Context* ctx) {
   return *t;
 }
 
-void build_seg_tables(const int64_t* offs, int nsets, SegTables* T) {
+// Cuts the items into at most `ctas` ranges of about equal cost and notes
+// each run's CTAs.  A run costs `run_cost` tiles besides its own: a row's
+// first tiles admit the bulk of its candidates, so equal numbers of items left
+// the CTAs with many short runs working twice as long as the others (24 clouds
+// of 2k-50k points: 24 M against 12 M cycles).
+void cut_items(std::vector<TileItem>& items, std::vector<RunInfo>& runs, int ctas, double run_cost,
+               std::vector<int64_t>* cuts) {
+  const int64_t n = (int64_t)items.size();
+  const int grid = (int)std::min<int64_t>(ctas, n);
+  const double total = (double)n + run_cost * (double)runs.size();
+  cuts->assign(1, 0);
+  double done = 0.0;
+  for (const RunInfo& r : runs) {
+    const double per = 1.0 + run_cost / (double)r.len;
+    for (int64_t i = 0; i < r.len; ++i) {
+      // a new CTA where its share begins, leaving at least one item for every CTA
+      if ((int)cuts->size() < grid && r.first + i > cuts->back() &&
+          (done >= total * (double)cuts->size() / grid || n - (r.first + i) <= grid - (int64_t)cuts->size()))
+        cuts->push_back(r.first + i);
+      done += per;
+    }
+  }
+  cuts->push_back(n);
+  int c = 0;
+  for (RunInfo& r : runs) {
+    while ((*cuts)[c + 1] <= r.first) ++c;
+    r.c0 = r.c1 = c;
+    while ((*cuts)[r.c1 + 1] < r.first + r.len) ++r.c1;
+    for (int64_t i = 0; i < r.len; ++i) items[(size_t)(r.first + i)].run_cta = r.c0;
+  }
+}
+constexpr double SEG_RUN_COST = 30.0, SEG_SEED_RUN_COST = 1.0;  // in tiles
+
+void build_seg_tables(const int64_t* offs, int nsets, int ctas, SegTables* T) {
   uint64_t h = 1469598103934665603ull;
   for (int c = 0; c <= nsets; ++c) {
     h ^= (uint64_t)offs[c];
@@ -3351,18 +3508,20 @@ void build_seg_tables(const int64_t* offs, int nsets, SegTables* T) {
     const int64_t s1 = (o + nc + SEG_SEED_STRIDE - 1) / SEG_SEED_STRIDE;
     for (int64_t q = 0; q < nc; q += BM) {
       const int64_t first = (int64_t)T->items.size();
-      for (int64_t t = 0; t < nc; t += BN) T->items.push_back(TileItem{o + q, o + nc, o + t, o + nc, first});
+      for (int64_t t = 0; t < nc; t += BN) T->items.push_back(TileItem{o + q, o + nc, o + t, o + nc, first, 0});
       const int32_t r = (int32_t)T->runs.size();
-      T->runs.push_back(RunInfo{first, (int64_t)T->items.size() - first});
+      T->runs.push_back(RunInfo{first, (int64_t)T->items.size() - first, 0, 0});
       for (int64_t row = o + q; row < std::min(o + q + BM, o + nc); ++row) T->row_run[(size_t)row] = r;
       const int64_t sfirst = (int64_t)T->sitems.size();
-      for (int64_t t = s0; t < s1; t += BN) T->sitems.push_back(TileItem{o + q, o + nc, t, s1, sfirst});
-      if (s1 == s0) T->sitems.push_back(TileItem{o + q, o + nc, s0, s0, sfirst});  // no sample: an empty item
+      for (int64_t t = s0; t < s1; t += BN) T->sitems.push_back(TileItem{o + q, o + nc, t, s1, sfirst, 0});
+      if (s1 == s0) T->sitems.push_back(TileItem{o + q, o + nc, s0, s0, sfirst, 0});  // no sample: an empty item
       const int32_t sr = (int32_t)T->sruns.size();
-      T->sruns.push_back(RunInfo{sfirst, (int64_t)T->sitems.size() - sfirst});
+      T->sruns.push_back(RunInfo{sfirst, (int64_t)T->sitems.size() - sfirst, 0, 0});
       for (int64_t row = o + q; row < std::min(o + q + BM, o + nc); ++row) T->srow_run[(size_t)row] = sr;
     }
   }
+  cut_items(T->items, T->runs, ctas, SEG_RUN_COST, &T->cuts);
+  cut_items(T->sitems, T->sruns, ctas, SEG_SEED_RUN_COST, &T->scuts);
   T->hash = h;
 }
 
@@ -3387,12 +3546,15 @@ mann_status knn_bf16_batched_keys(Context* ctx, cudaStream_t s, const float* dat
     return fail(MANN_EINVAL_ARG, "batched graphs: Euclidean or SqEuclidean");
   const int64_t N = offs_host[nsets];
   SegTables& T = seg_tables(ctx);
-  build_seg_tables(offs_host, nsets, &T);
+  build_seg_tables(offs_host, nsets, ctx->num_sms, &T);
   TileItem* d_items = nullptr;
   RunInfo* d_runs = nullptr;
   int32_t* d_row_run = nullptr;
   MANN_TRY(ctx->scratch_t(SLOT_SEG_ITEMS, T.items.size(), &d_items));
-  MANN_TRY(ctx->scratch_t(SLOT_SEG_RUNS, T.runs.size(), &d_runs));
+  // the runs, then the CTA cuts of both passes
+  MANN_TRY(ctx->scratch_t(SLOT_SEG_RUNS, T.runs.size() + T.cuts.size() + T.scuts.size(), &d_runs));
+  int64_t* d_cuts = reinterpret_cast<int64_t*>(d_runs + T.runs.size());
+  int64_t* d_scuts = d_cuts + T.cuts.size();
   MANN_TRY(ctx->scratch_t(SLOT_SEG_ROWRUN, (size_t)N, &d_row_run));
   TileItem* d_sitems = nullptr;
   RunInfo* d_sruns = nullptr;
@@ -3403,6 +3565,8 @@ mann_status knn_bf16_batched_keys(Context* ctx, cudaStream_t s, const float* dat
   if (T.uploaded != d_items || T.suploaded != d_sitems || T.uploaded_hash != T.hash) {
     MANN_CUDA_TRY(cudaMemcpyAsync(d_items, T.items.data(), sizeof(TileItem) * T.items.size(), cudaMemcpyHostToDevice, s));
     MANN_CUDA_TRY(cudaMemcpyAsync(d_runs, T.runs.data(), sizeof(RunInfo) * T.runs.size(), cudaMemcpyHostToDevice, s));
+    MANN_CUDA_TRY(cudaMemcpyAsync(d_cuts, T.cuts.data(), sizeof(int64_t) * T.cuts.size(), cudaMemcpyHostToDevice, s));
+    MANN_CUDA_TRY(cudaMemcpyAsync(d_scuts, T.scuts.data(), sizeof(int64_t) * T.scuts.size(), cudaMemcpyHostToDevice, s));
     MANN_CUDA_TRY(cudaMemcpyAsync(d_row_run, T.row_run.data(), sizeof(int32_t) * N, cudaMemcpyHostToDevice, s));
     MANN_CUDA_TRY(cudaMemcpyAsync(d_sitems, T.sitems.data(), sizeof(TileItem) * T.sitems.size(),
                                   cudaMemcpyHostToDevice, s));
@@ -3434,10 +3598,11 @@ mann_status knn_bf16_batched_keys(Context* ctx, cudaStream_t s, const float* dat
   sp.row_run = d_row_run;
   sp.runs_host = T.runs.data();
   sp.nruns = (int64_t)T.runs.size();
-  // ---- seed pass: each row's SEED_DEPTH-th smallest chunk minimum over
-  // every SEG_SEED_STRIDE-th point of its own set bounds its estimates from
-  // above (a set with no sampled point gets no seed), so the main pass admits
-  // ~3x fewer candidates
+  sp.cuts = d_cuts;
+  sp.grid = (int)T.cuts.size() - 1;
+  // ---- seed pass: a low-ranked half-chunk minimum of each row over every
+  // SEG_SEED_STRIDE-th point of its own set bounds its estimates from above (a
+  // set with too few sampled points gets no seed)
   SegPass ssp;
   ssp.items = d_sitems;
   ssp.nitems = (int64_t)T.sitems.size();
@@ -3445,14 +3610,18 @@ mann_status knn_bf16_batched_keys(Context* ctx, cudaStream_t s, const float* dat
   ssp.row_run = d_srow_run;
   ssp.runs_host = T.sruns.data();
   ssp.nruns = (int64_t)T.sruns.size();
+  ssp.cuts = d_scuts;
+  ssp.grid = (int)T.scuts.size() - 1;
   uint64_t* slists = nullptr;
   const int64_t nsample = (N + SEG_SEED_STRIDE - 1) / SEG_SEED_STRIDE;
+  const int rank = seed_rank(kreq, SEG_SEED_STRIDE, N);
   MANN_TRY(run_main_pass(ctx, s, mapA, P.B.xb, SEG_SEED_STRIDE, P.Q.info, P.B.info, P.B.norms, nsample, N, d, P.width,
-                         P.mainw, P.augx, SEED_DEPTH, nullptr, P.err, SLOT_SEED_PARTIAL, SLOT_SEED_LISTS, false, &slists,
-                         1, &ssp, nullptr, nullptr, P.f16));
+                         P.mainw, P.augx, rank, nullptr, P.err, SLOT_SEED_PARTIAL, SLOT_SEED_LISTS, false, &slists,
+                         2, &ssp, nullptr, nullptr, P.f16));
   float* seed = nullptr;
   MANN_TRY(ctx->scratch_t(SLOT_SEED, (size_t)N, &seed));
-  seed_from_lists_kernel<<<(unsigned)ceil_div(N, 256), 256, 0, s>>>(slists, N, SEED_DEPTH - 1, seed);
+  seed_from_lists_kernel<<<(unsigned)ceil_div(N, 256), 256, 0, s>>>(
+      slists, N, rank - 1, seed);
   MANN_CHECK_LAUNCH();
   uint64_t* lists = nullptr;
   MANN_TRY(run_main_pass(ctx, s, mapA, P.B.xb, 1, P.Q.info, P.B.info, P.B.norms, N, N, d, P.width, P.mainw, P.augx, depth, seed,
