@@ -29,19 +29,19 @@ mann_status check_common(const mann_knn_params* p, int64_t n, int32_t d) {
 mann_status search_device_body(Context* ctx, cudaStream_t s, const mann_knn_params* p,
                                const float* base, int64_t n, const float* qs, int64_t nq, int d,
                                int64_t graph_self, int kreq, int kout, int32_t* ids, float* dists,
-                               mann_knn_report* rep);
+                               mann_knn_report* rep, int tie_entries);
 
 // One exact search on device buffers.  graph_self >= 0: the queries are the
 // points themselves (row r is point r) and `kreq` = k+1 lists drop the self id.
 mann_status search_device(Context* ctx, cudaStream_t s, const mann_knn_params* p,
                           const float* base, int64_t n, const float* qs, int64_t nq, int d,
                           int64_t graph_self, int kreq, int kout, int32_t* ids, float* dists,
-                          mann_knn_report* rep) {
+                          mann_knn_report* rep, int tie_entries = TIE_ENTRIES) {
   const int64_t launches0 = launch_count();
   ctx->timing = (p->flags & MANN_FLAG_TIME_KERNEL) != 0;
   ctx->timed = false;
   mann_status st = search_device_body(ctx, s, p, base, n, qs, nq, d, graph_self, kreq, kout, ids,
-                                      dists, rep);
+                                      dists, rep, tie_entries);
   if (rep) {
     rep->launches = launch_count() - launches0;
     rep->kernel_ms = -1.0;
@@ -59,7 +59,7 @@ mann_status search_device(Context* ctx, cudaStream_t s, const mann_knn_params* p
 mann_status search_device_body(Context* ctx, cudaStream_t s, const mann_knn_params* p,
                                const float* base, int64_t n, const float* qs, int64_t nq, int d,
                                int64_t graph_self, int kreq, int kout, int32_t* ids, float* dists,
-                               mann_knn_report* rep) {
+                               mann_knn_report* rep, int tie_entries) {
   if (rep) {
     *rep = mann_knn_report{};
     rep->rows = nq;
@@ -102,7 +102,7 @@ mann_status search_device_body(Context* ctx, cudaStream_t s, const mann_knn_para
     if (rep) rep->rows = nq;
   } else if (p->flags & MANN_FLAG_FP64_TIES) {
     // FP32 scan with a few extra entries, then FP64 order for near-ties
-    const int kk = (int)std::min<int64_t>(std::min<int64_t>(n, KMAX_FUSED), (int64_t)kreq + 32);
+    const int kk = (int)std::min<int64_t>(std::min<int64_t>(n, KMAX_FUSED), (int64_t)kreq + tie_entries);
     uint64_t* fkeys = nullptr;
     MANN_TRY(knn_fp32_keys(ctx, s, base, n, qs, nq, d, p->metric, kk, nullptr, qn, bn, &fkeys,
                            SLOT_PARTIAL, SLOT_KEYS));
@@ -228,8 +228,8 @@ mann_status knn_dataset_impl(const mann_knn_params* p, const void* owner, uint64
 mann_status exact_search_device(Context* ctx, cudaStream_t s, const mann_knn_params* p,
                                 const float* base, int64_t n, const float* qs, int64_t nq, int d,
                                 int64_t graph_self, int kreq, int kout, int32_t* ids, float* dists,
-                                mann_knn_report* rep) {
-  return search_device(ctx, s, p, base, n, qs, nq, d, graph_self, kreq, kout, ids, dists, rep);
+                                mann_knn_report* rep, int tie_entries) {
+  return search_device(ctx, s, p, base, n, qs, nq, d, graph_self, kreq, kout, ids, dists, rep, tie_entries);
 }
 
 }  // namespace mann
