@@ -1,5 +1,6 @@
 // api.cu -- extern "C" entry points of libmanngpu (declared in include/mann.h).
 #include <atomic>
+#include <cstring>
 #include <new>
 #include <string>
 
@@ -108,14 +109,50 @@ mann_status search_device_body(Context* ctx, cudaStream_t s, const mann_knn_para
                            SLOT_PARTIAL, SLOT_KEYS));
     MANN_TRY(fp32_then_resolve(ctx, s, base, qs, n, nq, d, p->metric, kk, kreq, fkeys, qn, bn, &keys, rep));
   } else {
-    MANN_TRY(knn_fp32_keys(ctx, s, base, n, qs, nq, d, p->metric, kreq, nullptr, qn, bn, &keys,
-                           SLOT_PARTIAL, SLOT_KEYS));
+    MANN_TRY(knn_fp32_finished(ctx, s, base, n, qs, nq, d, p->metric, kreq, qn, bn, kout, graph_self, ids, dists));
   }
-  MANN_TRY(launch_finish(keys, nq, kreq, kout, graph_self, nullptr, ids, dists, s));
+  if (keys) MANN_TRY(launch_finish(keys, nq, kreq, kout, graph_self, nullptr, ids, dists, s));
   if (rep && (p->flags & MANN_FLAG_FP64_ERR))
     MANN_TRY(fp64_max_error(ctx, s, base, qs, d, p->metric, nq, kout, ids, dists, &rep->max_abs_err_fp64));
   return MANN_OK;
 }
+
+// Results of a host call: device buffers that are copied back at the end, or,
+// for a few of them, the context's page-locked staging, which the kernels
+// write directly (a single query's two copies into pageable memory cost as
+// much as its kernels).
+struct HostResults {
+  int32_t* ids = nullptr;
+  float* dists = nullptr;
+  size_t count = 0;
+  bool staged = false;
+
+  mann_status reserve(Context* ctx, size_t n) {
+    count = n;
+    staged = n * (sizeof(int32_t) + sizeof(float)) <= SMALL_BYTES;
+    if (staged) {
+      ids = static_cast<int32_t*>(ctx->small_dev);
+      dists = reinterpret_cast<float*>(ids + n);
+      return MANN_OK;
+    }
+    MANN_TRY(ctx->scratch_t(SLOT_OUT_IDS, n, &ids));
+    return ctx->scratch_t(SLOT_OUT_DISTS, n, &dists);
+  }
+  // waits for the call's work and hands the results over
+  mann_status deliver(Context* ctx, cudaStream_t s, int32_t* out_ids, float* out_dists) const {
+    if (!staged) {
+      MANN_CUDA_TRY(cudaMemcpyAsync(out_ids, ids, sizeof(int32_t) * count, cudaMemcpyDeviceToHost, s));
+      MANN_CUDA_TRY(cudaMemcpyAsync(out_dists, dists, sizeof(float) * count, cudaMemcpyDeviceToHost, s));
+    }
+    MANN_CUDA_TRY(cudaStreamSynchronize(s));
+    if (staged) {
+      std::memcpy(out_ids, ctx->small_host, sizeof(int32_t) * count);
+      std::memcpy(out_dists, static_cast<const char*>(ctx->small_host) + sizeof(int32_t) * count,
+                  sizeof(float) * count);
+    }
+    return MANN_OK;
+  }
+};
 
 mann_status knn_impl(const mann_knn_params* p, const float* base, int64_t n, const float* qs,
                      int64_t q, int32_t d, int32_t* ids, float* dists, mann_knn_report* rep,
@@ -134,19 +171,15 @@ mann_status knn_impl(const mann_knn_params* p, const float* base, int64_t n, con
   CallScope scope(ctx, s);
   if (!host) return search_device(ctx, s, p, base, n, qs, q, d, -1, kreq, kout, ids, dists, rep);
 
-  float *db = nullptr, *dq = nullptr, *dd = nullptr;
-  int32_t* di = nullptr;
+  float *db = nullptr, *dq = nullptr;
+  HostResults r;
   MANN_TRY(ctx->scratch_t(SLOT_BASE, (size_t)n * d, &db));
   MANN_TRY(ctx->scratch_t(SLOT_QUERIES, (size_t)q * d, &dq));
-  MANN_TRY(ctx->scratch_t(SLOT_OUT_IDS, (size_t)q * kout, &di));
-  MANN_TRY(ctx->scratch_t(SLOT_OUT_DISTS, (size_t)q * kout, &dd));
+  MANN_TRY(r.reserve(ctx, (size_t)q * kout));
   MANN_CUDA_TRY(cudaMemcpyAsync(db, base, sizeof(float) * n * d, cudaMemcpyHostToDevice, s));
   MANN_CUDA_TRY(cudaMemcpyAsync(dq, qs, sizeof(float) * q * d, cudaMemcpyHostToDevice, s));
-  MANN_TRY(search_device(ctx, s, p, db, n, dq, q, d, -1, kreq, kout, di, dd, rep));
-  MANN_CUDA_TRY(cudaMemcpyAsync(ids, di, sizeof(int32_t) * q * kout, cudaMemcpyDeviceToHost, s));
-  MANN_CUDA_TRY(cudaMemcpyAsync(dists, dd, sizeof(float) * q * kout, cudaMemcpyDeviceToHost, s));
-  MANN_CUDA_TRY(cudaStreamSynchronize(s));
-  return MANN_OK;
+  MANN_TRY(search_device(ctx, s, p, db, n, dq, q, d, -1, kreq, kout, r.ids, r.dists, rep));
+  return r.deliver(ctx, s, ids, dists);
 }
 
 mann_status graph_impl(const mann_knn_params* p, const float* data, int64_t n, int32_t d,
@@ -208,19 +241,15 @@ mann_status knn_dataset_impl(const mann_knn_params* p, const void* owner, uint64
   CallScope scope(ctx, s);
   PointsOwnerScope owner_scope(ctx, owner, dbase, generation);
   const int64_t rows = qs ? q : n;
-  float *dq = nullptr, *dd = nullptr;
-  int32_t* di = nullptr;
+  float* dq = nullptr;
   if (qs) {
     MANN_TRY(ctx->scratch_t(SLOT_QUERIES, (size_t)q * d, &dq));
     MANN_CUDA_TRY(cudaMemcpyAsync(dq, qs, sizeof(float) * q * d, cudaMemcpyHostToDevice, s));
   }
-  MANN_TRY(ctx->scratch_t(SLOT_OUT_IDS, (size_t)rows * kout, &di));
-  MANN_TRY(ctx->scratch_t(SLOT_OUT_DISTS, (size_t)rows * kout, &dd));
-  MANN_TRY(search_device(ctx, s, p, dbase, n, qs ? dq : dbase, rows, d, graph_self, kreq, kout, di, dd, rep));
-  MANN_CUDA_TRY(cudaMemcpyAsync(ids, di, sizeof(int32_t) * rows * kout, cudaMemcpyDeviceToHost, s));
-  MANN_CUDA_TRY(cudaMemcpyAsync(dists, dd, sizeof(float) * rows * kout, cudaMemcpyDeviceToHost, s));
-  MANN_CUDA_TRY(cudaStreamSynchronize(s));
-  return MANN_OK;
+  HostResults r;
+  MANN_TRY(r.reserve(ctx, (size_t)rows * kout));
+  MANN_TRY(search_device(ctx, s, p, dbase, n, qs ? dq : dbase, rows, d, graph_self, kreq, kout, r.ids, r.dists, rep));
+  return r.deliver(ctx, s, ids, dists);
 }
 
 }  // namespace

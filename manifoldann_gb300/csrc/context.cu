@@ -94,6 +94,11 @@ mann_status get_context(Context** out) {
     MANN_CUDA_TRY(cudaEventCreateWithFlags(&c->last_use, cudaEventDisableTiming));
     MANN_CUDA_TRY(cudaEventCreate(&c->time_a));
     MANN_CUDA_TRY(cudaEventCreate(&c->time_b));
+    MANN_CUDA_TRY(cudaMalloc(&c->few_ticket, sizeof(unsigned)));
+    MANN_CUDA_TRY(cudaMemsetAsync(c->few_ticket, 0, sizeof(unsigned), c->stream));
+    MANN_CUDA_TRY(cudaHostAlloc(&c->small_host, SMALL_BYTES, cudaHostAllocMapped));
+    MANN_CUDA_TRY(cudaHostGetDevicePointer(&c->small_dev, c->small_host, 0));
+    MANN_CUDA_TRY(cudaStreamSynchronize(c->stream));
     g_ctx[dev] = std::move(c);
   }
   *out = g_ctx[dev].get();

@@ -134,6 +134,11 @@ struct Context {
   cudaEvent_t last_use = nullptr;  // recorded after every call that used scratch
   void* slot_ptr[SLOT_COUNT] = {};
   size_t slot_bytes[SLOT_COUNT] = {};
+  // counter of the few-row search's finished blocks, zero between searches
+  unsigned* few_ticket = nullptr;
+  // page-locked, device-mapped staging for the results of small host calls
+  void* small_host = nullptr;
+  void* small_dev = nullptr;
   // optional timing of the call's dominant kernel (MANN_FLAG_TIME_KERNEL)
   cudaEvent_t time_a = nullptr, time_b = nullptr;
   bool timing = false;  // requested for the current call
@@ -162,6 +167,9 @@ struct Context {
     return s;
   }
 };
+
+// bytes of Context::small_host
+constexpr size_t SMALL_BYTES = size_t(64) << 10;
 
 // The context of the current device (created on first use).
 mann_status get_context(Context** out);

@@ -19,6 +19,12 @@ mann_status knn_fp32_keys(Context* ctx, cudaStream_t s, const float* base, int64
                           const int32_t* rows, const float* qn, const float* bn,
                           uint64_t** out_keys, int slot_partial, int slot_keys);
 
+// The same search with its results written as launch_finish writes them (row i
+// to output row i), in the launch that merges the lists.
+mann_status knn_fp32_finished(Context* ctx, cudaStream_t s, const float* base, int64_t n, const float* qs, int64_t nq,
+                              int d, int metric, int kk, const float* qn, const float* bn, int kout,
+                              int64_t graph_self, int32_t* ids, float* dists);
+
 // Keys [nq][kk] -> ids/dists [*][kout].  Key row i goes to output row
 // rows[i] (identity when rows is NULL).  With graph_self >= 0 the query of
 // output row r is point (graph_self + r) and is dropped wherever it appears

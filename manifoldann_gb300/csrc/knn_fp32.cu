@@ -196,6 +196,15 @@ __device__ __forceinline__ uint64_t cmpex(uint64_t v, int j, bool keep_min) {
   return keep_min == (o < v) ? o : v;
 }
 
+// Ascending sort of one key per lane.
+__device__ __forceinline__ uint64_t sort32(uint64_t c, int lane) {
+#pragma unroll
+  for (int w = 2; w <= 32; w <<= 1)
+#pragma unroll
+    for (int j = w >> 1; j > 0; j >>= 1) c = cmpex(c, j, ((lane & j) == 0) == ((lane & w) == 0));
+  return c;
+}
+
 // The cnt <= 32 queued candidates of a row into its sorted list of 32 KW
 // entries.  KW = 1: the candidates are sorted across the lanes (16-wide when
 // that holds them) and merged in one bitonic step -- reverse, lane-wise
@@ -692,27 +701,74 @@ __global__ void __launch_bounds__(FEW_T, 2)
   }
 }
 
+// Sorted ascending lists of 32 keys, one entry per lane: the 32 smallest of both.
+__device__ __forceinline__ uint64_t merge32(uint64_t a, uint64_t b, int lane) {
+  const uint64_t r = __shfl_sync(FULL, (unsigned long long)b, 31 - lane);
+  uint64_t m = r < a ? r : a;
+#pragma unroll
+  for (int j = 16; j > 0; j >>= 1) m = cmpex(m, j, (lane & j) == 0);
+  return m;
+}
+
+// Where a search's results go: its keys, or -- with ids set -- the ids and
+// distances of its rows (launch_finish's rules, row i to output row i).
+struct FewOut {
+  uint64_t* keys;  // [nq][k]
+  int32_t* ids;    // [nq][kout]
+  float* dists;
+  int kout;
+  int64_t graph_self;
+};
+
+// One row's sorted keys (lane e: entry e, k <= 32 of them) as ids and distances.
+__device__ __forceinline__ void finish_row32(const FewOut& o, int64_t q, uint64_t key, int k, int lane) {
+  const bool keep = lane < k && key != KEY_NONE && !(o.graph_self >= 0 && (int64_t)key_id(key) == o.graph_self + q);
+  const unsigned have = __ballot_sync(FULL, keep);
+  const int pos = __popc(have & ((1u << lane) - 1u));
+  if (keep && pos < o.kout) {
+    o.ids[q * o.kout + pos] = key_id(key);
+    o.dists[q * o.kout + pos] = key_dist(key);
+  }
+  for (int e = __popc(have) + lane; e < o.kout; e += 32) {
+    o.ids[q * o.kout + e] = -1;
+    o.dists[q * o.kout + e] = __int_as_float(0x7F800000);
+  }
+}
+
 // few_rows_kernel for nq <= FEW_QS rows of d <= FEW_STAGED_D: the rows sit in
 // shared memory ([FEW_QS][d], staged once), and each thread reads its point
 // with eight float4 loads in flight and no barrier per chunk (the chunked
 // form waits for its loads 25 times per point at d = 784); the same
-// sequential sums in dimension order, the same lists and layout.
+// sequential sums in dimension order.  Every warp keeps its own list of every
+// row -- 32 new distances are sorted and merged at once when many of them
+// count, so no warp waits for another's insertions -- and a block merges its
+// warps' lists at the end.
+//
+// With a ticket (lists of at most 32) the last block to finish merges all the
+// blocks' lists and writes the results: a single query is one launch instead
+// of three (1 x 10,000 x 64: 22 us of kernels with two gaps, now 11).
 template <int METRIC, int KW, bool VEC>
 __global__ void __launch_bounds__(FEW_T, 2)
     few_rows_staged_kernel(const float* __restrict__ base, int64_t n, const float* __restrict__ qs,
                            const int32_t* __restrict__ qrows, int nq, int d, const float* __restrict__ qnorm,
-                           const float* __restrict__ bnorm, int k, uint64_t* __restrict__ partial) {
-  extern __shared__ __align__(16) float fq[];  // [FEW_QS][d]
-  __shared__ float dsm[FEW_QS][FEW_T + 1];
+                           const float* __restrict__ bnorm, int k, uint64_t* __restrict__ partial,
+                           unsigned* __restrict__ ticket, FewOut out) {
+  extern __shared__ __align__(16) float fq[];  // [nq][d], then the warps' lists
+  uint64_t(*wl)[FEW_QS][32 * KW] = reinterpret_cast<uint64_t(*)[FEW_QS][32 * KW]>(fq);
+  __shared__ int last;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  for (int e = t; e < FEW_QS * d; e += FEW_T) {
+  for (int e = t; e < nq * d; e += FEW_T) {
     const int r = e / d, c = e % d;
-    fq[e] = r < nq ? __ldg(&qs[(int64_t)(qrows ? qrows[r] : r) * d + c]) : 0.0f;
+    fq[e] = __ldg(&qs[(int64_t)(qrows ? qrows[r] : r) * d + c]);
   }
   __syncthreads();
-  uint64_t L[1][KW];
+  uint64_t L[FEW_QS][KW], thr[FEW_QS];
 #pragma unroll
-  for (int s = 0; s < KW; ++s) L[0][s] = KEY_NONE;
+  for (int j = 0; j < FEW_QS; ++j) {
+    thr[j] = KEY_NONE;
+#pragma unroll
+    for (int s = 0; s < KW; ++s) L[j][s] = KEY_NONE;
+  }
   for (int64_t p0 = (int64_t)blockIdx.x * FEW_T; p0 < n; p0 += (int64_t)gridDim.x * FEW_T) {
     const int64_t pi = p0 + t;
     const bool valid = pi < n;
@@ -768,32 +824,112 @@ __global__ void __launch_bounds__(FEW_T, 2)
         }
       }
     }
-    __syncthreads();  // the previous points' fold has read dsm
 #pragma unroll
-    for (int j = 0; j < FEW_QS; ++j)
-      if (j < nq) dsm[j][t] = few_distance<METRIC>(acc[j], qnorm, qrows ? qrows[j] : j, bnorm, pi, valid);
-    __syncthreads();
-    few_fold<KW, 1>(dsm, L, nq, warp, lane, p0, (int)min((int64_t)FEW_T, n - p0), k);
+    for (int j = 0; j < FEW_QS; ++j) {
+      if (j >= nq) break;  // uniform
+      const float v = few_distance<METRIC>(acc[j], qnorm, qrows ? qrows[j] : j, bnorm, pi, valid);
+      uint64_t key = valid ? make_key(v, (uint32_t)pi) : KEY_NONE;
+      unsigned pend = __ballot_sync(FULL, key < thr[j]);
+      if (pend == 0) continue;
+      if (KW == 1 && __popc(pend) > 3) {
+        L[j][0] = merge32(L[j][0], sort32(key < thr[j] ? key : KEY_NONE, lane), lane);
+        thr[j] = list_get<KW>(L[j], k - 1);
+        continue;
+      }
+      while (pend) {
+        const int src = __ffs(pend) - 1;
+        pend &= pend - 1;
+        const uint64_t cnd = __shfl_sync(FULL, (unsigned long long)key, src);
+        if (cnd < thr[j]) {
+          list_insert<KW>(L[j], cnd, lane);
+          thr[j] = list_get<KW>(L[j], k - 1);
+        }
+      }
+    }
   }
+  // the block's lists: row j's by warp j
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < FEW_QS; ++j)
+#pragma unroll
+    for (int s = 0; s < KW; ++s) wl[warp][j][s * 32 + lane] = L[j][s];
+  __syncthreads();
   if (warp < nq) {
+    uint64_t B[KW];
+#pragma unroll
+    for (int s = 0; s < KW; ++s) B[s] = wl[0][warp][s * 32 + lane];
+    for (int w = 1; w < FEW_T / 32; ++w) {
+      if constexpr (KW == 1) {
+        B[0] = merge32(B[0], wl[w][warp][lane], lane);
+      } else {
+        uint64_t th = list_get<KW>(B, k - 1);
+        for (int e = 0; e < k; ++e) {
+          const uint64_t cnd = wl[w][warp][e];  // ascending: the rest cannot enter either
+          if (!(cnd < th)) break;
+          list_insert<KW>(B, cnd, lane);
+          th = list_get<KW>(B, k - 1);
+        }
+      }
+    }
     uint64_t* dst = partial + ((int64_t)warp * gridDim.x + blockIdx.x) * k;
 #pragma unroll
     for (int s = 0; s < KW; ++s) {
       const int e = s * 32 + lane;
-      if (e < k) dst[e] = L[0][s];
+      if (e < k) dst[e] = B[s];
     }
   }
+  if constexpr (KW == 1) {
+    if (!ticket) return;
+    __threadfence();
+    __syncthreads();
+    if (t == 0) {
+      last = atomicAdd(ticket, 1u) + 1u == gridDim.x;
+      if (last) *ticket = 0u;  // for the next search
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    // every warp merges a share of the blocks' lists of every row
+    const int nb = gridDim.x;
+    __syncthreads();
+    for (int j = 0; j < nq; ++j) {
+      const uint64_t* src = partial + (int64_t)j * nb * k;
+      uint64_t B = KEY_NONE;
+#pragma unroll 4
+      for (int g = warp; g < nb; g += FEW_T / 32)
+        B = merge32(B, lane < k ? __ldcg(src + (int64_t)g * k + lane) : KEY_NONE, lane);
+      wl[warp][j][lane] = B;
+    }
+    __syncthreads();
+    if (warp >= nq) return;
+    uint64_t B = wl[0][warp][lane];
+    for (int w = 1; w < FEW_T / 32; ++w) B = merge32(B, wl[w][warp][lane], lane);
+    if (out.ids)
+      finish_row32(out, warp, B, k, lane);
+    else if (lane < k)
+      out.keys[(int64_t)warp * k + lane] = B;
+  }
+}
+
+constexpr size_t few_list_bytes(int kw) { return sizeof(uint64_t) * (FEW_T / 32) * FEW_QS * 32 * kw; }
+
+// fused: the kernel itself merges the blocks' lists into `out` (with a ticket)
+bool few_fused(int nq, int d, int kk, const unsigned* ticket) {
+  return ticket && nq <= FEW_QS && d <= FEW_STAGED_D && kk <= 32;
 }
 
 template <int METRIC, bool VEC>
 mann_status launch_few_m(int grid, const float* base, int64_t n, const float* qs, const int32_t* rows, int nq,
-                         int d, const float* qn, const float* bn, int kk, uint64_t* partial, cudaStream_t s) {
+                         int d, const float* qn, const float* bn, int kk, uint64_t* partial, unsigned* ticket,
+                         const FewOut& out, cudaStream_t s) {
   if (nq <= FEW_QS && d <= FEW_STAGED_D) {
-    const size_t smem = sizeof(float) * FEW_QS * d;  // <= 32 KB
+    const size_t smem = std::max(sizeof(float) * nq * d, few_list_bytes(kk <= 32 ? 1 : 2));  // <= 32 KB
     if (kk <= 32)
-      few_rows_staged_kernel<METRIC, 1, VEC><<<grid, FEW_T, smem, s>>>(base, n, qs, rows, nq, d, qn, bn, kk, partial);
+      few_rows_staged_kernel<METRIC, 1, VEC><<<grid, FEW_T, smem, s>>>(base, n, qs, rows, nq, d, qn, bn, kk, partial,
+                                                                       ticket, out);
     else
-      few_rows_staged_kernel<METRIC, 2, VEC><<<grid, FEW_T, smem, s>>>(base, n, qs, rows, nq, d, qn, bn, kk, partial);
+      few_rows_staged_kernel<METRIC, 2, VEC><<<grid, FEW_T, smem, s>>>(base, n, qs, rows, nq, d, qn, bn, kk, partial,
+                                                                       nullptr, out);
   } else if (kk <= 32) {
     few_rows_kernel<METRIC, 1, VEC><<<grid, FEW_T, 0, s>>>(base, n, qs, rows, nq, d, qn, bn, kk, partial);
   } else {
@@ -803,12 +939,27 @@ mann_status launch_few_m(int grid, const float* base, int64_t n, const float* qs
   return MANN_OK;
 }
 
+// The few-row scan for any metric and alignment.
+mann_status run_few(int metric, int grid, const float* base, int64_t n, const float* qs, const int32_t* rows, int nq,
+                    int d, const float* qn, const float* bn, int kk, uint64_t* partial, unsigned* ticket,
+                    const FewOut& out, cudaStream_t s) {
+  const bool vec = (d % 4 == 0) && ((reinterpret_cast<uintptr_t>(base) & 15) == 0);
+#define FEW_METRIC(M)                                                                                        \
+  return vec ? launch_few_m<M, true>(grid, base, n, qs, rows, nq, d, qn, bn, kk, partial, ticket, out, s)    \
+             : launch_few_m<M, false>(grid, base, n, qs, rows, nq, d, qn, bn, kk, partial, ticket, out, s)
+  if (metric == MANN_METRIC_EUCLIDEAN) FEW_METRIC(MANN_METRIC_EUCLIDEAN);
+  if (metric == MANN_METRIC_SQEUCLIDEAN) FEW_METRIC(MANN_METRIC_SQEUCLIDEAN);
+  FEW_METRIC(MANN_METRIC_COSINE);
+#undef FEW_METRIC
+}
+
 // Merge up to `slots` sorted lists of k keys per query into one sorted list
 // of k.  One warp per query; lane s walks list s (and s+32, ...).  A balanced
 // walk of the tile kernel (w.per > 0, bq rows per block) wrote only the slots
-// of the CTAs that its query block met.
+// of the CTAs that its query block met.  With o.ids the results are written as
+// finish_kernel writes them, without a launch of its own.
 __global__ void merge_lists_kernel(const uint64_t* __restrict__ partial, int64_t nq, int slots,
-                                   int k, uint64_t* __restrict__ out, int64_t tiles, int64_t per, int bq) {
+                                   int k, FewOut o, int64_t tiles, int64_t per, int bq) {
   const int lane = threadIdx.x & 31;
   const int64_t q = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (q >= nq) return;
@@ -827,13 +978,22 @@ __global__ void merge_lists_kernel(const uint64_t* __restrict__ partial, int64_t
     head[t] = 0;
     cur[t] = (s < nsplit) ? src[(int64_t)s * k] : KEY_NONE;
   }
+  int found = 0;
   for (int e = 0; e < k; ++e) {
     uint64_t m = cur[0];
 #pragma unroll
     for (int t = 1; t < MAXL; ++t) m = min(m, cur[t]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = min(m, (uint64_t)__shfl_xor_sync(FULL, m, o));
-    if (lane == 0) out[q * k + e] = m;
+    if (!o.ids) {
+      if (lane == 0) o.keys[q * k + e] = m;
+    } else if (m != KEY_NONE && found < o.kout && !(o.graph_self >= 0 && (int64_t)key_id(m) == o.graph_self + q)) {
+      if (lane == 0) {
+        o.ids[q * o.kout + found] = key_id(m);
+        o.dists[q * o.kout + found] = key_dist(m);
+      }
+      ++found;
+    }
     if (m == KEY_NONE) continue;
 #pragma unroll
     for (int t = 0; t < MAXL; ++t) {
@@ -844,6 +1004,11 @@ __global__ void merge_lists_kernel(const uint64_t* __restrict__ partial, int64_t
       }
     }
   }
+  if (o.ids)
+    for (int e = found + lane; e < o.kout; e += 32) {
+      o.ids[q * o.kout + e] = -1;
+      o.dists[q * o.kout + e] = __int_as_float(0x7F800000);
+    }
 }
 
 __global__ void finish_kernel(const uint64_t* __restrict__ keys, int64_t nq, int kk, int kout,
@@ -990,7 +1155,8 @@ mann_status launch_merge_lists(const uint64_t* partial, int64_t nq, int nsplit, 
                                cudaStream_t s) {
   if (nq <= 0) return MANN_OK;
   if (nsplit > 128) return fail(MANN_EINVAL_ARG, "at most 128 lists per query can be merged");
-  merge_lists_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, s>>>(partial, nq, nsplit, k, out, 0, 0, 1);
+  merge_lists_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, s>>>(partial, nq, nsplit, k, FewOut{out, nullptr, nullptr, 0, -1}, 0,
+                                                               0, 1);
   MANN_CHECK_LAUNCH();
   return MANN_OK;
 }
@@ -1011,63 +1177,59 @@ mann_status launch_finish(const uint64_t* keys, int64_t nq, int kk, int kout, in
   return MANN_OK;
 }
 
-mann_status knn_fp32_keys(Context* ctx, cudaStream_t s, const float* base, int64_t n,
-                          const float* qs, int64_t nq, int d, int metric, int kk,
-                          const int32_t* rows, const float* qn, const float* bn,
-                          uint64_t** out_keys, int slot_partial, int slot_keys) {
+// knn_fp32_keys, or with o.ids set the finished results (nothing in *out_keys).
+static mann_status fp32_search(Context* ctx, cudaStream_t s, const float* base, int64_t n, const float* qs, int64_t nq,
+                               int d, int metric, int kk, const int32_t* rows, const float* qn, const float* bn,
+                               FewOut o, uint64_t** out_keys, int slot_partial, int slot_keys) {
   if (kk < 1 || kk > KMAX_FUSED)
     return fail(MANN_EINVAL_ARG, "fused top-k supports 1 <= k <= " + std::to_string(KMAX_FUSED));
   if (nq <= 0) return MANN_OK;
   if (metric == MANN_METRIC_COSINE && (qn == nullptr || bn == nullptr))
     return fail(MANN_EINVAL_ARG, "cosine search needs row norms");
-  if (nq <= FEW_Q && kk <= 64) {
-    // a handful of rows: one point per thread across the whole GPU
-    const int grid = (int)std::min<int64_t>(256, ceil_div(n, FEW_T));  // one pass for n <= 65536
-    uint64_t* partial = nullptr;
-    MANN_TRY(ctx->scratch_t(slot_partial, (size_t)nq * grid * kk, &partial));
-    const bool vec4 = (d % 4 == 0) && ((reinterpret_cast<uintptr_t>(base) & 15) == 0);
+  const bool few = nq <= FEW_Q && kk <= 64;
+  // a handful of rows: one point per thread across the whole GPU (one pass for n <= 65536)
+  const int grid = few ? (int)std::min<int64_t>(256, ceil_div(n, FEW_T)) : 0;
+  const K1Walk w = few ? K1Walk{} : k1_walk(ctx->num_sms, n, nq, kk, 0);
+  const int slots = few ? grid : w.slots;
+  const bool fused = few && few_fused((int)nq, d, kk, ctx->few_ticket);
+  uint64_t* partial = nullptr;
+  MANN_TRY(ctx->scratch_t(slot_partial, (size_t)nq * slots * kk, &partial));
+  if (!o.ids && (fused || slots > 1)) MANN_TRY(ctx->scratch_t(slot_keys, (size_t)nq * kk, &o.keys));
+  if (few) {
     ctx->time_begin(s);
-    switch (metric) {
-      case MANN_METRIC_EUCLIDEAN:
-        MANN_TRY((vec4 ? launch_few_m<MANN_METRIC_EUCLIDEAN, true>(grid, base, n, qs, rows, (int)nq, d, qn, bn, kk, partial, s)
-                       : launch_few_m<MANN_METRIC_EUCLIDEAN, false>(grid, base, n, qs, rows, (int)nq, d, qn, bn, kk, partial, s)));
-        break;
-      case MANN_METRIC_SQEUCLIDEAN:
-        MANN_TRY((vec4 ? launch_few_m<MANN_METRIC_SQEUCLIDEAN, true>(grid, base, n, qs, rows, (int)nq, d, qn, bn, kk, partial, s)
-                       : launch_few_m<MANN_METRIC_SQEUCLIDEAN, false>(grid, base, n, qs, rows, (int)nq, d, qn, bn, kk, partial, s)));
-        break;
-      default:
-        MANN_TRY((vec4 ? launch_few_m<MANN_METRIC_COSINE, true>(grid, base, n, qs, rows, (int)nq, d, qn, bn, kk, partial, s)
-                       : launch_few_m<MANN_METRIC_COSINE, false>(grid, base, n, qs, rows, (int)nq, d, qn, bn, kk, partial, s)));
-        break;
-    }
+    MANN_TRY(run_few(metric, grid, base, n, qs, rows, (int)nq, d, qn, bn, kk, partial, fused ? ctx->few_ticket : nullptr,
+                     o, s));
     ctx->time_end(s);
-    if (grid == 1) {
+  } else {
+    MANN_TRY(run_k1(ctx, metric, kk, base, n, qs, rows, nq, d, qn, bn, w, partial, s));
+  }
+  if (!fused) {
+    if (slots == 1) {
+      if (o.ids) return launch_finish(partial, nq, kk, o.kout, o.graph_self, nullptr, o.ids, o.dists, s);
       *out_keys = partial;
       return MANN_OK;
     }
-    uint64_t* keys = nullptr;
-    MANN_TRY(ctx->scratch_t(slot_keys, (size_t)nq * kk, &keys));
-    merge_lists_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, s>>>(partial, nq, grid, kk, keys, 0, 0, 1);
+    merge_lists_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, s>>>(partial, nq, slots, kk, o, few ? 0 : w.tiles,
+                                                                 few ? 0 : w.per, few ? 1 : k1_rows(nq, kk));
     MANN_CHECK_LAUNCH();
-    *out_keys = keys;
-    return MANN_OK;
   }
-  const K1Walk w = k1_walk(ctx->num_sms, n, nq, kk, 0);
-  uint64_t* partial = nullptr;
-  MANN_TRY(ctx->scratch_t(slot_partial, (size_t)nq * w.slots * kk, &partial));
-  MANN_TRY(run_k1(ctx, metric, kk, base, n, qs, rows, nq, d, qn, bn, w, partial, s));
-  if (w.slots == 1) {
-    *out_keys = partial;
-    return MANN_OK;
-  }
-  uint64_t* keys = nullptr;
-  MANN_TRY(ctx->scratch_t(slot_keys, (size_t)nq * kk, &keys));
-  merge_lists_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, s>>>(partial, nq, w.slots, kk, keys, w.tiles, w.per,
-                                                               k1_rows(nq, kk));
-  MANN_CHECK_LAUNCH();
-  *out_keys = keys;
+  if (!o.ids) *out_keys = o.keys;
   return MANN_OK;
+}
+
+mann_status knn_fp32_keys(Context* ctx, cudaStream_t s, const float* base, int64_t n,
+                          const float* qs, int64_t nq, int d, int metric, int kk,
+                          const int32_t* rows, const float* qn, const float* bn,
+                          uint64_t** out_keys, int slot_partial, int slot_keys) {
+  return fp32_search(ctx, s, base, n, qs, nq, d, metric, kk, rows, qn, bn, FewOut{nullptr, nullptr, nullptr, 0, -1},
+                     out_keys, slot_partial, slot_keys);
+}
+
+mann_status knn_fp32_finished(Context* ctx, cudaStream_t s, const float* base, int64_t n, const float* qs, int64_t nq,
+                              int d, int metric, int kk, const float* qn, const float* bn, int kout,
+                              int64_t graph_self, int32_t* ids, float* dists) {
+  return fp32_search(ctx, s, base, n, qs, nq, d, metric, kk, nullptr, qn, bn,
+                     FewOut{nullptr, ids, dists, kout, graph_self}, nullptr, SLOT_PARTIAL, SLOT_KEYS);
 }
 
 }  // namespace mann
@@ -1116,22 +1278,9 @@ mann_status knn_fp32_keys_on(int num_sms, cudaStream_t s, const float* base, int
   uint64_t* partial = scratch;
   mann_status st;
   if (nq <= FEW_Q && kk <= 64) {
-    // the few-row kernel, exactly as knn_fp32_keys runs it (grid = nsplit)
-    const bool vec4 = (d % 4 == 0) && ((reinterpret_cast<uintptr_t>(base) & 15) == 0);
-    switch (metric) {
-      case MANN_METRIC_EUCLIDEAN:
-        st = vec4 ? launch_few_m<MANN_METRIC_EUCLIDEAN, true>(nsplit, base, n, qs, nullptr, (int)nq, d, qn, bn, kk, partial, s)
-                  : launch_few_m<MANN_METRIC_EUCLIDEAN, false>(nsplit, base, n, qs, nullptr, (int)nq, d, qn, bn, kk, partial, s);
-        break;
-      case MANN_METRIC_SQEUCLIDEAN:
-        st = vec4 ? launch_few_m<MANN_METRIC_SQEUCLIDEAN, true>(nsplit, base, n, qs, nullptr, (int)nq, d, qn, bn, kk, partial, s)
-                  : launch_few_m<MANN_METRIC_SQEUCLIDEAN, false>(nsplit, base, n, qs, nullptr, (int)nq, d, qn, bn, kk, partial, s);
-        break;
-      default:
-        st = vec4 ? launch_few_m<MANN_METRIC_COSINE, true>(nsplit, base, n, qs, nullptr, (int)nq, d, qn, bn, kk, partial, s)
-                  : launch_few_m<MANN_METRIC_COSINE, false>(nsplit, base, n, qs, nullptr, (int)nq, d, qn, bn, kk, partial, s);
-        break;
-    }
+    // the few-row kernel, as knn_fp32_keys runs it (grid = nsplit), its lists merged by a launch of their own
+    st = run_few(metric, nsplit, base, n, qs, nullptr, (int)nq, d, qn, bn, kk, partial, nullptr,
+                 FewOut{nullptr, nullptr, nullptr, 0, -1}, s);
   } else {
     Context plain;  // carries the SM count; no timing, no scratch
     plain.num_sms = num_sms;
@@ -1144,7 +1293,8 @@ mann_status knn_fp32_keys_on(int num_sms, cudaStream_t s, const float* base, int
     return MANN_OK;
   }
   uint64_t* keys = partial + (size_t)nq * nsplit * kk;
-  merge_lists_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, s>>>(partial, nq, nsplit, kk, keys, 0, 0, 1);
+  merge_lists_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, s>>>(partial, nq, nsplit, kk,
+                                                               FewOut{keys, nullptr, nullptr, 0, -1}, 0, 0, 1);
   MANN_CHECK_LAUNCH();
   *out_keys = keys;
   return MANN_OK;
