@@ -15,6 +15,7 @@
 // id); the reference's heap keeps an arbitrary member of an exact tie at the
 // k-th place, this keeps the lower id.
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "f32x2.cuh"
@@ -26,8 +27,9 @@ namespace mann {
 namespace {
 
 constexpr int SCAN_Q = 32;    // queries per CTA (at most)
-constexpr int SCAN_T = 256;   // threads = points per pass
-constexpr int SCAN_DC = 32;   // dimensions per register batch of a point row
+constexpr int SCAN_T = 128;   // threads
+constexpr int SCAN_P = 256;   // points per pass: two per thread
+constexpr int SCAN_DC = 16;   // dimensions per staged slice of a point row
 
 __global__ void ivf_lists_kernel(const int64_t* __restrict__ start, const int64_t* __restrict__ members,
                                  int k, int64_t n, int64_t* __restrict__ offsets,
@@ -98,11 +100,15 @@ __global__ void __launch_bounds__(1024) probe_scan_kernel(const unsigned* __rest
   }
 }
 
+// (query, probe rank) pairs grouped by list, and the list of every chunk (a
+// search for it in each scan block was a chain of a dozen dependent loads)
 __global__ void probe_scatter_kernel(const int32_t* __restrict__ probes, int64_t nq, int nprobe,
-                                     int nlist, const int64_t* __restrict__ qoff,
+                                     int nlist, const int64_t* __restrict__ qoff, const int64_t* __restrict__ choff,
                                      unsigned* __restrict__ cursor, int32_t* __restrict__ pair_q,
-                                     int32_t* __restrict__ pair_r) {
+                                     int32_t* __restrict__ pair_r, int32_t* __restrict__ chunk_list) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (int64_t l = i; l < nlist; l += (int64_t)gridDim.x * blockDim.x)
+    for (int64_t c = choff[l]; c < choff[l + 1]; ++c) chunk_list[c] = (int32_t)l;
   if (i >= nq * nprobe) return;
   const int l = probes[i];
   if (l < 0 || l >= nlist) return;
@@ -111,135 +117,292 @@ __global__ void probe_scatter_kernel(const int32_t* __restrict__ probes, int64_t
   pair_r[pos] = (int32_t)(i % nprobe);
 }
 
-// One CTA: list l and up to QC (16 or 32) of its queries.  Each thread takes one point
-// of the list per pass (read in place through the list's ids) and computes
-// its distance to every query of the CTA -- the point's coordinates in
-// registers, the queries' in shared memory, each distance the sequential
-// difference-form sum over dimensions 0..d-1 of the FP32 form.  Warp w keeps
-// the sorted top-k of queries w, w+8, ... as warp-distributed lists.
+// One stage of a warp's bitonic network over 32-bit values (lane holds one).
+__device__ __forceinline__ uint32_t cmpex32(uint32_t v, int j, bool keep_min) {
+  const uint32_t o = __shfl_xor_sync(wl::FULL, v, j);
+  return keep_min ? min(v, o) : max(v, o);
+}
+
+// One pass's distances of one query (dist[0, np), bits not negative) into its
+// sorted list of at most 32 keys.  The k-th smallest of the lanes' minima is
+// an upper bound of the pass's k-th distance, so a list that is not full sees
+// about k distances instead of all of them (at k = 10, 12 of 256); those that
+// pass are sorted and merged 32 at a time.  Entering them one by one took more
+// instructions than the distances themselves.
+__device__ __forceinline__ void pass_topk32(const float* __restrict__ dist, int np, const int32_t* __restrict__ ids,
+                                            uint64_t& L, int k, uint64_t* __restrict__ buf, int lane) {
+  constexpr int G = SCAN_P / 32;
+  uint32_t v[G];
+  uint32_t low = 0xFFFFFFFFu;
+#pragma unroll
+  for (int g = 0; g < G; ++g) {
+    const int col = 32 * g + lane;
+    const float f = col < np ? dist[col] : 0.0f;
+    v[g] = col < np ? (f == f ? __float_as_uint(f) : 0x7FC00000u) : 0xFFFFFFFFu;
+    low = min(low, v[g]);
+  }
+  const uint64_t kth = __shfl_sync(wl::FULL, (unsigned long long)L, k - 1);
+  uint32_t thr;  // bits of the largest distance that may still enter
+  if (kth != KEY_NONE) {
+    thr = __float_as_uint(key_dist(kth));
+  } else {
+#pragma unroll
+    for (int w = 2; w <= 32; w <<= 1)
+#pragma unroll
+      for (int j = w >> 1; j > 0; j >>= 1) low = cmpex32(low, j, ((lane & j) == 0) == ((lane & w) == 0));
+    thr = __shfl_sync(wl::FULL, low, k - 1);  // all bits set: fewer than k lanes hold a point
+  }
+  unsigned pend = 0;
+#pragma unroll
+  for (int g = 0; g < G; ++g) pend |= (v[g] <= thr && 32 * g + lane < np ? 1u : 0u) << g;
+  while (__any_sync(wl::FULL, pend != 0)) {
+    int base = 0;
+    __syncwarp();
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      const bool mine = (pend >> g) & 1u;
+      const unsigned m = __ballot_sync(wl::FULL, mine);
+      const int pos = base + __popc(m & ((1u << lane) - 1u));
+      if (mine && pos < 32) {
+        const int col = 32 * g + lane;
+        buf[pos] = make_key(__uint_as_float(v[g]), (uint32_t)ids[col]);
+        pend &= ~(1u << g);
+      }
+      base += __popc(m);
+    }
+    __syncwarp();
+    L = wl::merge32(L, wl::sort32(lane < base ? buf[lane] : KEY_NONE, lane), lane);
+    if (base > 32) {  // the rest is tested again against the list's new k-th
+      const uint64_t now = __shfl_sync(wl::FULL, (unsigned long long)L, k - 1);
+      if (now != KEY_NONE) {
+        const uint32_t t = __float_as_uint(key_dist(now));
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+          if (v[g] > t) pend &= ~(1u << g);
+      }
+    }
+  }
+}
+
+// Shared memory of a scan CTA: the staged queries, then a slice of every row, over which the pass's distances are laid when the arithmetic is done.
+template <int QC>
+struct ScanSmem {
+  static constexpr int SDQ = QC == 16 ? 128 : 64;  // query dimensions per stage
+  static constexpr int QS = QC + 4;                // stride (floats), a multiple of 4
+  static constexpr int XS = SCAN_DC + 4;           // stride of a staged row slice
+  static constexpr int DS = SCAN_P + 1;            // stride of a query's distances
+  static constexpr size_t QUERIES = (size_t)SDQ * QS;
+  static constexpr size_t ROWS = (size_t)SCAN_P * XS;
+  static constexpr size_t DISTS = (size_t)QC * DS;
+  static constexpr size_t BYTES = sizeof(float) * (QUERIES + (ROWS > DISTS ? ROWS : DISTS));
+};
+
+// One CTA: list l and up to QC (16 or 32) of its queries.  Each thread takes
+// two points of the list per pass (read in place through the list's ids) and
+// computes their distances to every query of the CTA, each distance the
+// sequential difference-form sum over dimensions 0..d-1 of the FP32 form.
+// Warp w keeps the sorted top-k of queries w, w+4, ... as warp-distributed lists.
+//
+// A warp brings in its 64 rows a 16-dimension slice at a time, four lanes to a
+// row (cp.async), and each thread reads its own rows back from shared memory;
+// the slices are the warp's own, so no block barrier falls inside the
+// arithmetic, and six CTAs per SM cover each other's loads.  What bounds it is shared-memory reads of the
+// queries, one 16-byte broadcast per four queries and dimension: two points
+// per thread halve them.
 template <int METRIC, int KW, bool VEC, int QC>
-__global__ void __launch_bounds__(SCAN_T, QC == 16 ? 3 : 2)
+__global__ void __launch_bounds__(SCAN_T, QC == 16 ? 6 : 3)
     ivf_scan_kernel(const float* __restrict__ data, const int64_t* __restrict__ loff,
                     const int32_t* __restrict__ lids, const float* __restrict__ qs, int d,
                     const int64_t* __restrict__ qoff, const int32_t* __restrict__ pair_q,
-                    const int32_t* __restrict__ pair_r, const int64_t* __restrict__ choff, int nlist,
+                    const int32_t* __restrict__ pair_r, const int64_t* __restrict__ choff,
+                    const int32_t* __restrict__ chunk_list, int nlist,
                     int k, int nprobe, uint64_t* __restrict__ partial) {
   // queries staged transposed, [dimension][query] with a padded stride, so one
   // 16-byte broadcast read gives four queries' value at one dimension
-  constexpr int SDQ = QC == 16 ? 128 : 64;  // dimensions per stage
-  constexpr int QS = QC + 4;                // stride (floats), a multiple of 4
-  __shared__ __align__(16) float qsm[SDQ * QS];
-  __shared__ float dsm[QC][SCAN_T + 1];
+  using S = ScanSmem<QC>;
+  constexpr int SDQ = S::SDQ, QS = S::QS, XS = S::XS;
+  constexpr int NW = SCAN_T / 32;
+  extern __shared__ __align__(16) float scan_smem[];
+  float* qsm = scan_smem;
+  float* rows = qsm + S::QUERIES;  // [SCAN_P][XS]
+  float* dsm = rows;               // [QC][DS]
   __shared__ int32_t s_q[QC];
+  __shared__ uint64_t s_buf[NW][32];
 
   const int64_t w = blockIdx.x;
   if (w >= choff[nlist]) return;
-  int lo = 0, hi = nlist - 1;
-  while (lo < hi) {  // last list whose chunk offset <= w
-    const int mid = (lo + hi + 1) >> 1;
-    if (choff[mid] <= w) lo = mid;
-    else hi = mid - 1;
-  }
-  const int l = lo;
+  const int l = chunk_list[w];
   const int64_t e0 = qoff[l] + (w - choff[l]) * QC;
   const int nqe = (int)min((int64_t)QC, qoff[l + 1] - e0);
   const int64_t p_begin = loff[l], p_end = loff[l + 1];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   if (t < nqe) s_q[t] = pair_q[e0 + t];
-  __syncthreads();
 
-  constexpr int MW = QC / 8;  // queries per warp
+  constexpr int MW = QC / NW;  // queries per warp
   uint64_t L[MW][KW];
 #pragma unroll
   for (int m = 0; m < MW; ++m)
 #pragma unroll
     for (int s = 0; s < KW; ++s) L[m][s] = KEY_NONE;
 
-  for (int64_t p0 = p_begin; p0 < p_end; p0 += SCAN_T) {
-    const int64_t pi = p0 + t;
-    const bool valid = pi < p_end;
-    const float* prow = data + (valid ? (int64_t)lids[pi] : 0) * d;
+  float* wrows = rows + warp * 64 * XS;  // the warp's 64 rows: lane's are lane and lane + 32
+  for (int64_t p0 = p_begin; p0 < p_end; p0 += SCAN_P) {
+    int32_t row[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int64_t pi = p0 + warp * 64 + 32 * h + lane;
+      row[h] = pi < p_end ? lids[pi] : -1;
+    }
+    // dimensions [c0, c0 + SCAN_DC) of the warp's rows (VEC: what lies below d)
+    auto fetch = [&](int c0) {
+      float* dst = wrows;
+      if constexpr (VEC) {
+        const int c = (lane & 3) * 4;
+#pragma unroll
+        for (int it = 0; it < 8; ++it) {
+          const int r = it * 8 + (lane >> 2);
+          const int32_t src = __shfl_sync(wl::FULL, row[it >> 2], r & 31);
+          if (src >= 0 && c0 + c < d) {
+            const uint32_t sa = (uint32_t)__cvta_generic_to_shared(dst + r * XS + c);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sa), "l"(data + (int64_t)src * d + c0 + c)
+                         : "memory");
+          }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+      } else {
+        const int c = c0 + (lane & 15);
+        for (int it = 0; it < 32; ++it) {
+          const int r = it * 2 + (lane >> 4);
+          const int32_t a = __shfl_sync(wl::FULL, row[0], r & 31), b = __shfl_sync(wl::FULL, row[1], r & 31);
+          const int32_t src = r < 32 ? a : b;
+          dst[r * XS + (lane & 15)] = src >= 0 && c < d ? __ldg(data + (int64_t)src * d + c) : 0.0f;
+        }
+      }
+    };
+    // the arithmetic is what the scan costs, so it stops where the list does:
+    // a warp past the end computes nothing, one with at most 32 rows one half
+    const int halves = (int)min((int64_t)2, max((int64_t)0, (p_end - p0 - warp * 64 + 31) / 32));
+    if (p0 > p_begin) __syncthreads();  // the last pass's distances lie over the slices
+    if (halves > 0) fetch(0);
     // queries 2i and 2i+1 in one f32x2 pair: each lane rounds as the scalar
     // difference form, dimension by dimension in order
-    uint64_t acc2[QC / 2];
+    uint64_t acc2[2][QC / 2];
 #pragma unroll
-    for (int i = 0; i < QC / 2; ++i) acc2[i] = 0ull;
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int i = 0; i < QC / 2; ++i) acc2[h][i] = 0ull;
     const int ng4 = (nqe + 3) >> 2;  // groups of four staged queries in use
-    for (int c0 = 0; c0 < d; c0 += SDQ) {
-      const int dq = min(SDQ, d - c0);
-      __syncthreads();
-      for (int e = t; e < QC * SDQ; e += SCAN_T) {
-        const int r = e / SDQ, c = e % SDQ;
-        qsm[c * QS + r] = (r < nqe && c < dq) ? __ldg(&qs[(int64_t)s_q[r] * d + c0 + c]) : 0.0f;
-      }
-      __syncthreads();
-      for (int cb = 0; cb < dq; cb += SCAN_DC) {
-        const int dc = min(SCAN_DC, dq - cb);
-        float pv[SCAN_DC];
-        if (VEC && dc == SCAN_DC) {
+    for (int c0 = 0; c0 < d; c0 += SCAN_DC) {
+      const int cq = c0 % SDQ;  // within the staged queries
+      if (cq == 0 && (d > SDQ || p0 == p_begin)) {
+        const int dq = min(SDQ, d - c0);
+        __syncthreads();
+        // consecutive threads take consecutive queries: distinct banks
+        for (int e = t; e < QC * SDQ / 4; e += SCAN_T) {
+          const int r = e % QC, c = e / QC * 4;
+          float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+          if (r < nqe) {
+            const float* q = qs + (int64_t)s_q[r] * d + c0 + c;
 #pragma unroll
-          for (int c = 0; c < SCAN_DC; c += 4) {
-            const float4 v =
-                valid ? __ldg(reinterpret_cast<const float4*>(prow + c0 + cb + c)) : make_float4(0, 0, 0, 0);
-            pv[c] = v.x;
-            pv[c + 1] = v.y;
-            pv[c + 2] = v.z;
-            pv[c + 3] = v.w;
+            for (int i = 0; i < 4; ++i)
+              if (c + i < dq) v[i] = __ldg(q + i);
           }
-        } else {
 #pragma unroll
-          for (int c = 0; c < SCAN_DC; ++c) pv[c] = (valid && c < dc) ? __ldg(prow + c0 + cb + c) : 0.0f;
+          for (int i = 0; i < 4; ++i) qsm[(c + i) * QS + r] = v[i];
         }
-        // dimensions past d are zero in both operands: (0 - 0)^2 adds nothing
+        __syncthreads();
+      }
+      if (halves == 0) continue;
+      if (c0 > 0) fetch(c0);
+      if constexpr (VEC) asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncwarp();
+      const float* own = wrows + lane * XS;
+      const int dc = min(SCAN_DC, d - c0);
+      // four dimensions of NH points against the staged queries
+      auto four = [&](int c4, auto nh) {
+        constexpr int NH = decltype(nh)::value;
+        float x[NH][4];
 #pragma unroll
-        for (int c = 0; c < SCAN_DC; ++c) {
-          const uint64_t x2 = f2::pack(pv[c], pv[c]);
-          const float4* qrow4 = reinterpret_cast<const float4*>(&qsm[(cb + c) * QS]);
+        for (int h = 0; h < NH; ++h) {
+          const float4 v = *reinterpret_cast<const float4*>(own + 32 * h * XS + c4);
+          x[h][0] = v.x;
+          x[h][1] = v.y;
+          x[h][2] = v.z;
+          x[h][3] = v.w;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float4* qrow4 = reinterpret_cast<const float4*>(&qsm[(cq + c4 + i) * QS]);
 #pragma unroll
           for (int g = 0; g < QC / 4; ++g) {
             if (g < ng4) {  // block-uniform
               const float4 q4 = qrow4[g];
-              uint64_t u = f2::sub(f2::pack(q4.x, q4.y), x2);
-              acc2[2 * g] = f2::fma(u, u, acc2[2 * g]);
-              u = f2::sub(f2::pack(q4.z, q4.w), x2);
-              acc2[2 * g + 1] = f2::fma(u, u, acc2[2 * g + 1]);
+              const uint64_t lo = f2::pack(q4.x, q4.y), hi = f2::pack(q4.z, q4.w);
+#pragma unroll
+              for (int h = 0; h < NH; ++h) {
+                const uint64_t x2 = f2::pack(x[h][i], x[h][i]);
+                uint64_t u = f2::sub(lo, x2);
+                acc2[h][2 * g] = f2::fma(u, u, acc2[h][2 * g]);
+                u = f2::sub(hi, x2);
+                acc2[h][2 * g + 1] = f2::fma(u, u, acc2[h][2 * g + 1]);
+              }
+            }
+          }
+        }
+      };
+      // past d (VEC: no such dimension) both sides hold zeros
+      if (halves == 2) {
+#pragma unroll 1
+        for (int c4 = 0; c4 < dc; c4 += 4) four(c4, std::integral_constant<int, 2>());
+      } else {
+#pragma unroll 1
+        for (int c4 = 0; c4 < dc; c4 += 4) four(c4, std::integral_constant<int, 1>());
+      }
+      __syncwarp();  // every lane has read the slice before it is replaced
+    }
+    __syncthreads();  // every warp has read its slices
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int i = 0; i < QC / 2; ++i) {
+        float a, b;
+        f2::unpack(acc2[h][i], a, b);
+        const int col = warp * 64 + 32 * h + lane;
+        if (2 * i < nqe) dsm[(2 * i) * S::DS + col] = METRIC == MANN_METRIC_EUCLIDEAN ? __fsqrt_rn(a) : a;
+        if (2 * i + 1 < nqe) dsm[(2 * i + 1) * S::DS + col] = METRIC == MANN_METRIC_EUCLIDEAN ? __fsqrt_rn(b) : b;
+      }
+    __syncthreads();
+    const int np = (int)min((int64_t)SCAN_P, p_end - p0);
+#pragma unroll
+    for (int m = 0; m < MW; ++m) {
+      const int j = warp + NW * m;
+      if (j >= nqe) continue;  // warp-uniform
+      const float* dist = dsm + j * S::DS;
+      if constexpr (KW == 1) {
+        pass_topk32(dist, np, lids + p0, L[m][0], k, s_buf[warp], lane);
+      } else {
+        uint64_t thr = wl::list_get<KW>(L[m], k - 1);
+        for (int c8 = 0; c8 < SCAN_P; c8 += 32) {
+          const int col = c8 + lane;
+          const uint64_t key = col < np ? make_key(dist[col], (uint32_t)lids[p0 + col]) : KEY_NONE;
+          unsigned pend = __ballot_sync(wl::FULL, key < thr);
+          while (pend) {
+            const int src = __ffs(pend) - 1;
+            pend &= pend - 1;
+            const uint64_t cnd = __shfl_sync(wl::FULL, key, src);
+            if (cnd < thr) {
+              wl::list_insert<KW>(L[m], cnd, lane);
+              thr = wl::list_get<KW>(L[m], k - 1);
             }
           }
         }
       }
     }
-    float acc[QC];
-#pragma unroll
-    for (int i = 0; i < QC / 2; ++i) f2::unpack(acc2[i], acc[2 * i], acc[2 * i + 1]);
-#pragma unroll
-    for (int j = 0; j < QC; ++j)
-      if (j < nqe) dsm[j][t] = METRIC == MANN_METRIC_EUCLIDEAN ? __fsqrt_rn(acc[j]) : acc[j];
-    __syncthreads();
-    const int np = (int)min((int64_t)SCAN_T, p_end - p0);
-#pragma unroll
-    for (int m = 0; m < MW; ++m) {
-      const int j = warp + 8 * m;
-      if (j >= nqe) continue;  // warp-uniform
-      uint64_t thr = wl::list_get<KW>(L[m], k - 1);
-      for (int c8 = 0; c8 < SCAN_T; c8 += 32) {
-        const int col = c8 + lane;
-        const uint64_t key = col < np ? make_key(dsm[j][col], (uint32_t)lids[p0 + col]) : KEY_NONE;
-        unsigned pend = __ballot_sync(wl::FULL, key < thr);
-        while (pend) {
-          const int src = __ffs(pend) - 1;
-          pend &= pend - 1;
-          const uint64_t cnd = __shfl_sync(wl::FULL, key, src);
-          if (cnd < thr) {
-            wl::list_insert<KW>(L[m], cnd, lane);
-            thr = wl::list_get<KW>(L[m], k - 1);
-          }
-        }
-      }
-    }
   }
+  __syncthreads();  // an empty list ran no pass
 #pragma unroll
   for (int m = 0; m < MW; ++m) {
-    const int j = warp + 8 * m;
+    const int j = warp + NW * m;
     if (j >= nqe) continue;
     uint64_t* dst = partial + ((int64_t)s_q[j] * nprobe + pair_r[e0 + j]) * k;
 #pragma unroll
@@ -250,36 +413,46 @@ __global__ void __launch_bounds__(SCAN_T, QC == 16 ? 3 : 2)
   }
 }
 
+template <int METRIC, int KW, bool VEC, int QC>
+mann_status launch_scan_q(cudaStream_t s, int64_t grid, const float* data, const int64_t* loff, const int32_t* lids,
+                          const float* qs, int d, const int64_t* qoff, const int32_t* pair_q, const int32_t* pair_r,
+                          const int64_t* choff, const int32_t* chunk_list, int nlist, int k, int nprobe,
+                          uint64_t* partial) {
+  auto kern = ivf_scan_kernel<METRIC, KW, VEC, QC>;
+  constexpr size_t smem = ScanSmem<QC>::BYTES;
+  MANN_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<(unsigned)grid, SCAN_T, smem, s>>>(data, loff, lids, qs, d, qoff, pair_q, pair_r, choff, chunk_list, nlist, k,
+                                            nprobe, partial);
+  MANN_CHECK_LAUNCH();
+  return MANN_OK;
+}
 
 template <int METRIC, int KW, bool VEC>
 mann_status launch_scan_t(cudaStream_t s, int qc, int64_t grid, const float* data, const int64_t* loff,
                           const int32_t* lids, const float* qs, int d, const int64_t* qoff,
-                          const int32_t* pair_q, const int32_t* pair_r, const int64_t* choff, int nlist, int k,
-                          int nprobe, uint64_t* partial) {
+                          const int32_t* pair_q, const int32_t* pair_r, const int64_t* choff,
+                          const int32_t* chunk_list, int nlist, int k, int nprobe, uint64_t* partial) {
   if (qc == 16)
-    ivf_scan_kernel<METRIC, KW, VEC, 16><<<(unsigned)grid, SCAN_T, 0, s>>>(data, loff, lids, qs, d, qoff, pair_q,
-                                                                           pair_r, choff, nlist, k, nprobe, partial);
-  else
-    ivf_scan_kernel<METRIC, KW, VEC, 32><<<(unsigned)grid, SCAN_T, 0, s>>>(data, loff, lids, qs, d, qoff, pair_q,
-                                                                           pair_r, choff, nlist, k, nprobe, partial);
-  MANN_CHECK_LAUNCH();
-  return MANN_OK;
+    return launch_scan_q<METRIC, KW, VEC, 16>(s, grid, data, loff, lids, qs, d, qoff, pair_q, pair_r, choff, chunk_list,
+                                              nlist, k, nprobe, partial);
+  return launch_scan_q<METRIC, KW, VEC, 32>(s, grid, data, loff, lids, qs, d, qoff, pair_q, pair_r, choff, chunk_list,
+                                            nlist, k, nprobe, partial);
 }
 
 template <int METRIC>
 mann_status launch_scan_m(cudaStream_t s, int qc, int64_t grid, bool vec, const float* data, const int64_t* loff,
                           const int32_t* lids, const float* qs, int d, const int64_t* qoff,
-                          const int32_t* pair_q, const int32_t* pair_r, const int64_t* choff, int nlist, int k,
-                          int nprobe, uint64_t* partial) {
+                          const int32_t* pair_q, const int32_t* pair_r, const int64_t* choff,
+                          const int32_t* chunk_list, int nlist, int k, int nprobe, uint64_t* partial) {
   if (k <= 32)
     return vec ? launch_scan_t<METRIC, 1, true>(s, qc, grid, data, loff, lids, qs, d, qoff, pair_q, pair_r, choff,
-                                                nlist, k, nprobe, partial)
+                                                chunk_list, nlist, k, nprobe, partial)
                : launch_scan_t<METRIC, 1, false>(s, qc, grid, data, loff, lids, qs, d, qoff, pair_q, pair_r, choff,
-                                                 nlist, k, nprobe, partial);
+                                                 chunk_list, nlist, k, nprobe, partial);
   return vec ? launch_scan_t<METRIC, 2, true>(s, qc, grid, data, loff, lids, qs, d, qoff, pair_q, pair_r, choff,
-                                              nlist, k, nprobe, partial)
+                                              chunk_list, nlist, k, nprobe, partial)
              : launch_scan_t<METRIC, 2, false>(s, qc, grid, data, loff, lids, qs, d, qoff, pair_q, pair_r, choff,
-                                               nlist, k, nprobe, partial);
+                                               chunk_list, nlist, k, nprobe, partial);
 }
 
 }  // namespace
@@ -303,31 +476,33 @@ mann_status ivf_scan_device(Context* ctx, cudaStream_t s, const float* data, int
   MANN_TRY(ctx->scratch_t(SLOT_IVF_CNT, (size_t)2 * nlist + 4, &cnt));
   MANN_TRY(ctx->scratch_t(SLOT_IVF_OFF, (size_t)2 * (nlist + 1), &qoff));
   choff = qoff + (nlist + 1);
-  MANN_TRY(ctx->scratch_t(SLOT_IVF_PAIRS, (size_t)2 * nq * nprobe, &pair_q));
+  // 16-query chunks when lists see few queries (more, lighter CTAs), else 32
+  const int qc = nq * nprobe <= (int64_t)12 * nlist ? 16 : SCAN_Q;
+  // chunks <= pairs/qc + lists; blocks past the real count return at once
+  const int64_t max_chunks = ceil_div(nq * nprobe, qc) + nlist;
+  int32_t* chunk_list = nullptr;
+  MANN_TRY(ctx->scratch_t(SLOT_IVF_PAIRS, (size_t)2 * nq * nprobe + (size_t)max_chunks, &pair_q));
   pair_r = pair_q + nq * nprobe;
+  chunk_list = pair_r + nq * nprobe;
   MANN_TRY(ctx->scratch_t(SLOT_IVF_PARTIAL, (size_t)nq * nprobe * k, &partial));
   MANN_TRY(ctx->scratch_t(SLOT_IVF_KEYS, (size_t)nq * k, &keys));
   MANN_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(unsigned) * (2 * nlist + 4), s));
   MANN_CUDA_TRY(cudaMemsetAsync(partial, 0xFF, sizeof(uint64_t) * nq * nprobe * k, s));
   probe_count_kernel<<<(unsigned)ceil_div(nq * nprobe, 256), 256, 0, s>>>(probes, nq * nprobe, nlist, cnt);
   MANN_CHECK_LAUNCH();
-  // 16-query chunks when lists see few queries (more, lighter CTAs), else 32
-  const int qc = nq * nprobe <= (int64_t)12 * nlist ? 16 : SCAN_Q;
   probe_scan_kernel<<<1, 1024, 0, s>>>(cnt, nlist, qc, qoff, choff);
   MANN_CHECK_LAUNCH();
   probe_scatter_kernel<<<(unsigned)ceil_div(nq * nprobe, 256), 256, 0, s>>>(
-      probes, nq, nprobe, nlist, qoff, cnt + nlist, pair_q, pair_r);
+      probes, nq, nprobe, nlist, qoff, choff, cnt + nlist, pair_q, pair_r, chunk_list);
   MANN_CHECK_LAUNCH();
-  // chunks <= pairs/32 + lists; blocks past the real count return at once
-  const int64_t max_chunks = ceil_div(nq * nprobe, qc) + nlist;
   const bool vec = (d % 4) == 0 && (reinterpret_cast<uintptr_t>(data) & 15) == 0;
   ctx->time_begin(s);
   if (metric == MANN_METRIC_EUCLIDEAN)
     MANN_TRY(launch_scan_m<MANN_METRIC_EUCLIDEAN>(s, qc, max_chunks, vec, data, loff, lids, qs, d, qoff, pair_q, pair_r,
-                                                  choff, nlist, k, nprobe, partial));
+                                                  choff, chunk_list, nlist, k, nprobe, partial));
   else
     MANN_TRY(launch_scan_m<MANN_METRIC_SQEUCLIDEAN>(s, qc, max_chunks, vec, data, loff, lids, qs, d, qoff, pair_q,
-                                                    pair_r, choff, nlist, k, nprobe, partial));
+                                                    pair_r, choff, chunk_list, nlist, k, nprobe, partial));
   ctx->time_end(s);
   MANN_TRY(launch_merge_lists(partial, nq, nprobe, k, keys, s));
   MANN_TRY(launch_finish(keys, nq, k, k, -1, nullptr, out_ids, out_dists, s));

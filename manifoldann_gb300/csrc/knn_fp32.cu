@@ -28,6 +28,9 @@ constexpr int K1_DRAIN = 8;  // ... and the number at which it is merged into th
 constexpr unsigned FULL = 0xFFFFFFFFu;
 using wl::list_get;
 using wl::list_insert;
+using wl::cmpex;
+using wl::merge32;
+using wl::sort32;
 
 // Squared row norms as the FP32 form's sequential sum (dimension order, one
 // fmaf per term).  One warp per 32 rows: 32 x 32 tiles come in through
@@ -188,21 +191,6 @@ __device__ __forceinline__ float select_tree(const float (&v)[N], int j) {
     for (int i = 0; i < w; ++i) t[i] = (j & bit) ? t[2 * i + 1] : t[2 * i];
   }
   return t[0];
-}
-
-// One compare-exchange stage of a warp bitonic network (lane holds one key).
-__device__ __forceinline__ uint64_t cmpex(uint64_t v, int j, bool keep_min) {
-  const uint64_t o = __shfl_xor_sync(FULL, (unsigned long long)v, j);
-  return keep_min == (o < v) ? o : v;
-}
-
-// Ascending sort of one key per lane.
-__device__ __forceinline__ uint64_t sort32(uint64_t c, int lane) {
-#pragma unroll
-  for (int w = 2; w <= 32; w <<= 1)
-#pragma unroll
-    for (int j = w >> 1; j > 0; j >>= 1) c = cmpex(c, j, ((lane & j) == 0) == ((lane & w) == 0));
-  return c;
 }
 
 // The cnt <= 32 queued candidates of a row into its sorted list of 32 KW
@@ -699,15 +687,6 @@ __global__ void __launch_bounds__(FEW_T, 2)
       if (e < k) dst[e] = L[m][s];
     }
   }
-}
-
-// Sorted ascending lists of 32 keys, one entry per lane: the 32 smallest of both.
-__device__ __forceinline__ uint64_t merge32(uint64_t a, uint64_t b, int lane) {
-  const uint64_t r = __shfl_sync(FULL, (unsigned long long)b, 31 - lane);
-  uint64_t m = r < a ? r : a;
-#pragma unroll
-  for (int j = 16; j > 0; j >>= 1) m = cmpex(m, j, (lane & j) == 0);
-  return m;
 }
 
 // Where a search's results go: its keys, or -- with ids set -- the ids and

@@ -1,7 +1,7 @@
 // warp_list.cuh -- a sorted list of uint64 keys distributed over the 32
 // lanes of a warp (entry e lives in register slot e/32 of lane e%32), with
-// ballot-based insertion.  Used by the fused top-k epilogues of the FP32 tile
-// kernel and of the IVF list scan.
+// ballot-based insertion, and bitonic sorts and merges of 32 keys.  Used by
+// the fused top-k epilogues of the FP32 kernels and of the IVF list scan.
 #pragma once
 #include <stdint.h>
 
@@ -41,6 +41,30 @@ __device__ __forceinline__ uint64_t list_get(const uint64_t (&L)[KW], int e) {
   for (int s = 1; s < KW; ++s)
     if (slot == s) v = L[s];
   return __shfl_sync(FULL, v, ln);
+}
+
+// One compare-exchange stage of a warp bitonic network (lane holds one key).
+__device__ __forceinline__ uint64_t cmpex(uint64_t v, int j, bool keep_min) {
+  const uint64_t o = __shfl_xor_sync(FULL, (unsigned long long)v, j);
+  return keep_min == (o < v) ? o : v;
+}
+
+// Ascending sort of one key per lane.
+__device__ __forceinline__ uint64_t sort32(uint64_t c, int lane) {
+#pragma unroll
+  for (int w = 2; w <= 32; w <<= 1)
+#pragma unroll
+    for (int j = w >> 1; j > 0; j >>= 1) c = cmpex(c, j, ((lane & j) == 0) == ((lane & w) == 0));
+  return c;
+}
+
+// Sorted ascending lists of 32 keys, one entry per lane: the 32 smallest of both.
+__device__ __forceinline__ uint64_t merge32(uint64_t a, uint64_t b, int lane) {
+  const uint64_t r = __shfl_sync(FULL, (unsigned long long)b, 31 - lane);
+  uint64_t m = r < a ? r : a;
+#pragma unroll
+  for (int j = 16; j > 0; j >>= 1) m = cmpex(m, j, (lane & j) == 0);
+  return m;
 }
 
 }  // namespace wl
