@@ -47,6 +47,7 @@ typedef int32_t mann_status;
                             top-(k+m), exact FP32 rerank (never chosen by AUTO: its certified
                             window is far wider than BF16's on the measured sets) */
 #define MANN_PREC_AUTO 3 /* library picks: the tensor-core form when k <= 24, d >= 128 and n >= 4096
+                            (n >= 2048 in searches of at least 2e9 multiply-adds)
                             (FP16 rows when BF16 cannot hold the centred, scaled data exactly, BF16
                             rows otherwise), else the FP32 form */
 #define MANN_PREC_FP16 4 /* FP16 tcgen05 tiles: rows centred and scaled by a power of two into

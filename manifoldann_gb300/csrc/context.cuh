@@ -49,6 +49,10 @@ enum ScratchSlot : int {
   SLOT_KM_I,
   SLOT_KM_J,
   SLOT_KM_DIST,       // assignment distances
+  SLOT_KM_BOUNDS,     // Lloyd: bounds of every point's two nearest distances, centroid movements
+  SLOT_KM_ACTIVE,     // Lloyd: points to assign anew
+  SLOT_KM_TOP2,       // Lloyd: two nearest centroids of those points
+  SLOT_KM_GATHER,     // Lloyd: their rows
   SLOT_KM_X,          // host-pointer KMeans calls: points
   SLOT_KM_CENT,       // centroids
   SLOT_KM_ASSIGN,     // assignments

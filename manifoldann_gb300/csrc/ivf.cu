@@ -516,7 +516,9 @@ mann_status ivf_route_device(Context* ctx, cudaStream_t s, const float* centroid
   mann_knn_params p{};
   p.metric = centroid_metric;
   p.k = nprobe;
-  p.precision = MANN_PREC_AUTO;
+  // a short search is over in the FP32 form before the tensor-core form's
+  // dozen launches are (100 queries x 4,096 x 128)
+  p.precision = (double)nq * nlist * d < 1e9 ? MANN_PREC_FP32 : MANN_PREC_AUTO;
   float* dd = nullptr;
   MANN_TRY(ctx->scratch_t(SLOT_IVF_ROUTE_D, (size_t)nq * nprobe, &dd));
   return exact_search_device(ctx, s, &p, centroids, nlist, qs, nq, d, -1, std::min(nprobe, nlist),
