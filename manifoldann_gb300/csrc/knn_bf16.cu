@@ -70,7 +70,11 @@ struct Stg {
 
 constexpr int AUG = 24;                              // norm-fold columns read after a BF16 row's main part
 constexpr int LIST = 32;                             // candidates kept per query row
-constexpr int SEED_SAMPLE = 2048;                    // most points sampled by the seed pass
+// points sampled by the seed pass: every 32nd, within these bounds, from 16
+// SEED_SAMPLE points (below that every SEED_STRIDE-th).  Of 290k points 2,048
+// leave a seed near the 560th neighbour, 9,062 near the 190th (290k x 256, 10k
+// queries: main pass 1.73 -> 1.60 ms, with a seed pass of 56 us)
+constexpr int SEED_SAMPLE = 2048, SEED_SAMPLE_MAX = 16384;
 // densest sample: every 8th point (below 16 SEED_SAMPLE points; without a seed
 // the 10,000 x 4,096 x 128 routing of an inverted file, all admissions, took
 // 375 us, with one and two epilogue sets 120)
@@ -3128,10 +3132,8 @@ static mann_status prep_finish(Context* ctx, cudaStream_t s, const float* mqs, i
   } else {
     MANN_TRY(ctx->scratch_t(SLOT_BF16_Q, (size_t)nq * width, &Q.xb));
     MANN_TRY(ctx->scratch_t(SLOT_ROWINFO_Q, (size_t)nq, &Q.info));
-    convert_rows_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, s>>>(mqs, nq, d, dp, augx, width, mu, scale, Q.xb,
-                                                                  Q.info, nullptr, nullptr, split, 0, f16 ? 1 : 0,
-                                                                  rn_q);
-    MANN_CHECK_LAUNCH();
+    MANN_TRY(launch_convert_rows(s, mqs, nq, d, dp, augx, width, mu, scale, Q.xb, Q.info, nullptr, nullptr, split, 0,
+                                 f16 ? 1 : 0, rn_q));
   }
   unsigned long long* counters = nullptr;
   MANN_TRY(ctx->scratch_t(SLOT_COUNTERS, 64, &counters));
