@@ -105,21 +105,42 @@ __global__ void gather_rows_kernel(const float* __restrict__ X, int d, const int
 // distances are summed in PP_CHUNK-point blocks and over the blocks, and the
 // running sum is searched for u * total -- all sums in FP64, in point order.
 //
-// One launch per step: a CTA updates PP_PTS points, the last CTA of a block
-// sums the block, and the last block's CTA searches (tickets below).  FP64
-// additions are slow and a chain of them slower still (one thread per 1024
-// additions took 110 us per step, as did the one-thread search), so sums are
-// made in 64-bit integers, in parallel, whenever that is exact: with every
-// term a multiple of 2^L and the total at most 2^53 units, each partial sum is
-// a double, so the ordered FP64 sum rounds nowhere and equals the integer one.
-// Where the terms' range does not allow it, one thread adds in order.
-// Measured (262,144 x 128, 1,024 centroids): 265 -> 50 us per step; the row
-// reads (134 MB per step) are what is left.
-constexpr int PP_PTS = 128;  // points (and threads) per CTA
-constexpr int PP_DC = 64;    // dimensions staged at a time
-constexpr int PP_STR = PP_DC + 4;
+// One CTA, or four, update a block of points; its last one sums it, and the last
+// of all searches the blocks' sums.  What bounds a step is the reading of rows
+// (134 MB at 262,144 x 128: 20 us) while most points are open, and a chain of
+// loads, barriers and tickets (about 16 us) at all times:
+// - in large sets a point whose centroid lies too far from the new one to lose
+//   it (pp_reach_kernel) is not read at all, and the rest is staged with three
+//   slices of columns in flight;
+// - FP64 additions are slow and a chain of them slower still (one thread per
+//   1024 additions took 110 us per step, as did the one-thread search), so sums
+//   are made in 64-bit integers, in parallel, whenever that is exact: with every
+//   term a multiple of 2^L and the total at most 2^53 units, each partial sum is
+//   a double, so the ordered FP64 sum rounds nowhere and equals the integer one.
+//   Where the terms' range does not allow it, one thread adds in order;
+// - a step's kernels start while their predecessor still runs and wait for it
+//   where they need it (262,144 x 128: 34.3 -> 29.4 ms for 1,023 steps).
+// Measured, all steps, against 128-point CTAs that read every point and start one
+// after the other: 262,144 x 128 in 1,024 groups, 1,024 centroids 44 -> 29.5 ms;
+// 131,072 x 64 22.6 -> 19.1; 60,000 x 64, 256 centroids 5.1 -> 4.1; 20,000 x 48,
+// 128 centroids 2.2 -> 2.0.
+constexpr int PP_T = 256;     // threads
+constexpr int PP_STAGES = 3;  // slices of rows in flight
+// The CTAs of a block of points, the rows they stage at a time and the columns
+// of a slice (106 and 109 KB in all, two CTAs per SM).
+template <int PARTS>
+struct PpShape {
+  static constexpr int PTS = PP_CHUNK / PARTS, PER = PTS / PP_T;  // points of a CTA, of a thread
+  static constexpr int ROWS = PARTS == 1 ? 128 : 256, DC = PARTS == 1 ? 64 : 32, STR = DC + 4;
+  static constexpr int TILE = (ROWS + 1) * STR;  // the last row: the centroid's
+};
+// coordinates from which leaving points out pays for a second kernel per step:
+// it costs 3 us, and 32 MB of rows are read in 5 (60,000 x 64 = 15 MB, 255
+// steps: 4.5 ms with it, 4.1 without; 131,072 x 64, 1,023 steps: 19.1 and 24.8;
+// 262,144 x 128: 29.4 and 40.3)
+constexpr int64_t PP_PRUNE = 1ll << 23;
 constexpr long long PP_EXACT = 1ll << 53;
-static_assert(PP_CHUNK % PP_PTS == 0, "a CTA belongs to one block of points");
+static_assert(PP_CHUNK % (4 * PP_T) == 0 && PP_CHUNK < 32768, "points per thread, indices");
 
 // v = mant * 2^exp2 with an odd mantissa (or 0); false for inf and NaN
 __device__ __forceinline__ bool pp_split(double v, long long& mant, int& exp2) {
@@ -133,6 +154,18 @@ __device__ __forceinline__ bool pp_split(double v, long long& mant, int& exp2) {
     exp2 += tz;
   }
   return e != 0x7FF && bits >= 0;
+}
+__device__ __forceinline__ bool pp_split(float v, long long& mant, int& exp2) {
+  const int bits = __float_as_int(v), e = (bits >> 23) & 0xFF;  // (bits < 0: refused below)
+  int m = (bits & 0x7FFFFF) | (e ? 1 << 23 : 0);
+  exp2 = (e ? e : 1) - 150;
+  if (m) {
+    const int tz = __ffs(m) - 1;
+    m >>= tz;
+    exp2 += tz;
+  }
+  mant = m;
+  return e != 0xFF && bits >= 0;
 }
 // 2^e as a double, -1022 <= e <= 1023
 __device__ __forceinline__ double pp_pow2(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
@@ -151,7 +184,7 @@ __device__ __forceinline__ int pp_block_min(int v, int* red) {
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
   v = red[0];
-  for (int w = 1; w < PP_PTS / 32; ++w) v = min(v, red[w]);
+  for (int w = 1; w < PP_T / 32; ++w) v = min(v, red[w]);
   return v;
 }
 
@@ -168,7 +201,7 @@ __device__ __forceinline__ long long pp_block_scan(long long v, long long* red, 
   __syncthreads();
   long long base = 0;
   total = 0;
-  for (int i = 0; i < PP_PTS / 32; ++i) {
+  for (int i = 0; i < PP_T / 32; ++i) {
     if (i < w) base += red[i];
     total += red[i];
   }
@@ -186,7 +219,7 @@ __device__ bool pp_exact_sum(double acc, int64_t i0, int64_t i1, Term term, int*
   constexpr int NO_LOW = 1 << 20;
   int low = NO_LOW;
   bool ok = true;
-  auto part = [&](double v, long long& m, int& e) {
+  auto part = [&](auto v, long long& m, int& e) {
     ok &= pp_split(v, m, e);
     if (m) low = min(low, e);
   };
@@ -212,7 +245,7 @@ __device__ bool pp_exact_sum(double acc, int64_t i0, int64_t i1, Term term, int*
   if (!__syncthreads_and(ok)) return false;
   long long sum;
   long long run = a0 + pp_block_scan(mine, redl, sum);
-  if (a0 + sum > PP_EXACT) return false;  // at most 129 * 2^53: no overflow
+  if (a0 + sum > PP_EXACT) return false;  // at most 257 * 2^53: no overflow
   const double unit = pp_pow2(low);
   total = (double)(a0 + sum) * unit;
   const double g = goal(total);
@@ -240,111 +273,223 @@ struct PpArgs {
   int64_t* idx;
   float* mind;        // [n]
   double* bsum;       // [blocks]
-  unsigned* tickets;  // [blocks + 1], zero between steps
+  unsigned* tickets;  // the step's and the blocks', zero between steps
+  int prune;          // leave points out by `reach`
+  int* near;          // [n] the centroid mind was measured to (prune)
+  float* reach;       // [k] by pp_reach_kernel
 };
 
-__global__ void __launch_bounds__(PP_PTS) pp_step_kernel(PpArgs a) {
-  extern __shared__ __align__(16) float pp_tile[];  // [PP_PTS][PP_STR], then the block's values
-  __shared__ float cs[PP_DC];
-  __shared__ int redi[PP_PTS / 32];
-  __shared__ long long redl[PP_PTS / 32];
+// reach[m]: a point of centroid m whose squared distance is below it lies at
+// least as far from the centroid chosen last.  By the triangle inequality that
+// holds below a quarter of the centroids' squared distance; every FP32 sum here
+// is within (d + 3) u of the exact one in relative terms (nothing near 1e-30 is
+// denormal), which 8 (d + 8) u outweighs, so the point's FP32 distance to the
+// new centroid would not be smaller either and mind stays the same, bit by bit.
+__global__ void __launch_bounds__(PP_T) pp_reach_kernel(PpArgs a) {
+  const int lane = threadIdx.x & 31, m = blockIdx.x * (PP_T / 32) + (threadIdx.x >> 5);
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // the step before: its choice
+  asm volatile("griddepcontrol.launch_dependents;");
+  if (m >= a.i - 1) return;
+  const float* x = a.X + a.idx[m] * a.d;
+  const float* c = a.X + a.idx[a.i - 1] * a.d;
+  float s = 0.0f;
+#pragma unroll 4
+  for (int e = lane; e < a.d; e += 32) {
+    const float v = __fsub_rn(__ldg(x + e), __ldg(c + e));
+    s = __fmaf_rn(v, v, s);
+  }
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) {
+    const float keep = 1.0f - 8.0f * (float)(a.d + 8) * 5.9604644775390625e-08f;
+    const float r = __fmul_rd(__fmul_rd(0.25f, keep), s);
+    // 0 (no point is below it) where the bound says nothing: overflow, NaN, huge d
+    a.reach[m] = keep > 0.5f && r >= 1e-30f && s < __int_as_float(0x7F800000) ? r : 0.0f;
+  }
+}
+
+// cp.async of n <= ROWS rows' columns [c0, c0 + DC) -- rows who[0 .. n) of the
+// points at x0 -- and of the centroid's (row ROWS); columns past d are zero on
+// both sides and add nothing.
+template <typename S>
+__device__ __forceinline__ void pp_stage(float* tile, const float* __restrict__ x0, const float* __restrict__ c,
+                                         const short* who, int n, int c0, int d, int vec) {
+  const int cw = min(S::DC, d - c0);
+  if (vec) {
+    constexpr int Q = S::DC / 4;
+    for (int e = threadIdx.x; e < (n + 1) * Q; e += PP_T) {
+      const int r = e / Q, cc = (e % Q) * 4;
+      float* dst = tile + (r < n ? r : S::ROWS) * S::STR + cc;
+      const float* src = (r < n ? x0 + (int64_t)who[r] * d : c) + c0 + cc;
+      if (cc < cw) {
+        const uint32_t sa = (uint32_t)__cvta_generic_to_shared(dst);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sa), "l"(src) : "memory");
+      } else {
+        *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    }
+  } else {
+    for (int e = threadIdx.x; e < (n + 1) * S::DC; e += PP_T) {
+      const int r = e / S::DC, cc = e % S::DC;
+      const float* src = (r < n ? x0 + (int64_t)who[r] * d : c) + c0 + cc;
+      tile[(r < n ? r : S::ROWS) * S::STR + cc] = cc < cw ? __ldg(src) : 0.0f;
+    }
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// PARTS CTAs share a block of points; with several, the last of them sums it.
+template <int PARTS>
+__global__ void __launch_bounds__(PP_T) pp_step_kernel(PpArgs a) {
+  extern __shared__ __align__(16) float pp_smem[];  // [PP_STAGES] tiles
+  using S = PpShape<PARTS>;
+  __shared__ float own[S::PTS];  // the CTA's points' distances
+  __shared__ short who[S::PTS];
+  float* vals = PARTS == 1 ? own : pp_smem;  // a block's
+  __shared__ int redi[PP_T / 32];
+  __shared__ long long redl[PP_T / 32];
   __shared__ int s_last;
   __shared__ long long s_pick;
   __shared__ double s_acc;
-  const int t = threadIdx.x;
+  constexpr int PER = S::PER;
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   const int64_t n = a.n;
   const int d = a.d;
-  const int64_t j0 = (int64_t)blockIdx.x * PP_PTS;
-  const int64_t j = j0 + t;
-  const float* c = a.X + a.idx[a.i - 1] * d;
+  const int64_t nb = (n + PP_CHUNK - 1) / PP_CHUNK;
+  const int64_t b0 = (int64_t)blockIdx.x * S::PTS;
+  const int len = (int)min((int64_t)S::PTS, n - b0);
+  // The next kernel's CTAs may take their places; they wait for this kernel's
+  // end.  After a reach kernel this one was launched once every CTA of it had
+  // seen the step before complete, so all but `reach` is there already.
+  asm volatile("griddepcontrol.launch_dependents;");
+  const bool prune = a.prune && a.i > 1;
+  if (!prune) asm volatile("griddepcontrol.wait;" ::: "memory");
+  const float* c = a.X + __ldcg(a.idx + a.i - 1) * d;
 
-  // squared distances in the FP32 form (dimension order), rows staged with
-  // every load of a slice in flight; columns past d are zero on both sides
-  float s = 0.0f;
-  const int rows = (int)min((int64_t)PP_PTS, n - j0);
-  for (int c0 = 0; c0 < d; c0 += PP_DC) {
-    const int cw = min(PP_DC, d - c0);
-    __syncthreads();
-    if (a.vec) {
-      const int q = cw >> 2;
-      for (int e = t; e < PP_PTS * (PP_DC / 4); e += PP_PTS) {
-        const int r = e / (PP_DC / 4), cc = e % (PP_DC / 4);
-        float* dst = pp_tile + r * PP_STR + cc * 4;
-        if (r < rows && cc < q) {
-          const uint32_t sa = (uint32_t)__cvta_generic_to_shared(dst);
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sa), "l"(a.X + (j0 + r) * d + c0 + cc * 4)
-                       : "memory");
-        } else {
-          *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-    } else {
-      for (int e = t; e < PP_PTS * PP_DC; e += PP_PTS) {
-        const int r = e / PP_DC, cc = e % PP_DC;
-        pp_tile[r * PP_STR + cc] = (r < rows && cc < cw) ? __ldg(a.X + (j0 + r) * d + c0 + cc) : 0.0f;
+  // the points that the new centroid may be nearer to
+  int rows = 0;
+  {
+    unsigned opens[PER];
+    float old[PER];
+    int near[PER];
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int e = u * PP_T + t;
+      old[u] = __int_as_float(0x7F800000);
+      near[u] = 0;
+      if (a.i > 1 && e < len) {
+        old[u] = __ldcg(a.mind + b0 + e);
+        if (prune) near[u] = __ldcg(a.near + b0 + e);
       }
     }
-    if (t < PP_DC) cs[t] = t < cw ? __ldg(c + c0 + t) : 0.0f;
+    if (prune) asm volatile("griddepcontrol.wait;" ::: "memory");
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int e = u * PP_T + t;
+      const bool open = e < len && !(prune && old[u] < a.reach[near[u]]);
+      own[e] = old[u];
+      opens[u] = __ballot_sync(0xffffffffu, open);
+    }
+    int mine = 0;
+#pragma unroll
+    for (int u = 0; u < PER; ++u) mine += __popc(opens[u]);
+    if (lane == 0) redi[w] = mine;
     __syncthreads();
-    const float* row = pp_tile + t * PP_STR;
+    int slot = 0;
+    for (int v = 0; v < PP_T / 32; ++v) {
+      if (v < w) slot += redi[v];
+      rows += redi[v];
+    }
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      if (opens[u] >> lane & 1u) who[slot + __popc(opens[u] & ((1u << lane) - 1u))] = (short)(u * PP_T + t);
+      slot += __popc(opens[u]);
+    }
+    __syncthreads();
+  }
+
+  // squared distances in the FP32 form (dimension order): groups of ROWS
+  // rows, a slice of columns at a time; groups of half the CTA take turns
+  const int slices = (d + S::DC - 1) / S::DC, steps = (rows + S::ROWS - 1) / S::ROWS * slices;
+  auto stage = [&](int it) {
+    if (it < steps) {
+      const int g = it / slices * S::ROWS;
+      pp_stage<S>(pp_smem + it % PP_STAGES * S::TILE, a.X + b0 * d, c, who + g, min(S::ROWS, rows - g),
+               it % slices * S::DC, d, a.vec);
+    } else {
+      asm volatile("cp.async.commit_group;" ::: "memory");  // the waits count groups
+    }
+  };
+  for (int it = 0; it < PP_STAGES - 1; ++it) stage(it);
+  float s = 0.0f;
+  for (int it = 0; it < steps; ++it) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(PP_STAGES - 2) : "memory");
+    __syncthreads();  // slice it has landed for every thread; slice it - 1 is read
+    stage(it + PP_STAGES - 1);
+    const int g = it / slices, sl = it - g * slices, r = g * S::ROWS + t % S::ROWS;
+    if (t / S::ROWS != g % (PP_T / S::ROWS) || r >= rows) continue;
+    const float* tile = pp_smem + it % PP_STAGES * S::TILE;
+    const float *x = tile + t % S::ROWS * S::STR, *cs = tile + S::ROWS * S::STR;
+    const int cw = min(S::DC, d - sl * S::DC);
+    if (sl == 0) s = 0.0f;
 #pragma unroll 4
     for (int cc = 0; cc < cw; cc += 4) {
-      const float4 x = *reinterpret_cast<const float4*>(row + cc);
-      float v = __fsub_rn(x.x, cs[cc]);
+      const float4 xv = *reinterpret_cast<const float4*>(x + cc), cv = *reinterpret_cast<const float4*>(cs + cc);
+      float v = __fsub_rn(xv.x, cv.x);
       s = __fmaf_rn(v, v, s);
-      v = __fsub_rn(x.y, cs[cc + 1]);
+      v = __fsub_rn(xv.y, cv.y);
       s = __fmaf_rn(v, v, s);
-      v = __fsub_rn(x.z, cs[cc + 2]);
+      v = __fsub_rn(xv.z, cv.z);
       s = __fmaf_rn(v, v, s);
-      v = __fsub_rn(x.w, cs[cc + 3]);
+      v = __fsub_rn(xv.w, cv.w);
       s = __fmaf_rn(v, v, s);
     }
+    if (sl == slices - 1) {
+      const int e = who[r];
+      const float old = own[e];
+      if (a.i == 1 || s < old) {
+        const float now = s < old ? s : old;
+        own[e] = now;
+        a.mind[b0 + e] = now;
+        if (a.prune) a.near[b0 + e] = a.i - 1;
+      }
+    }
   }
-  if (j < n) {
-    const float old = a.i == 1 ? __int_as_float(0x7F800000) : a.mind[j];
-    a.mind[j] = s < old ? s : old;
-  }
+  __syncthreads();
 
-  // the last CTA of the block of points sums it
-  const int64_t nb = (n + PP_CHUNK - 1) / PP_CHUNK;
-  const int64_t blk = j0 / PP_CHUNK;
-  const int64_t b0 = blk * PP_CHUNK;
-  const int len = (int)min((int64_t)PP_CHUNK, n - b0);
-  __threadfence();
-  __syncthreads();
-  if (t == 0) {
-    const unsigned turn = (unsigned)((len + PP_PTS - 1) / PP_PTS);
-    s_last = atomicAdd(&a.tickets[blk], 1u) + 1u == turn;
-    if (s_last) a.tickets[blk] = 0u;
+  // the block's sum
+  const int64_t blk = blockIdx.x / PARTS, s0 = blk * PP_CHUNK;
+  const int slen = (int)min((int64_t)PP_CHUNK, n - s0);
+  if constexpr (PARTS > 1) {
+    __threadfence();
+    __syncthreads();
+    if (t == 0) {
+      s_last = atomicAdd(a.tickets + 1 + blk, 1u) + 1u == (unsigned)((slen + S::PTS - 1) / S::PTS);
+      if (s_last) a.tickets[1 + blk] = 0u;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    for (int e = t; e < slen; e += PP_T) vals[e] = __ldcg(a.mind + s0 + e);
+    __syncthreads();
   }
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  float* vals = pp_tile;
-  constexpr int PER = PP_CHUNK / PP_PTS;
-  auto load_block = [&](int64_t first, int count) {
-    __syncthreads();
-    for (int e = t; e < count; e += PP_PTS) vals[e] = __ldcg(a.mind + first + e);
-    __syncthreads();
-  };
-  auto value = [&](int64_t e) { return (double)vals[e]; };
-  load_block(b0, len);
+  constexpr int RUN = PP_CHUNK / PP_T;
+  auto value = [&](int64_t e) { return vals[e]; };
   double total = 0.0, before = 0.0;
   int64_t at;
   const double never = __longlong_as_double(0x7FF8000000000000ll);  // a goal that no sum reaches
-  if (!pp_exact_sum(0.0, min(len, t * PER), min(len, (t + 1) * PER), value, redi, redl, total,
+  if (!pp_exact_sum(0.0, min(slen, t * RUN), min(slen, (t + 1) * RUN), value, redi, redl, total,
                     [&](double) { return never; }, at, before)) {
     total = 0.0;
     if (t == 0)
-      for (int e = 0; e < len; ++e) total += (double)vals[e];
+      for (int e = 0; e < slen; ++e) total += (double)vals[e];
   }
+  __threadfence();
+  __syncthreads();
   if (t == 0) {
     a.bsum[blk] = total;
     __threadfence();
-    s_last = atomicAdd(&a.tickets[nb], 1u) + 1u == (unsigned)nb;
-    if (s_last) a.tickets[nb] = 0u;
+    s_last = atomicAdd(a.tickets, 1u) + 1u == (unsigned)nb;
+    if (s_last) *a.tickets = 0u;
   }
   __syncthreads();
   if (!s_last) return;
@@ -356,7 +501,7 @@ __global__ void __launch_bounds__(PP_PTS) pp_step_kernel(PpArgs a) {
     s_acc = 0.0;
   }
   __syncthreads();
-  const int64_t per = (nb + PP_PTS - 1) / PP_PTS;
+  const int64_t per = (nb + PP_T - 1) / PP_T;
   const double draw = a.u[a.i];
   auto block_sum = [&](int64_t b) { return __ldcg(a.bsum + b); };
   const bool exact = pp_exact_sum(0.0, min(nb, t * per), min(nb, (t + 1) * per), block_sum, redi, redl, total,
@@ -391,10 +536,11 @@ __global__ void __launch_bounds__(PP_PTS) pp_step_kernel(PpArgs a) {
   }
   const int64_t f0 = pb * PP_CHUNK;
   const int flen = (int)min((int64_t)PP_CHUNK, n - f0);
-  load_block(f0, flen);
+  for (int e = t; e < flen; e += PP_T) vals[e] = __ldcg(a.mind + f0 + e);
+  __syncthreads();  // s_pick is read
   if (t == 0) s_pick = n - 1;
   __syncthreads();
-  if (pp_exact_sum(acc, min(flen, t * PER), min(flen, (t + 1) * PER), value, redi, redl, total,
+  if (pp_exact_sum(acc, min(flen, t * RUN), min(flen, (t + 1) * RUN), value, redi, redl, total,
                    [&](double) { return thr; }, at, before)) {
     if (at >= 0) atomicMin(&s_pick, (long long)(f0 + at));
   } else if (t == 0) {
@@ -799,7 +945,7 @@ mann_status kmeanspp_device(Context* ctx, cudaStream_t s, const float* X, int64_
   double *bsum = nullptr, *u = nullptr;
   unsigned* tickets = nullptr;
   const int64_t nb = ceil_div(n, PP_CHUNK);
-  MANN_TRY(ctx->scratch_t(SLOT_KM_A, (size_t)n, &mind));
+  MANN_TRY(ctx->scratch_t(SLOT_KM_A, (size_t)n * 2 + k, &mind));  // mind, near, reach
   MANN_TRY(ctx->scratch_t(SLOT_KM_B, (size_t)nb * 2 + 1, &bsum));
   tickets = reinterpret_cast<unsigned*>(bsum + nb);
   MANN_TRY(ctx->scratch_t(SLOT_KM_C, (size_t)k, &u));
@@ -807,10 +953,32 @@ mann_status kmeanspp_device(Context* ctx, cudaStream_t s, const float* X, int64_
   MANN_CUDA_TRY(cudaMemcpyAsync(idx_dev, &first, sizeof(int64_t), cudaMemcpyHostToDevice, s));
   MANN_CUDA_TRY(cudaMemsetAsync(tickets, 0, sizeof(unsigned) * (nb + 1), s));
   PpArgs a{X, n, d, 0, (d % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0) ? 1 : 0, u, idx_dev, mind, bsum,
-           tickets};
+           tickets, n * d >= PP_PRUNE ? 1 : 0, reinterpret_cast<int*>(mind + n), mind + 2 * n};
+  // four CTAs per block while all of them run at once: one reads its 1,024 rows
+  // with the bandwidth of one SM (60,000 x 64, 256 centroids: 6.2 ms with one CTA,
+  // 4.1 with four; 131,072 x 64, 1,024: 19.1 and 21.0)
+  const int parts = nb * 4 <= ctx->num_sms * 2 ? 4 : 1;
+  const auto step = parts == 1 ? pp_step_kernel<1> : pp_step_kernel<4>;
+  const int smem = (int)sizeof(float) * PP_STAGES * (parts == 1 ? PpShape<1>::TILE : PpShape<4>::TILE);
+  MANN_CUDA_TRY(cudaFuncSetAttribute(step, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   for (a.i = 1; a.i < k; ++a.i) {
-    pp_step_kernel<<<(unsigned)ceil_div(n, PP_PTS), PP_PTS, sizeof(float) * PP_PTS * PP_STR, s>>>(a);
-    MANN_CHECK_LAUNCH();
+    // (a launch with the attribute starts while its predecessor still runs, as
+    // far as the kernels' own waits let it)
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.blockDim = dim3(PP_T);
+    cfg.stream = s;
+    cfg.attrs = &early;
+    cfg.numAttrs = a.i > 1 ? 1 : 0;
+    if (a.prune && a.i > 1) {
+      cfg.gridDim = dim3((unsigned)ceil_div(a.i - 1, PP_T / 32));
+      MANN_CUDA_TRY(cudaLaunchKernelEx(&cfg, pp_reach_kernel, a));
+    }
+    cfg.gridDim = dim3((unsigned)ceil_div(n, PP_CHUNK / parts));
+    cfg.dynamicSmemBytes = smem;
+    MANN_CUDA_TRY(cudaLaunchKernelEx(&cfg, step, a));
   }
   return MANN_OK;
 }
