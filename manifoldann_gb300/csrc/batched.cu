@@ -291,6 +291,12 @@ mann_status knn_graph_batched_device(Context* ctx, cudaStream_t s, const mann_kn
     for (const int(&c)[2] : cand) {
       make_plan(offs, nsets, c[0], c[1], &pl);
       MANN_TRY(prepare(ctx, s, sh, offs, pl, &b, st));
+      // loaded first, on an empty queue: the first launch of a kernel takes about
+      // a millisecond, which made two splits (23.6 ms at 338,792 rows x 32) win
+      // over none (22.7)
+      MANN_TRY(launch_publish_queue(b.queue, 0, nullptr, ++st.epoch, s));
+      MANN_TRY(launch_k1_persistent(ctx->num_sms, sh.data, b.items, b.queue, st.epoch, QUEUE_WAIT_CYCLES, sh.d,
+                                    sh.metric, pl.bq, sh.kk, pl.S, pl.S > 1 ? b.partial : b.keys, s));
       cudaEventRecord(e0, s);
       MANN_TRY(issue(ctx->num_sms, sh, pl, b, ++st.epoch, true, QUEUE_WAIT_CYCLES, s));
       cudaEventRecord(e1, s);
