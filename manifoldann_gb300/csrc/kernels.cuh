@@ -118,11 +118,14 @@ struct SegQueue {
   int pad[3];
 };
 // Persistent segmented kernel: resident CTAs consume the items of `q` (k <= 64).
-// `qrows` (optional) maps an item's query index i to the query row qrows[i]
-// (the lists still go to slot i).
 mann_status launch_k1_persistent(int num_sms, const float* data, const SegItem* items, SegQueue* q, unsigned epoch,
                                  long long wait_cycles, int d, int metric, int bq, int k, int nsplit,
-                                 uint64_t* partial, cudaStream_t s, const int32_t* qrows = nullptr);
+                                 uint64_t* partial, cudaStream_t s);
+// Exact lists (32 entries, Euclidean or SqEuclidean) of `cnt` rows of `data`, each
+// against the set of offs[0 .. nsets] that holds it, in nsplit chunks of points:
+// partial [cnt][nsplit][32].
+mann_status launch_seg_rows(const float* data, const int32_t* rows, int cnt, const int64_t* offs, int nsets, int nsplit,
+                            int64_t chunk, int d, int metric, uint64_t* partial, cudaStream_t s);
 // Publishes a work queue of `count` items (head 0, status 0, then the epoch).
 // count_dev (optional) supplies the count from device memory instead.
 mann_status launch_publish_queue(SegQueue* q, int count, const int* count_dev, unsigned epoch, cudaStream_t s);

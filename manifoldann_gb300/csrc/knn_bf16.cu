@@ -2140,34 +2140,6 @@ __global__ void k2_scatter_fallback(const uint64_t* __restrict__ keys, const int
   }
 }
 
-// Work items of the segmented fallback: item i * nsplit + c is row
-// r = fb_rows[i] against points [c * chunk, (c + 1) * chunk) of the set
-// holding it (empty past the set's end); its exact FP32 list goes to split
-// slot c of compact row i.
-__global__ void fb_items_kernel(const int* __restrict__ fb_rows, int cnt, const int64_t* __restrict__ offs,
-                                int nsets, int nsplit, int64_t chunk, SegItem* __restrict__ items) {
-  const int64_t total = (int64_t)cnt * nsplit;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int i = (int)(t / nsplit), c = (int)(t % nsplit);
-    const int64_t r = fb_rows[i];
-    int lo = 0, hi = nsets - 1;
-    while (lo < hi) {  // last set whose offset <= r
-      const int mid = (lo + hi + 1) >> 1;
-      if (offs[mid] <= r) lo = mid;
-      else hi = mid - 1;
-    }
-    SegItem it{};
-    it.q0 = i;
-    it.qend = i + 1;
-    it.nb1 = offs[lo + 1];
-    it.nb0 = min(it.nb1, offs[lo] + c * chunk);
-    it.nb1 = min(it.nb1, it.nb0 + chunk);
-    it.split = c;
-    items[t] = it;
-  }
-}
-
 // The fallback rows' exact FP32 top-LIST lists (compact row i) go to their
 // candidate slots, with their counts and floors (the LIST-th distance bounds
 // every other point).
@@ -3843,14 +3815,12 @@ mann_status knn_bf16_batched_keys(Context* ctx, cudaStream_t s, const float* dat
   k2_rerank<<<(unsigned)std::min<int64_t>(ceil_div(N, RR_WARPS), (int64_t)ctx->num_sms * 6), 32 * RR_WARPS, 0,
               s>>>(ra);
   MANN_CHECK_LAUNCH();
-  // ---- uncertified rows: exact FP32 scan of their own set, on the device;
-  // each row's set is cut into FB_CHUNK-point items so that a few rows of the
-  // largest sets spread over the GPU (one item per row: 1.8 ms for 124 rows)
+  // ---- uncertified rows: exact FP32 scan of their own set, on the device,
+  // FB_CHUNK points to a CTA so that a few rows of the largest sets spread over
+  // the GPU
   int h_fbc = 0;
   MANN_CUDA_TRY(cudaMemcpyAsync(&h_fbc, P.fb_count, sizeof(int), cudaMemcpyDeviceToHost, s));
   MANN_CUDA_TRY(cudaStreamSynchronize(s));
-  SegQueue* fq = nullptr;
-  MANN_TRY(ctx->scratch_t(SLOT_SEG_QUEUE, 1, &fq));
   if (h_fbc > 0) {
     int64_t max_set = 1;
     for (int i = 0; i < nsets; ++i) max_set = std::max(max_set, offs_host[i + 1] - offs_host[i]);
@@ -3858,20 +3828,13 @@ mann_status knn_bf16_batched_keys(Context* ctx, cudaStream_t s, const float* dat
     const int nsplit = (int)ceil_div(max_set, chunk);
     const int64_t nitems = (int64_t)h_fbc * nsplit;
     if (nitems > INT32_MAX) return fail(MANN_EINVAL_ARG, "batched graphs: too many fallback items");
-    SegItem* fitems = nullptr;
     uint64_t* fpart = nullptr;
     uint64_t* fkeys = nullptr;
-    MANN_TRY(ctx->scratch_t(SLOT_FALLBACK_KEYS, (size_t)nitems, &fitems));
     MANN_TRY(ctx->scratch_t(SLOT_PARTIAL, (size_t)nitems * L, &fpart));  // the main pass's slots are merged
     MANN_TRY(ctx->scratch_t(SLOT_SEED_PARTIAL, (size_t)h_fbc * L, &fkeys));
     const int gfb = ctx->num_sms * 8;
-    fb_items_kernel<<<gfb, 256, 0, s>>>(fb_rows, h_fbc, offs_dev, nsets, nsplit, chunk, fitems);
-    MANN_CHECK_LAUNCH();
-    static unsigned fb_epoch = 0x40000000u;
-    const unsigned ep = ++fb_epoch;
-    MANN_TRY(launch_publish_queue(fq, (int)nitems, nullptr, ep, s));
-    MANN_TRY(launch_k1_persistent(ctx->num_sms, data, fitems, fq, ep, 1ll << 31, d, metric, 32, L, nsplit,
-                                  nsplit > 1 ? fpart : fkeys, s, fb_rows));
+    MANN_TRY(launch_seg_rows(data, fb_rows, h_fbc, offs_dev, nsets, nsplit, chunk, d, metric,
+                             nsplit > 1 ? fpart : fkeys, s));
     if (nsplit > 1) MANN_TRY(launch_merge_lists(fpart, h_fbc, nsplit, L, fkeys, s));
     fb_finish_kernel<<<gfb, 256, 0, s>>>(fb_rows, h_fbc, fkeys, cand, cand_count, floor_val);
     MANN_CHECK_LAUNCH();
@@ -3884,14 +3847,11 @@ mann_status knn_bf16_batched_keys(Context* ctx, cudaStream_t s, const float* dat
   // ---- status, report, and the depth for the next call of this layout
   unsigned long long hc[64];
   MANN_CUDA_TRY(cudaMemcpyAsync(hc, P.counters, sizeof(hc), cudaMemcpyDeviceToHost, s));
-  int qstatus = 0;  // (the queue is published only when some row fell back)
-  if (h_fbc > 0) MANN_CUDA_TRY(cudaMemcpyAsync(&qstatus, &fq->status, sizeof(int), cudaMemcpyDeviceToHost, s));
   MANN_CUDA_TRY(cudaStreamSynchronize(s));
   const int h_err = reinterpret_cast<const int*>(hc + 8)[0];
   const int h_fb = reinterpret_cast<const int*>(hc + 8)[1];
   if (h_err != 0)
     return fail(MANN_ETIMEOUT, "tensor-core kernel: a bounded wait ran out (role " + std::to_string(h_err) + ")");
-  if (qstatus != 0) return fail(MANN_ETIMEOUT, "batched graphs: the fallback work queue was not published in time");
   if (margin <= 0) ctx->tune[tkey] = (uint64_t)tuned_depth(hc + 16, kreq);
   if (rep) {
     rep->rows_fallback = h_fb;

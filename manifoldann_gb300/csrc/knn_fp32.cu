@@ -499,7 +499,9 @@ __global__ void __launch_bounds__(K1_THREADS, k1_ctas<BQ, KW>())
 // CTA waits until the queue of this call is published (q->epoch == epoch,
 // written with the plan ahead of the kernel in stream order); the wait is
 // bounded by `wait_cycles`, after which the CTA records MANN_ETIMEOUT in
-// q->status and returns without touching any list.
+// q->status and returns without touching any list.  `qrows` is null; with the
+// constant in its place the compiler spills in the inner loop (338,792 rows x 32:
+// 22.7 -> 23.6 ms).
 template <int METRIC, int BQ, int KW, bool VEC>
 __global__ void __launch_bounds__(K1_THREADS, k1_ctas<BQ, KW>())
     k1_persistent(const float* __restrict__ data, const SegItem* __restrict__ items, SegQueue* q, unsigned epoch,
@@ -890,6 +892,103 @@ __global__ void __launch_bounds__(FEW_T, 2)
   }
 }
 
+// Exact lists of single rows, each against its own set: CTA (i, c) scans points
+// [c chunk, (c + 1) chunk) of the set that holds row rows[i] of `data`, and
+// writes the 32 nearest to partial[i][c].  A warp takes 64 points at a time,
+// brought in 16 columns at a time with four lanes to a row (a thread that reads
+// its own row touches 32 lines per load), and keeps its own list; the slices are
+// the warp's own, so no barrier falls inside.  Bound by the latency of the
+// slices, which the 40 warps of an SM cover.  Replaces 32-row tiles holding one
+// row each (124 rows of sets of up to 50,000 x 32: 295 to 445 us, now 57).
+constexpr int SR_T = 256, SR_W = SR_T / 32, SR_DC = 16, SR_XS = SR_DC + 4;
+template <int METRIC, bool VEC>
+__global__ void __launch_bounds__(SR_T, 5)
+    seg_rows_kernel(const float* __restrict__ data, const int32_t* __restrict__ rows, const int64_t* __restrict__ offs,
+                    int nsets, int nsplit, int64_t chunk, int d, uint64_t* __restrict__ partial) {
+  __shared__ __align__(16) float xs[SR_W][64][SR_XS];
+  __shared__ __align__(16) float qs[SR_W][SR_DC];
+  __shared__ uint64_t lists[SR_W][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t i = blockIdx.x / nsplit;
+  const int64_t row = rows[i];
+  // the last set that starts at or before the row: 32 candidates a step
+  int lo = 0;
+  for (int len = nsets; len > 1;) {
+    const int st = (len + 31) / 32, p = lane * st;
+    const unsigned le = __ballot_sync(FULL, p < len && offs[lo + p] <= row);
+    const int hit = (31 - __clz(le)) * st;  // lane 0's always is
+    lo += hit;
+    len = min(st, len - hit);
+  }
+  const int64_t end = offs[lo + 1];
+  const int64_t p_begin = min(end, offs[lo] + (int64_t)(blockIdx.x % nsplit) * chunk), p_end = min(end, p_begin + chunk);
+  const float* q = data + row * d;
+  uint64_t L = KEY_NONE, thr = KEY_NONE;
+  for (int64_t p0 = p_begin + w * 64; p0 < p_end; p0 += SR_W * 64) {
+    const int np = (int)min((int64_t)64, p_end - p0);
+    float acc[2] = {0.0f, 0.0f};
+    for (int c0 = 0; c0 < d; c0 += SR_DC) {
+      __syncwarp();
+      if constexpr (VEC) {
+        const int c = (lane & 3) * 4;
+#pragma unroll
+        for (int it = 0; it < 8; ++it) {
+          const int r = it * 8 + (lane >> 2);
+          if (r < np && c0 + c < d) {
+            const uint32_t sa = (uint32_t)__cvta_generic_to_shared(&xs[w][r][c]);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sa), "l"(data + (p0 + r) * d + c0 + c)
+                         : "memory");
+          } else {
+            *reinterpret_cast<float4*>(&xs[w][r][c]) = make_float4(0.f, 0.f, 0.f, 0.f);
+          }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+      } else {
+        const int c = lane & 15;
+#pragma unroll 8
+        for (int it = 0; it < 32; ++it) {
+          const int r = it * 2 + (lane >> 4);
+          xs[w][r][c] = r < np && c0 + c < d ? __ldg(data + (p0 + r) * d + c0 + c) : 0.0f;
+        }
+      }
+      if (lane < SR_DC) qs[w][lane] = c0 + lane < d ? __ldg(q + c0 + lane) : 0.0f;
+      if constexpr (VEC) asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncwarp();
+      // columns past d are zero on both sides and add nothing
+#pragma unroll
+      for (int c = 0; c < SR_DC; c += 4) {
+        const float4 q4 = *reinterpret_cast<const float4*>(&qs[w][c]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const float4 v = *reinterpret_cast<const float4*>(&xs[w][32 * h + lane][c]);
+          float u = __fsub_rn(q4.x, v.x);
+          acc[h] = __fmaf_rn(u, u, acc[h]);
+          u = __fsub_rn(q4.y, v.y);
+          acc[h] = __fmaf_rn(u, u, acc[h]);
+          u = __fsub_rn(q4.z, v.z);
+          acc[h] = __fmaf_rn(u, u, acc[h]);
+          u = __fsub_rn(q4.w, v.w);
+          acc[h] = __fmaf_rn(u, u, acc[h]);
+        }
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = 32 * h + lane;
+      const float v = few_distance<METRIC>(acc[h], nullptr, 0, nullptr, 0, false);
+      const uint64_t key = r < np ? make_key(v, (uint32_t)(p0 + r)) : KEY_NONE;
+      if (!__any_sync(FULL, key < thr)) continue;
+      L = merge32(L, sort32(key < thr ? key : KEY_NONE, lane), lane);
+      thr = __shfl_sync(FULL, (unsigned long long)L, 31);
+    }
+  }
+  lists[w][lane] = L;
+  __syncthreads();
+  if (w > 0) return;
+  for (int v = 1; v < SR_W; ++v) L = merge32(L, lists[v][lane], lane);
+  partial[(int64_t)blockIdx.x * 32 + lane] = L;
+}
+
 constexpr size_t few_list_bytes(int kw) { return sizeof(uint64_t) * (FEW_T / 32) * FEW_QS * 32 * kw; }
 
 // fused: the kernel itself merges the blocks' lists into `out` (with a ticket)
@@ -1109,28 +1208,28 @@ mann_status run_k1(Context* ctx, int metric, int k, const float* base, int64_t n
 template <int METRIC, int BQ, int KW, bool VEC>
 static mann_status launch_pers_t(int num_sms, const float* data, const SegItem* items, SegQueue* q, unsigned epoch,
                                  long long wait_cycles, int d, int k, int nsplit, uint64_t* partial,
-                                 const int32_t* qrows, cudaStream_t s) {
+                                 cudaStream_t s) {
   constexpr size_t smem = k1_smem_bytes<BQ, KW>();
   auto kern = k1_persistent<METRIC, BQ, KW, VEC>;
   MANN_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per_sm = 0;
   MANN_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, K1_THREADS, smem));
   const int grid = std::max(1, per_sm) * num_sms;  // every CTA resident: the queue needs no co-scheduling
-  kern<<<(unsigned)grid, K1_THREADS, smem, s>>>(data, items, q, epoch, wait_cycles, d, k, nsplit, partial, qrows);
+  kern<<<(unsigned)grid, K1_THREADS, smem, s>>>(data, items, q, epoch, wait_cycles, d, k, nsplit, partial, nullptr);
   MANN_CHECK_LAUNCH();
   return MANN_OK;
 }
 
 mann_status launch_k1_persistent(int num_sms, const float* data, const SegItem* items, SegQueue* q, unsigned epoch,
                                  long long wait_cycles, int d, int metric, int bq, int k, int nsplit,
-                                 uint64_t* partial, cudaStream_t s, const int32_t* qrows) {
+                                 uint64_t* partial, cudaStream_t s) {
   if (k < 1 || k > 64) return fail(MANN_EINVAL_ARG, "batched graphs support 1 <= k <= 64 (k+1 with self)");
   const bool vec = (d % 4) == 0;
 #define PERS_CASE(M, B, KW)                                                                                      \
   return vec ? launch_pers_t<M, B, KW, true>(num_sms, data, items, q, epoch, wait_cycles, d, k, nsplit, partial, \
-                                             qrows, s)                                                          \
+                                             s)                                                                 \
              : launch_pers_t<M, B, KW, false>(num_sms, data, items, q, epoch, wait_cycles, d, k, nsplit, partial, \
-                                              qrows, s)
+                                              s)
   if (metric == MANN_METRIC_EUCLIDEAN) {
     if (k > 32) {
       if (bq == 32) PERS_CASE(MANN_METRIC_EUCLIDEAN, 32, 2);
@@ -1149,6 +1248,26 @@ mann_status launch_k1_persistent(int num_sms, const float* data, const SegItem* 
   }
 #undef PERS_CASE
   return fail(MANN_EINVAL_ARG, "batched graphs: Euclidean or SqEuclidean");
+}
+
+mann_status launch_seg_rows(const float* data, const int32_t* rows, int cnt, const int64_t* offs, int nsets, int nsplit,
+                            int64_t chunk, int d, int metric, uint64_t* partial, cudaStream_t s) {
+  if (cnt <= 0) return MANN_OK;
+  const int64_t grid = (int64_t)cnt * nsplit;
+  if (grid > INT32_MAX) return fail(MANN_EINVAL_ARG, "batched graphs: too many rows to scan");
+  const bool vec = d % 4 == 0 && (reinterpret_cast<uintptr_t>(data) & 15) == 0;
+#define SEG_ROWS(M)                                                                                                 \
+  (vec ? seg_rows_kernel<M, true> : seg_rows_kernel<M, false>)<<<(unsigned)grid, SR_T, 0, s>>>(data, rows, offs, nsets, \
+                                                                                      nsplit, chunk, d, partial)
+  if (metric == MANN_METRIC_EUCLIDEAN)
+    SEG_ROWS(MANN_METRIC_EUCLIDEAN);
+  else if (metric == MANN_METRIC_SQEUCLIDEAN)
+    SEG_ROWS(MANN_METRIC_SQEUCLIDEAN);
+  else
+    return fail(MANN_EINVAL_ARG, "batched graphs: Euclidean or SqEuclidean");
+#undef SEG_ROWS
+  MANN_CHECK_LAUNCH();
+  return MANN_OK;
 }
 
 mann_status launch_merge_lists(const uint64_t* partial, int64_t nq, int nsplit, int k, uint64_t* out,
