@@ -113,7 +113,7 @@ mann_status search_device_body(Context* ctx, cudaStream_t s, const mann_knn_para
   } else {
     MANN_TRY(knn_fp32_finished(ctx, s, base, n, qs, nq, d, p->metric, kreq, qn, bn, kout, graph_self, ids, dists));
   }
-  if (keys) MANN_TRY(launch_finish(keys, nq, kreq, kout, graph_self, nullptr, ids, dists, s));
+  if (keys) MANN_TRY(launch_finish(keys, nq, kreq, kout, graph_self, ids, dists, s));
   if (rep && (p->flags & MANN_FLAG_FP64_ERR))
     MANN_TRY(fp64_max_error(ctx, s, base, qs, d, p->metric, nq, kout, ids, dists, &rep->max_abs_err_fp64));
   return MANN_OK;

@@ -28,22 +28,6 @@
 namespace mann {
 namespace {
 
-__global__ void localize_ids_kernel(int32_t* __restrict__ ids, int64_t nrows, int k,
-                                    const int64_t* __restrict__ offs, int nsets) {
-  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= nrows) return;
-  int lo = 0, hi = nsets - 1;
-  while (lo < hi) {  // last set whose offset <= r
-    const int mid = (lo + hi + 1) >> 1;
-    if (offs[mid] <= r) lo = mid;
-    else hi = mid - 1;
-  }
-  const int32_t base = (int32_t)offs[lo];
-  int32_t* row = ids + r * k;
-  for (int j = 0; j < k; ++j)
-    if (row[j] >= 0) row[j] -= base;
-}
-
 __global__ void publish_queue_kernel(SegQueue* q, int count, const int* count_dev, unsigned epoch) {
   q->head = 0;
   q->count = count_dev ? *count_dev : count;
@@ -126,9 +110,7 @@ mann_status issue(int num_sms, const Shape& sh, const Plan& pl, const Bufs& b, u
   MANN_TRY(launch_k1_persistent(num_sms, sh.data, b.items, b.queue, epoch, wait_cycles, sh.d, sh.metric, pl.bq,
                                 sh.kk, pl.S, pl.S > 1 ? b.partial : b.keys, s));
   if (pl.S > 1) MANN_TRY(launch_merge_lists(b.partial, sh.N, pl.S, sh.kk, b.keys, s));
-  MANN_TRY(launch_finish(b.keys, sh.N, sh.kk, sh.k, sh.include_self ? -1 : 0, nullptr, sh.ids, sh.dists, s));
-  localize_ids_kernel<<<(unsigned)ceil_div(sh.N, 256), 256, 0, s>>>(sh.ids, sh.N, sh.k, b.offs, sh.nsets);
-  MANN_CHECK_LAUNCH();
+  MANN_TRY(launch_finish(b.keys, sh.N, sh.kk, sh.k, sh.include_self ? -1 : 0, sh.ids, sh.dists, s, b.offs, sh.nsets));
   return MANN_OK;
 }
 
@@ -222,7 +204,7 @@ mann_status run_graph(Context* ctx, cudaStream_t s, const Shape& sh, const Plan&
   }
   it->second.last_use = ++st.clock;
   MANN_CUDA_TRY(cudaGraphLaunch(it->second.exec, s));
-  for (int i = 0; i < (pl.S > 1 ? 5 : 4); ++i) note_launch();  // kernels in the graph
+  for (int i = 0; i < (pl.S > 1 ? 4 : 3); ++i) note_launch();  // kernels in the graph
   return MANN_OK;
 }
 
@@ -263,9 +245,7 @@ mann_status knn_graph_batched_device(Context* ctx, cudaStream_t s, const mann_kn
     MANN_TRY(knn_bf16_batched_keys(ctx, s, data, offs, offs_dev, nsets, d, p->metric, sh.kk, p->margin, &keys, rep,
                                    p->precision == MANN_PREC_FP16 ? FORM_FP16 : FORM_BF16));
     ctx->time_end(s);
-    MANN_TRY(launch_finish(keys, sh.N, sh.kk, k, include_self ? -1 : 0, nullptr, ids, dists, s));
-    localize_ids_kernel<<<(unsigned)ceil_div(sh.N, 256), 256, 0, s>>>(ids, sh.N, k, offs_dev, nsets);
-    MANN_CHECK_LAUNCH();
+    MANN_TRY(launch_finish(keys, sh.N, sh.kk, k, include_self ? -1 : 0, ids, dists, s, offs_dev, nsets));
     BatchState& st = state_of(ctx);
     std::lock_guard<std::mutex> lk(st.mu);
     st.uploaded_items = nullptr;  // the offsets buffer was rewritten: the FP32 plan re-uploads

@@ -505,7 +505,7 @@ mann_status ivf_scan_device(Context* ctx, cudaStream_t s, const float* data, int
                                                     pair_r, choff, chunk_list, nlist, k, nprobe, partial));
   ctx->time_end(s);
   MANN_TRY(launch_merge_lists(partial, nq, nprobe, k, keys, s));
-  MANN_TRY(launch_finish(keys, nq, k, k, -1, nullptr, out_ids, out_dists, s));
+  MANN_TRY(launch_finish(keys, nq, k, k, -1, out_ids, out_dists, s));
   return MANN_OK;
 }
 

@@ -25,13 +25,13 @@ mann_status knn_fp32_finished(Context* ctx, cudaStream_t s, const float* base, i
                               int d, int metric, int kk, const float* qn, const float* bn, int kout,
                               int64_t graph_self, int32_t* ids, float* dists);
 
-// Keys [nq][kk] -> ids/dists [*][kout].  Key row i goes to output row
-// rows[i] (identity when rows is NULL).  With graph_self >= 0 the query of
-// output row r is point (graph_self + r) and is dropped wherever it appears
+// Keys [nq][kk] -> ids/dists [*][kout].  With graph_self >= 0 the query of
+// row r is point (graph_self + r) and is dropped wherever it appears
 // (_prepare_neighbors, src/graphs/knn_graph.jl:105-130); entries without a key
-// become id -1 / +inf.
+// become id -1 / +inf.  With offs, ids count from the first row of the set of
+// offs[0 .. nsets] that holds row r.
 mann_status launch_finish(const uint64_t* keys, int64_t nq, int kk, int kout, int64_t graph_self,
-                          const int32_t* rows, int32_t* ids, float* dists, cudaStream_t s);
+                          int32_t* ids, float* dists, cudaStream_t s, const int64_t* offs = nullptr, int nsets = 0);
 
 // Operand forms of the tensor-core search: BF16 rows (the three-product split
 // when BF16 cannot hold the data), E4M3 rows with per-row power-of-two scales

@@ -124,6 +124,6 @@ extern "C" mann_status mann_knn_device_noalloc(const mann_knn_params* p, const f
   uint64_t* keys = nullptr;
   MANN_TRY(knn_fp32_keys_on(nd->num_sms, s, base, n, queries, q, d, p->metric, kreq, qn, bn,
                             nd->scratch + norm_words, NOALLOC_WORDS - norm_words, &keys));
-  MANN_TRY(launch_finish(keys, q, kreq, kout, -1, nullptr, out_ids, out_dists, s));
+  MANN_TRY(launch_finish(keys, q, kreq, kout, -1, out_ids, out_dists, s));
   return MANN_OK;
 }
