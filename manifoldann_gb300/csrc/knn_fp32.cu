@@ -732,24 +732,52 @@ __device__ __forceinline__ void finish_row32(const FewOut& o, int64_t q, uint64_
   }
 }
 
+// four more terms of a sum, in dimension order
+template <int METRIC>
+__device__ __forceinline__ void few_add(float& a, const float4& q4, const float4& v) {
+  if constexpr (METRIC == MANN_METRIC_COSINE) {
+    a = __fmaf_rn(q4.x, v.x, a);
+    a = __fmaf_rn(q4.y, v.y, a);
+    a = __fmaf_rn(q4.z, v.z, a);
+    a = __fmaf_rn(q4.w, v.w, a);
+  } else {
+    float u = __fsub_rn(q4.x, v.x);
+    a = __fmaf_rn(u, u, a);
+    u = __fsub_rn(q4.y, v.y);
+    a = __fmaf_rn(u, u, a);
+    u = __fsub_rn(q4.z, v.z);
+    a = __fmaf_rn(u, u, a);
+    u = __fsub_rn(q4.w, v.w);
+    a = __fmaf_rn(u, u, a);
+  }
+}
+
 // few_rows_kernel for nq <= FEW_QS rows of d <= FEW_STAGED_D: the rows sit in
-// shared memory ([FEW_QS][d], staged once), and each thread reads its point
-// with eight float4 loads in flight and no barrier per chunk (the chunked
-// form waits for its loads 25 times per point at d = 784); the same
-// sequential sums in dimension order.  Every warp keeps its own list of every
-// row -- 32 new distances are sorted and merged at once when many of them
-// count, so no warp waits for another's insertions -- and a block merges its
-// warps' lists at the end.
+// shared memory ([FEW_QS][d], staged once), and no barrier falls between a
+// point's columns (the chunked form waits for its loads 25 times per point at
+// d = 784); the same sequential sums in dimension order.  Every warp keeps its
+// own list of every row -- 32 new distances are sorted and merged at once when
+// many of them count, so no warp waits for another's insertions -- and a block
+// merges its warps' lists at the end.
 //
 // With a ticket (lists of at most 32) the last block to finish merges all the
 // blocks' lists and writes the results: a single query is one launch instead
 // of three (1 x 10,000 x 64: 22 us of kernels with two gaps, now 11).
+//
+// VEC (d a multiple of 4, 16-byte rows): the points come in through shared
+// memory, 32 columns of a warp's 32 rows at a time with eight lanes to a row and
+// the next slice in flight.  A thread that reads its own row touches 32 lines
+// per load, and the line lookups bound it: one row against 290,000 x 256 points
+// (297 MB, 44 us at the copy rate) took 98 us, now 78 from a cold cache; four
+// rows 145, now 109; 60,000 x 784 70, now 61; 10,000 x 64 14.3, now 12.3.
+constexpr int FEW_SD = 32, FEW_SS = FEW_SD + 4;  // columns of a slice, their stride
+constexpr size_t FEW_SLICE_BYTES = sizeof(float) * 2 * (FEW_T / 32) * 32 * FEW_SS;
 template <int METRIC, int KW, bool VEC>
 __global__ void __launch_bounds__(FEW_T, 2)
     few_rows_staged_kernel(const float* __restrict__ base, int64_t n, const float* __restrict__ qs,
                            const int32_t* __restrict__ qrows, int nq, int d, const float* __restrict__ qnorm,
                            const float* __restrict__ bnorm, int k, uint64_t* __restrict__ partial,
-                           unsigned* __restrict__ ticket, FewOut out) {
+                           unsigned* __restrict__ ticket, FewOut out, int slice_at) {
   extern __shared__ __align__(16) float fq[];  // [nq][d], then the warps' lists
   uint64_t(*wl)[FEW_QS][32 * KW] = reinterpret_cast<uint64_t(*)[FEW_QS][32 * KW]>(fq);
   __shared__ int last;
@@ -773,49 +801,52 @@ __global__ void __launch_bounds__(FEW_T, 2)
     float acc[FEW_QS];
 #pragma unroll
     for (int j = 0; j < FEW_QS; ++j) acc[j] = 0.0f;
-    if (valid) {
-      if (VEC) {  // d % 4 == 0 and 16-byte aligned rows
-#pragma unroll 8
-        for (int c = 0; c < d; c += 4) {
-          const float4 v = __ldg(reinterpret_cast<const float4*>(prow + c));
+    if constexpr (VEC) {
+      const int64_t w0 = p0 + warp * 32;  // the warp's first point
+      float* slices = fq + slice_at + warp * 2 * 32 * FEW_SS;
+      auto fetch = [&](int c0) {
+        const int c = (lane & 7) * 4;
+        float* dst = slices + (c0 / FEW_SD & 1) * 32 * FEW_SS;
 #pragma unroll
-          for (int j = 0; j < FEW_QS; ++j) {
-            if (j < nq) {
-              const float4 q4 = *reinterpret_cast<const float4*>(&fq[j * d + c]);
-              float a = acc[j];
-              if constexpr (METRIC == MANN_METRIC_COSINE) {
-                a = __fmaf_rn(q4.x, v.x, a);
-                a = __fmaf_rn(q4.y, v.y, a);
-                a = __fmaf_rn(q4.z, v.z, a);
-                a = __fmaf_rn(q4.w, v.w, a);
-              } else {
-                float u = __fsub_rn(q4.x, v.x);
-                a = __fmaf_rn(u, u, a);
-                u = __fsub_rn(q4.y, v.y);
-                a = __fmaf_rn(u, u, a);
-                u = __fsub_rn(q4.z, v.z);
-                a = __fmaf_rn(u, u, a);
-                u = __fsub_rn(q4.w, v.w);
-                a = __fmaf_rn(u, u, a);
-              }
-              acc[j] = a;
-            }
+        for (int it = 0; it < 8; ++it) {
+          const int r = it * 4 + (lane >> 3);
+          if (w0 + r < n && c0 + c < d) {
+            const uint32_t sa = (uint32_t)__cvta_generic_to_shared(dst + r * FEW_SS + c);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sa), "l"(base + (w0 + r) * d + c0 + c)
+                         : "memory");
           }
         }
-      } else {
-#pragma unroll 8
-        for (int c = 0; c < d; ++c) {
-          const float pv = __ldg(prow + c);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+      };
+      fetch(0);
+      for (int c0 = 0; c0 < d; c0 += FEW_SD) {
+        fetch(c0 + FEW_SD);  // nothing past d
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+        const float* x = slices + (c0 / FEW_SD & 1) * 32 * FEW_SS + lane * FEW_SS;
+        const int cw = min(FEW_SD, d - c0);
+#pragma unroll 4
+        for (int c = 0; c < cw; c += 4) {
+          const float4 v = *reinterpret_cast<const float4*>(x + c);
 #pragma unroll
-          for (int j = 0; j < FEW_QS; ++j) {
-            if (j < nq) {
-              const float qv = fq[j * d + c];
-              if constexpr (METRIC == MANN_METRIC_COSINE) {
-                acc[j] = __fmaf_rn(qv, pv, acc[j]);
-              } else {
-                const float u = __fsub_rn(qv, pv);
-                acc[j] = __fmaf_rn(u, u, acc[j]);
-              }
+          for (int j = 0; j < FEW_QS; ++j)
+            if (j < nq) few_add<METRIC>(acc[j], *reinterpret_cast<const float4*>(&fq[j * d + c0 + c]), v);
+        }
+        __syncwarp();
+      }
+    } else if (valid) {
+#pragma unroll 8
+      for (int c = 0; c < d; ++c) {
+        const float pv = __ldg(prow + c);
+#pragma unroll
+        for (int j = 0; j < FEW_QS; ++j) {
+          if (j < nq) {
+            const float qv = fq[j * d + c];
+            if constexpr (METRIC == MANN_METRIC_COSINE) {
+              acc[j] = __fmaf_rn(qv, pv, acc[j]);
+            } else {
+              const float u = __fsub_rn(qv, pv);
+              acc[j] = __fmaf_rn(u, u, acc[j]);
             }
           }
         }
@@ -1010,12 +1041,12 @@ mann_status launch_few_m(int grid, const float* base, int64_t n, const float* qs
                          const FewOut& out, cudaStream_t s) {
   if (nq <= FEW_QS && d <= FEW_STAGED_D) {
     const size_t smem = std::max(sizeof(float) * nq * d, few_list_bytes(kk <= 32 ? 1 : 2));  // <= 32 KB
-    if (kk <= 32)
-      few_rows_staged_kernel<METRIC, 1, VEC><<<grid, FEW_T, smem, s>>>(base, n, qs, rows, nq, d, qn, bn, kk, partial,
-                                                                       ticket, out);
-    else
-      few_rows_staged_kernel<METRIC, 2, VEC><<<grid, FEW_T, smem, s>>>(base, n, qs, rows, nq, d, qn, bn, kk, partial,
-                                                                       nullptr, out);
+    const size_t slices = VEC ? FEW_SLICE_BYTES : 0;
+    const auto kern = kk <= 32 ? few_rows_staged_kernel<METRIC, 1, VEC> : few_rows_staged_kernel<METRIC, 2, VEC>;
+    MANN_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(sizeof(float) * FEW_QS * FEW_STAGED_D + slices)));
+    kern<<<grid, FEW_T, smem + slices, s>>>(base, n, qs, rows, nq, d, qn, bn, kk, partial,
+                                            kk <= 32 ? ticket : nullptr, out, (int)(smem / sizeof(float)));
   } else if (kk <= 32) {
     few_rows_kernel<METRIC, 1, VEC><<<grid, FEW_T, 0, s>>>(base, n, qs, rows, nq, d, qn, bn, kk, partial);
   } else {
