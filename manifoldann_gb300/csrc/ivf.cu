@@ -26,7 +26,10 @@ namespace mann {
 
 namespace {
 
-constexpr int SCAN_Q = 32;    // queries per CTA (at most)
+// Queries per CTA (at most).  32 at three CTAs per SM, for lists that see more
+// than a dozen queries, were slower at every size: 220 lists of 600 x 64, 59
+// queries each 649 us against 450; 195 of 370 x 96, 412 each 2.14 ms and 1.76.
+constexpr int SCAN_Q = 16;
 constexpr int SCAN_T = 128;   // threads
 constexpr int SCAN_P = 256;   // points per pass: two per thread
 constexpr int SCAN_DC = 16;   // dimensions per staged slice of a point row
@@ -185,9 +188,9 @@ __device__ __forceinline__ void pass_topk32(const float* __restrict__ dist, int 
 }
 
 // Shared memory of a scan CTA: the staged queries, then a slice of every row, over which the pass's distances are laid when the arithmetic is done.
-template <int QC>
 struct ScanSmem {
-  static constexpr int SDQ = QC == 16 ? 128 : 64;  // query dimensions per stage
+  static constexpr int QC = SCAN_Q;
+  static constexpr int SDQ = 128;                  // query dimensions per stage
   static constexpr int QS = QC + 4;                // stride (floats), a multiple of 4
   static constexpr int XS = SCAN_DC + 4;           // stride of a staged row slice
   static constexpr int DS = SCAN_P + 1;            // stride of a query's distances
@@ -197,7 +200,7 @@ struct ScanSmem {
   static constexpr size_t BYTES = sizeof(float) * (QUERIES + (ROWS > DISTS ? ROWS : DISTS));
 };
 
-// One CTA: list l and up to QC (16 or 32) of its queries.  Each thread takes
+// One CTA: up to SCAN_Q of list l's queries and a part of the list (blockIdx.y).  Each thread takes
 // two points of the list per pass (read in place through the list's ids) and
 // computes their distances to every query of the CTA, each distance the
 // sequential difference-form sum over dimensions 0..d-1 of the FP32 form.
@@ -209,8 +212,8 @@ struct ScanSmem {
 // arithmetic, and six CTAs per SM cover each other's loads.  What bounds it is shared-memory reads of the
 // queries, one 16-byte broadcast per four queries and dimension: two points
 // per thread halve them.
-template <int METRIC, int KW, bool VEC, int QC>
-__global__ void __launch_bounds__(SCAN_T, QC == 16 ? 6 : 3)
+template <int METRIC, int KW, bool VEC>
+__global__ void __launch_bounds__(SCAN_T, 6)
     ivf_scan_kernel(const float* __restrict__ data, const int64_t* __restrict__ loff,
                     const int32_t* __restrict__ lids, const float* __restrict__ qs, int d,
                     const int64_t* __restrict__ qoff, const int32_t* __restrict__ pair_q,
@@ -219,8 +222,8 @@ __global__ void __launch_bounds__(SCAN_T, QC == 16 ? 6 : 3)
                     int k, int nprobe, uint64_t* __restrict__ partial) {
   // queries staged transposed, [dimension][query] with a padded stride, so one
   // 16-byte broadcast read gives four queries' value at one dimension
-  using S = ScanSmem<QC>;
-  constexpr int SDQ = S::SDQ, QS = S::QS, XS = S::XS;
+  using S = ScanSmem;
+  constexpr int QC = SCAN_Q, SDQ = S::SDQ, QS = S::QS, XS = S::XS;
   constexpr int NW = SCAN_T / 32;
   extern __shared__ __align__(16) float scan_smem[];
   float* qsm = scan_smem;
@@ -234,7 +237,10 @@ __global__ void __launch_bounds__(SCAN_T, QC == 16 ? 6 : 3)
   const int l = chunk_list[w];
   const int64_t e0 = qoff[l] + (w - choff[l]) * QC;
   const int nqe = (int)min((int64_t)QC, qoff[l + 1] - e0);
-  const int64_t p_begin = loff[l], p_end = loff[l + 1];
+  const int64_t l_end = loff[l + 1];
+  const int64_t part = ((l_end - loff[l] + gridDim.y - 1) / gridDim.y + SCAN_P - 1) / SCAN_P * SCAN_P;
+  const int64_t p_begin = min(l_end, loff[l] + blockIdx.y * part), p_end = min(l_end, p_begin + part);
+  if (blockIdx.y > 0 && p_begin == p_end) return;  // its lists are empty already
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   if (t < nqe) s_q[t] = pair_q[e0 + t];
 
@@ -404,7 +410,7 @@ __global__ void __launch_bounds__(SCAN_T, QC == 16 ? 6 : 3)
   for (int m = 0; m < MW; ++m) {
     const int j = warp + NW * m;
     if (j >= nqe) continue;
-    uint64_t* dst = partial + ((int64_t)s_q[j] * nprobe + pair_r[e0 + j]) * k;
+    uint64_t* dst = partial + (((int64_t)s_q[j] * nprobe + pair_r[e0 + j]) * gridDim.y + blockIdx.y) * k;
 #pragma unroll
     for (int s = 0; s < KW; ++s) {
       const int e = s * 32 + lane;
@@ -413,45 +419,33 @@ __global__ void __launch_bounds__(SCAN_T, QC == 16 ? 6 : 3)
   }
 }
 
-template <int METRIC, int KW, bool VEC, int QC>
-mann_status launch_scan_q(cudaStream_t s, int64_t grid, const float* data, const int64_t* loff, const int32_t* lids,
+template <int METRIC, int KW, bool VEC>
+mann_status launch_scan_t(cudaStream_t s, dim3 grid, const float* data, const int64_t* loff, const int32_t* lids,
                           const float* qs, int d, const int64_t* qoff, const int32_t* pair_q, const int32_t* pair_r,
                           const int64_t* choff, const int32_t* chunk_list, int nlist, int k, int nprobe,
                           uint64_t* partial) {
-  auto kern = ivf_scan_kernel<METRIC, KW, VEC, QC>;
-  constexpr size_t smem = ScanSmem<QC>::BYTES;
+  auto kern = ivf_scan_kernel<METRIC, KW, VEC>;
+  constexpr size_t smem = ScanSmem::BYTES;
   MANN_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<(unsigned)grid, SCAN_T, smem, s>>>(data, loff, lids, qs, d, qoff, pair_q, pair_r, choff, chunk_list, nlist, k,
-                                            nprobe, partial);
+  kern<<<grid, SCAN_T, smem, s>>>(data, loff, lids, qs, d, qoff, pair_q, pair_r, choff, chunk_list, nlist, k, nprobe,
+                                  partial);
   MANN_CHECK_LAUNCH();
   return MANN_OK;
 }
 
-template <int METRIC, int KW, bool VEC>
-mann_status launch_scan_t(cudaStream_t s, int qc, int64_t grid, const float* data, const int64_t* loff,
-                          const int32_t* lids, const float* qs, int d, const int64_t* qoff,
-                          const int32_t* pair_q, const int32_t* pair_r, const int64_t* choff,
-                          const int32_t* chunk_list, int nlist, int k, int nprobe, uint64_t* partial) {
-  if (qc == 16)
-    return launch_scan_q<METRIC, KW, VEC, 16>(s, grid, data, loff, lids, qs, d, qoff, pair_q, pair_r, choff, chunk_list,
-                                              nlist, k, nprobe, partial);
-  return launch_scan_q<METRIC, KW, VEC, 32>(s, grid, data, loff, lids, qs, d, qoff, pair_q, pair_r, choff, chunk_list,
-                                            nlist, k, nprobe, partial);
-}
-
 template <int METRIC>
-mann_status launch_scan_m(cudaStream_t s, int qc, int64_t grid, bool vec, const float* data, const int64_t* loff,
+mann_status launch_scan_m(cudaStream_t s, dim3 grid, bool vec, const float* data, const int64_t* loff,
                           const int32_t* lids, const float* qs, int d, const int64_t* qoff,
                           const int32_t* pair_q, const int32_t* pair_r, const int64_t* choff,
                           const int32_t* chunk_list, int nlist, int k, int nprobe, uint64_t* partial) {
   if (k <= 32)
-    return vec ? launch_scan_t<METRIC, 1, true>(s, qc, grid, data, loff, lids, qs, d, qoff, pair_q, pair_r, choff,
+    return vec ? launch_scan_t<METRIC, 1, true>(s, grid, data, loff, lids, qs, d, qoff, pair_q, pair_r, choff,
                                                 chunk_list, nlist, k, nprobe, partial)
-               : launch_scan_t<METRIC, 1, false>(s, qc, grid, data, loff, lids, qs, d, qoff, pair_q, pair_r, choff,
+               : launch_scan_t<METRIC, 1, false>(s, grid, data, loff, lids, qs, d, qoff, pair_q, pair_r, choff,
                                                  chunk_list, nlist, k, nprobe, partial);
-  return vec ? launch_scan_t<METRIC, 2, true>(s, qc, grid, data, loff, lids, qs, d, qoff, pair_q, pair_r, choff,
+  return vec ? launch_scan_t<METRIC, 2, true>(s, grid, data, loff, lids, qs, d, qoff, pair_q, pair_r, choff,
                                               chunk_list, nlist, k, nprobe, partial)
-             : launch_scan_t<METRIC, 2, false>(s, qc, grid, data, loff, lids, qs, d, qoff, pair_q, pair_r, choff,
+             : launch_scan_t<METRIC, 2, false>(s, grid, data, loff, lids, qs, d, qoff, pair_q, pair_r, choff,
                                                chunk_list, nlist, k, nprobe, partial);
 }
 
@@ -476,35 +470,42 @@ mann_status ivf_scan_device(Context* ctx, cudaStream_t s, const float* data, int
   MANN_TRY(ctx->scratch_t(SLOT_IVF_CNT, (size_t)2 * nlist + 4, &cnt));
   MANN_TRY(ctx->scratch_t(SLOT_IVF_OFF, (size_t)2 * (nlist + 1), &qoff));
   choff = qoff + (nlist + 1);
-  // 16-query chunks when lists see few queries (more, lighter CTAs), else 32
-  const int qc = nq * nprobe <= (int64_t)12 * nlist ? 16 : SCAN_Q;
-  // chunks <= pairs/qc + lists; blocks past the real count return at once
-  const int64_t max_chunks = ceil_div(nq * nprobe, qc) + nlist;
+  // chunks <= pairs / SCAN_Q + lists; blocks past the real count return at once
+  const int64_t pairs = nq * nprobe;
+  const int64_t max_chunks = ceil_div(pairs, SCAN_Q) + nlist;
+  // Lists are cut into parts while the chunks fill the chip's six CTAs per SM
+  // less than twice over: one CTA walks a long list alone (300 queries, 9 of 228
+  // lists of 476 x 128, uneven: 544 us whole, 250 in parts; 4,356 queries, 3 of
+  // 220 lists of 598 x 64: 450 and 363).
+  const int64_t chunks = ceil_div(pairs, SCAN_Q) + std::min<int64_t>(pairs, nlist);
+  const int parts = (int)std::max<int64_t>(
+      1, std::min<int64_t>({8, 128 / nprobe, ceil_div((int64_t)12 * ctx->num_sms, std::max<int64_t>(chunks, 1))}));
   int32_t* chunk_list = nullptr;
   MANN_TRY(ctx->scratch_t(SLOT_IVF_PAIRS, (size_t)2 * nq * nprobe + (size_t)max_chunks, &pair_q));
   pair_r = pair_q + nq * nprobe;
   chunk_list = pair_r + nq * nprobe;
-  MANN_TRY(ctx->scratch_t(SLOT_IVF_PARTIAL, (size_t)nq * nprobe * k, &partial));
+  MANN_TRY(ctx->scratch_t(SLOT_IVF_PARTIAL, (size_t)nq * nprobe * parts * k, &partial));
   MANN_TRY(ctx->scratch_t(SLOT_IVF_KEYS, (size_t)nq * k, &keys));
   MANN_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(unsigned) * (2 * nlist + 4), s));
-  MANN_CUDA_TRY(cudaMemsetAsync(partial, 0xFF, sizeof(uint64_t) * nq * nprobe * k, s));
+  MANN_CUDA_TRY(cudaMemsetAsync(partial, 0xFF, sizeof(uint64_t) * nq * nprobe * parts * k, s));
   probe_count_kernel<<<(unsigned)ceil_div(nq * nprobe, 256), 256, 0, s>>>(probes, nq * nprobe, nlist, cnt);
   MANN_CHECK_LAUNCH();
-  probe_scan_kernel<<<1, 1024, 0, s>>>(cnt, nlist, qc, qoff, choff);
+  probe_scan_kernel<<<1, 1024, 0, s>>>(cnt, nlist, SCAN_Q, qoff, choff);
   MANN_CHECK_LAUNCH();
   probe_scatter_kernel<<<(unsigned)ceil_div(nq * nprobe, 256), 256, 0, s>>>(
       probes, nq, nprobe, nlist, qoff, choff, cnt + nlist, pair_q, pair_r, chunk_list);
   MANN_CHECK_LAUNCH();
   const bool vec = (d % 4) == 0 && (reinterpret_cast<uintptr_t>(data) & 15) == 0;
+  const dim3 grid((unsigned)max_chunks, (unsigned)parts);
   ctx->time_begin(s);
   if (metric == MANN_METRIC_EUCLIDEAN)
-    MANN_TRY(launch_scan_m<MANN_METRIC_EUCLIDEAN>(s, qc, max_chunks, vec, data, loff, lids, qs, d, qoff, pair_q, pair_r,
+    MANN_TRY(launch_scan_m<MANN_METRIC_EUCLIDEAN>(s, grid, vec, data, loff, lids, qs, d, qoff, pair_q, pair_r,
                                                   choff, chunk_list, nlist, k, nprobe, partial));
   else
-    MANN_TRY(launch_scan_m<MANN_METRIC_SQEUCLIDEAN>(s, qc, max_chunks, vec, data, loff, lids, qs, d, qoff, pair_q,
+    MANN_TRY(launch_scan_m<MANN_METRIC_SQEUCLIDEAN>(s, grid, vec, data, loff, lids, qs, d, qoff, pair_q,
                                                     pair_r, choff, chunk_list, nlist, k, nprobe, partial));
   ctx->time_end(s);
-  MANN_TRY(launch_merge_lists(partial, nq, nprobe, k, keys, s));
+  MANN_TRY(launch_merge_lists(partial, nq, nprobe * parts, k, keys, s));
   MANN_TRY(launch_finish(keys, nq, k, k, -1, out_ids, out_dists, s));
   return MANN_OK;
 }
