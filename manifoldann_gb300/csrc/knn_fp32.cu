@@ -1283,7 +1283,7 @@ mann_status launch_k1_persistent(int num_sms, const float* data, const SegItem* 
                                  long long wait_cycles, int d, int metric, int bq, int k, int nsplit,
                                  uint64_t* partial, cudaStream_t s) {
   if (k < 1 || k > 64) return fail(MANN_EINVAL_ARG, "batched graphs support 1 <= k <= 64 (k+1 with self)");
-  const bool vec = (d % 4) == 0;
+  const bool vec = d % 4 == 0 && (reinterpret_cast<uintptr_t>(data) & 15) == 0;
 #define PERS_CASE(M, B, KW)                                                                                      \
   return vec ? launch_pers_t<M, B, KW, true>(num_sms, data, items, q, epoch, wait_cycles, d, k, nsplit, partial, \
                                              s)                                                                 \
