@@ -126,7 +126,10 @@ struct BatchState {
   std::map<std::string, std::pair<int, int>> tuned;  // signature -> (bq, S)
   uint64_t clock = 0;
   cudaStream_t cap = nullptr;
-  const void* uploaded_items = nullptr;  // device buffer holding the plan with hash uploaded_hash
+  // device buffers holding the items and offsets of the plan with hash
+  // uploaded_hash; dropped (items null) before anything that may replace them
+  const void* uploaded_items = nullptr;
+  const void* uploaded_offs = nullptr;
   uint64_t uploaded_hash = 0;
   unsigned epoch = 0;  // last epoch handed to a queue
 };
@@ -144,18 +147,23 @@ constexpr size_t MAX_GRAPHS = 16;
 
 mann_status prepare(Context* ctx, cudaStream_t s, const Shape& sh, const int64_t* offs_host, const Plan& pl,
                     Bufs* b, BatchState& st) {
+  // another plan's buffers may be freed below, and others come to lie at their
+  // addresses, before a request that fails
+  if (st.uploaded_hash != pl.hash) st.uploaded_items = nullptr;
   MANN_TRY(ctx->scratch_t(SLOT_BATCH_ITEMS, std::max<size_t>(pl.items.size(), 1), &b->items));
   MANN_TRY(ctx->scratch_t(SLOT_BATCH_OFFS, (size_t)sh.nsets + 1, &b->offs));
   MANN_TRY(ctx->scratch_t(SLOT_KEYS, (size_t)sh.N * sh.kk, &b->keys));
   MANN_TRY(ctx->scratch_t(SLOT_BATCH_QUEUE, 1, &b->queue));
   if (pl.S > 1) MANN_TRY(ctx->scratch_t(SLOT_PARTIAL, (size_t)sh.N * pl.S * sh.kk, &b->partial));
-  if (st.uploaded_items != b->items || st.uploaded_hash != pl.hash) {
+  if (st.uploaded_items != b->items || st.uploaded_offs != b->offs || st.uploaded_hash != pl.hash) {
+    st.uploaded_items = nullptr;
     MANN_CUDA_TRY(cudaMemcpyAsync(b->items, pl.items.data(), sizeof(SegItem) * pl.items.size(),
                                   cudaMemcpyHostToDevice, s));
     MANN_CUDA_TRY(cudaMemcpyAsync(b->offs, offs_host, sizeof(int64_t) * (sh.nsets + 1), cudaMemcpyHostToDevice, s));
     // the copies read pageable host memory: finish them before the plan can change
     MANN_CUDA_TRY(cudaStreamSynchronize(s));
     st.uploaded_items = b->items;
+    st.uploaded_offs = b->offs;
     st.uploaded_hash = pl.hash;
   }
   return MANN_OK;
@@ -237,6 +245,12 @@ mann_status knn_graph_batched_device(Context* ctx, cudaStream_t s, const mann_kn
   Shape sh{data, offs[nsets], nsets, d, p->metric, k, include_self ? k : k + 1, include_self ? 1 : 0, ids, dists};
   if (p->precision == MANN_PREC_BF16 || p->precision == MANN_PREC_FP16) {
     // the tensor-core form: one segmented pass over every set's (block, tile) items
+    {
+      // it writes the offsets buffer, whether or not the call succeeds: the FP32 plan re-uploads
+      BatchState& st = state_of(ctx);
+      std::lock_guard<std::mutex> lk(st.mu);
+      st.uploaded_items = nullptr;
+    }
     int64_t* offs_dev = nullptr;
     MANN_TRY(ctx->scratch_t(SLOT_BATCH_OFFS, (size_t)nsets + 1, &offs_dev));
     MANN_CUDA_TRY(cudaMemcpyAsync(offs_dev, offs, sizeof(int64_t) * (nsets + 1), cudaMemcpyHostToDevice, s));
@@ -245,11 +259,7 @@ mann_status knn_graph_batched_device(Context* ctx, cudaStream_t s, const mann_kn
     MANN_TRY(knn_bf16_batched_keys(ctx, s, data, offs, offs_dev, nsets, d, p->metric, sh.kk, p->margin, &keys, rep,
                                    p->precision == MANN_PREC_FP16 ? FORM_FP16 : FORM_BF16));
     ctx->time_end(s);
-    MANN_TRY(launch_finish(keys, sh.N, sh.kk, k, include_self ? -1 : 0, ids, dists, s, offs_dev, nsets));
-    BatchState& st = state_of(ctx);
-    std::lock_guard<std::mutex> lk(st.mu);
-    st.uploaded_items = nullptr;  // the offsets buffer was rewritten: the FP32 plan re-uploads
-    return MANN_OK;
+    return launch_finish(keys, sh.N, sh.kk, k, include_self ? -1 : 0, ids, dists, s, offs_dev, nsets);
   }
   if (sh.kk > 64) return fail(MANN_EINVAL_ARG, "batched graphs support k <= 63 (64 with include_self)");
   BatchState& st = state_of(ctx);

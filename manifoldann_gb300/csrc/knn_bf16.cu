@@ -3703,6 +3703,9 @@ mann_status knn_bf16_batched_keys(Context* ctx, cudaStream_t s, const float* dat
   const int64_t N = offs_host[nsets];
   SegTables& T = seg_tables(ctx);
   build_seg_tables(offs_host, nsets, ctx->num_sms, &T);
+  // other tables' buffers may be freed below, and others come to lie at their
+  // addresses, before a request that fails
+  if (T.uploaded_hash != T.hash) T.uploaded = nullptr;
   TileItem* d_items = nullptr;
   RunInfo* d_runs = nullptr;
   int32_t* d_row_run = nullptr;
@@ -3719,6 +3722,7 @@ mann_status knn_bf16_batched_keys(Context* ctx, cudaStream_t s, const float* dat
   MANN_TRY(ctx->scratch_t(SLOT_SEG_SRUNS, T.sruns.size(), &d_sruns));
   MANN_TRY(ctx->scratch_t(SLOT_SEG_SROWRUN, (size_t)N, &d_srow_run));
   if (T.uploaded != d_items || T.suploaded != d_sitems || T.uploaded_hash != T.hash) {
+    T.uploaded = nullptr;
     MANN_CUDA_TRY(cudaMemcpyAsync(d_items, T.items.data(), sizeof(TileItem) * T.items.size(), cudaMemcpyHostToDevice, s));
     MANN_CUDA_TRY(cudaMemcpyAsync(d_runs, T.runs.data(), sizeof(RunInfo) * T.runs.size(), cudaMemcpyHostToDevice, s));
     MANN_CUDA_TRY(cudaMemcpyAsync(d_cuts, T.cuts.data(), sizeof(int64_t) * T.cuts.size(), cudaMemcpyHostToDevice, s));
