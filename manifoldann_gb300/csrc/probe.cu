@@ -257,13 +257,9 @@ mann_status map_kmajor(CUtensorMap* m, const bf16* ptr, int64_t rows, int64_t co
 
 template <int EPI, int GN>
 mann_status launch_gemm_t(cudaStream_t s, const bf16* A, const bf16* B, const GemmArgs& g) {
-  static std::once_flag once;
-  static cudaError_t attr = cudaSuccess;
   constexpr size_t smem = GTile<GN>::SMEM;
-  std::call_once(once, [] {
-    attr = cudaFuncSetAttribute(probe_gemm<EPI, GN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  });
-  MANN_CUDA_TRY(attr);
+  // (belongs to the current device: set with every launch)
+  MANN_CUDA_TRY(cudaFuncSetAttribute(probe_gemm<EPI, GN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   CUtensorMap ma, mb;
   MANN_TRY(map_kmajor(&ma, A, g.M, g.K, GM));
   MANN_TRY(map_kmajor(&mb, B, g.N, g.K, GN));
@@ -1101,13 +1097,8 @@ mann_status fwd_bwd(ProbeModel* m, cudaStream_t s, Batch& b, int nb, bool grad, 
   if (!grad) return MANN_OK;
   SoftmaxArgs sa{b.logits, prior ? b.D : nullptr, w + P.theta, b.lb, b.L, nb, P.nout, P.noutp, Bp,
                  b.lse, b.loss_row, b.dL, b.dLt, prior ? b.theta_part : nullptr};
-  static std::once_flag once;
-  static cudaError_t attr = cudaSuccess;
-  std::call_once(once, [] {
-    attr = cudaFuncSetAttribute(softmax_stats_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(sizeof(float) * ROUTE_MAXCOLS));  // nout <= ROUTE_MAXCOLS
-  });
-  MANN_CUDA_TRY(attr);
+  MANN_CUDA_TRY(cudaFuncSetAttribute(softmax_stats_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)(sizeof(float) * ROUTE_MAXCOLS)));  // nout <= ROUTE_MAXCOLS
   softmax_stats_kernel<<<(unsigned)Bp, SS_THREADS, sizeof(float) * P.nout, s>>>(sa);
   MANN_CHECK_LAUNCH();
   softmax_grad_kernel<<<dim3((unsigned)ceil_div(P.noutp, 32 * SG_TILES), Bp / 32), 256, 0, s>>>(sa);
