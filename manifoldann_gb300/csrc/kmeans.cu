@@ -975,10 +975,12 @@ mann_status kmeanspp_device(Context* ctx, cudaStream_t s, const float* X, int64_
     if (a.prune && a.i > 1) {
       cfg.gridDim = dim3((unsigned)ceil_div(a.i - 1, PP_T / 32));
       MANN_CUDA_TRY(cudaLaunchKernelEx(&cfg, pp_reach_kernel, a));
+      MANN_CHECK_LAUNCH();
     }
     cfg.gridDim = dim3((unsigned)ceil_div(n, PP_CHUNK / parts));
     cfg.dynamicSmemBytes = smem;
     MANN_CUDA_TRY(cudaLaunchKernelEx(&cfg, step, a));
+    MANN_CHECK_LAUNCH();
   }
   return MANN_OK;
 }
