@@ -505,7 +505,8 @@ mann_status ivf_scan_device(Context* ctx, cudaStream_t s, const float* data, int
     MANN_TRY(launch_scan_m<MANN_METRIC_SQEUCLIDEAN>(s, grid, vec, data, loff, lids, qs, d, qoff, pair_q,
                                                     pair_r, choff, chunk_list, nlist, k, nprobe, partial));
   ctx->time_end(s);
-  MANN_TRY(launch_merge_lists(partial, nq, nprobe * parts, k, keys, s));
+  // (lists may have points in common: a point found in two of them is one result)
+  MANN_TRY(launch_merge_lists(partial, nq, nprobe * parts, k, keys, s, true));
   MANN_TRY(launch_finish(keys, nq, k, k, -1, out_ids, out_dists, s));
   return MANN_OK;
 }

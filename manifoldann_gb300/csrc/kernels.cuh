@@ -100,7 +100,6 @@ mann_status exact_search_device(Context* ctx, cudaStream_t s, const mann_knn_par
                                 int64_t graph_self, int kreq, int kout, int32_t* ids, float* dists,
                                 mann_knn_report* rep, int tie_entries = TIE_ENTRIES);
 
-// Merge nsplit sorted key lists of k per query (nsplit <= 128) into one.
 // Work item of the segmented FP32 tile kernel (batched point sets).
 struct SegItem {
   int64_t q0, qend, nb0, nb1;
@@ -134,8 +133,10 @@ mann_status knn_graph_batched_device(Context* ctx, cudaStream_t s, const mann_kn
                                      float* dists, mann_knn_report* rep);
 mann_status fp64_max_error(Context* ctx, cudaStream_t s, const float* base, const float* qs, int d, int metric,
                            int64_t nq, int kout, const int32_t* ids, const float* dists, double* out);
+// Sorted lists partial [nq][nsplit][k] (nsplit <= 128) -> the k smallest keys of every row; with
+// `shared` a key that several of a row's lists hold counts once.
 mann_status launch_merge_lists(const uint64_t* partial, int64_t nq, int nsplit, int k, uint64_t* out,
-                               cudaStream_t s);
+                               cudaStream_t s, bool shared = false);
 
 // KMeans pieces (kmeans.cu) used by the IVF index.
 mann_status kmeans_fit_device(Context* ctx, cudaStream_t s, const float* X, int64_t n, int d, int k,

@@ -1074,9 +1074,11 @@ mann_status run_few(int metric, int grid, const float* base, int64_t n, const fl
 // of k.  One warp per query; lane s walks list s (and s+32, ...).  A balanced
 // walk of the tile kernel (w.per > 0, bq rows per block) wrote only the slots
 // of the CTAs that its query block met.  With o.ids the results are written as
-// finish_kernel writes them, without a launch of its own.
+// finish_kernel writes them, without a launch of its own.  `shared`: several
+// lists may hold the same key (inverted lists with points in common); it counts
+// once.
 __global__ void merge_lists_kernel(const uint64_t* __restrict__ partial, int64_t nq, int slots,
-                                   int k, FewOut o, int64_t tiles, int64_t per, int bq) {
+                                   int k, FewOut o, int64_t tiles, int64_t per, int bq, bool shared) {
   const int lane = threadIdx.x & 31;
   const int64_t q = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (q >= nq) return;
@@ -1098,6 +1100,10 @@ __global__ void merge_lists_kernel(const uint64_t* __restrict__ partial, int64_t
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         if (g + u >= nsplit) break;  // uniform
+        if (shared) {  // entries that B holds already leave the list first
+          const bool twice = wl::contains32(B, v[u], lane);
+          if (__any_sync(FULL, twice)) v[u] = sort32(twice ? KEY_NONE : v[u], lane);
+        }
         B = merge32(B, v[u], lane);
       }
     }
@@ -1135,7 +1141,7 @@ __global__ void merge_lists_kernel(const uint64_t* __restrict__ partial, int64_t
     if (m == KEY_NONE) continue;
 #pragma unroll
     for (int t = 0; t < MAXL; ++t) {
-      if (cur[t] == m) {  // keys are unique (ids differ), so exactly one owner
+      if (cur[t] == m) {  // one owner, or every list that shares the key
         const int s = lane + 32 * t;
         ++head[t];
         cur[t] = head[t] < k ? src[(int64_t)s * k + head[t]] : KEY_NONE;
@@ -1330,11 +1336,11 @@ mann_status launch_seg_rows(const float* data, const int32_t* rows, int cnt, con
 }
 
 mann_status launch_merge_lists(const uint64_t* partial, int64_t nq, int nsplit, int k, uint64_t* out,
-                               cudaStream_t s) {
+                               cudaStream_t s, bool shared) {
   if (nq <= 0) return MANN_OK;
   if (nsplit > 128) return fail(MANN_EINVAL_ARG, "at most 128 lists per query can be merged");
   merge_lists_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, s>>>(partial, nq, nsplit, k, FewOut{out, nullptr, nullptr, 0, -1}, 0,
-                                                               0, 1);
+                                                               0, 1, shared);
   MANN_CHECK_LAUNCH();
   return MANN_OK;
 }
@@ -1391,7 +1397,7 @@ static mann_status fp32_search(Context* ctx, cudaStream_t s, const float* base, 
       return MANN_OK;
     }
     merge_lists_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, s>>>(partial, nq, slots, kk, o, few ? 0 : w.tiles,
-                                                                 few ? 0 : w.per, few ? 1 : k1_rows(nq, kk));
+                                                                 few ? 0 : w.per, few ? 1 : k1_rows(nq, kk), false);
     MANN_CHECK_LAUNCH();
   }
   if (!o.ids) *out_keys = o.keys;
@@ -1475,7 +1481,7 @@ mann_status knn_fp32_keys_on(int num_sms, cudaStream_t s, const float* base, int
   }
   uint64_t* keys = partial + (size_t)nq * nsplit * kk;
   merge_lists_kernel<<<(unsigned)ceil_div(nq, 8), 256, 0, s>>>(partial, nq, nsplit, kk,
-                                                               FewOut{keys, nullptr, nullptr, 0, -1}, 0, 0, 1);
+                                                               FewOut{keys, nullptr, nullptr, 0, -1}, 0, 0, 1, false);
   MANN_CHECK_LAUNCH();
   *out_keys = keys;
   return MANN_OK;

@@ -58,6 +58,17 @@ __device__ __forceinline__ uint64_t sort32(uint64_t c, int lane) {
   return c;
 }
 
+// Whether key (each lane its own, not KEY_NONE) is an entry of the sorted
+// ascending list of 32 keys that the lanes hold in `list`.
+__device__ __forceinline__ bool contains32(uint64_t list, uint64_t key, int lane) {
+  int at = 0;  // the last entry at or below key, or entry 0
+#pragma unroll
+  for (int w = 16; w > 0; w >>= 1)
+    if (__shfl_sync(FULL, (unsigned long long)list, at + w) <= key) at += w;
+  const uint64_t e = __shfl_sync(FULL, (unsigned long long)list, at);
+  return e == key && key != KEY_NONE;
+}
+
 // Sorted ascending lists of 32 keys, one entry per lane: the 32 smallest of both.
 __device__ __forceinline__ uint64_t merge32(uint64_t a, uint64_t b, int lane) {
   const uint64_t r = __shfl_sync(FULL, (unsigned long long)b, 31 - lane);
