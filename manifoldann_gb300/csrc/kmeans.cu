@@ -12,6 +12,7 @@
 // groups the points first -- so a fit is deterministic and matches the
 // oracle's restatement bit for bit from the same initial centroids.
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 #include <vector>
 
@@ -799,6 +800,9 @@ __global__ void bounds_from_top2_kernel(const int32_t* __restrict__ ids, const f
     d1 = __fsqrt_ru(d1);
     d2 = __fsqrt_rd(d2);
   }
+  // a square that overflowed says no more than that the distance is at least
+  // the root of the largest float: that centroid may come near
+  if (d2 == INFINITY) d2 = __fsqrt_rd(FLT_MAX);
   const float rel = dist_rel(d);
   assign[j] = ids[2 * i];
   ub[j] = __fadd_ru(__fmul_ru(d1, __fadd_ru(1.0f, rel)), DIST_ABS);
