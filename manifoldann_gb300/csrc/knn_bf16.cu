@@ -213,7 +213,8 @@ struct ScaleOut {
 __global__ void __launch_bounds__(256)
     scale_probe_kernel(const float* __restrict__ x, int64_t n, int d, int64_t stride, const float* __restrict__ rnorm,
                        ScaleOut o) {
-  __shared__ float wsum[8][NUM_SCALES + 1];
+  __shared__ double wsum[8][NUM_SCALES];
+  __shared__ float wmax[8];
   __shared__ int last, best;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t row = ((int64_t)blockIdx.x * 8 + w) * stride;
@@ -250,18 +251,18 @@ __global__ void __launch_bounds__(256)
   }
   if (lane == 0) {
 #pragma unroll
-    for (int i = 0; i < NUM_SCALES; ++i) wsum[w][i] = cc[i] > 0.0f ? rr[i] / cc[i] : 0.0f;
-    wsum[w][NUM_SCALES] = mx < 3.0e38f ? mx : 0.0f;
+    for (int i = 0; i < NUM_SCALES; ++i) wsum[w][i] = cc[i] > 0.0f ? (double)rr[i] / (double)cc[i] : 0.0;
+    wmax[w] = mx < 3.0e38f ? mx : 0.0f;
   }
   __syncthreads();
   if (threadIdx.x <= NUM_SCALES) {
     if (threadIdx.x < NUM_SCALES) {
       double t = 0.0;
-      for (int i = 0; i < 8; ++i) t += (double)wsum[i][threadIdx.x];
+      for (int i = 0; i < 8; ++i) t += wsum[i][threadIdx.x];
       atomicAdd(&o.score[threadIdx.x], t);
     } else {
       float t = 0.0f;
-      for (int i = 0; i < 8; ++i) t = fmaxf(t, wsum[i][NUM_SCALES]);
+      for (int i = 0; i < 8; ++i) t = fmaxf(t, wmax[i]);
       atomicMax(reinterpret_cast<unsigned*>(&o.score[NUM_SCALES]), __float_as_uint(t));
     }
     __threadfence();
