@@ -453,14 +453,23 @@ __device__ __forceinline__ void k1_body(const float* __restrict__ base, int64_t 
 // How the tile kernel's CTAs share the (query block, point tile) units.
 // Unit u is tile u % tiles of query block u / tiles.
 //   splits == 0: CTA c takes units [c per, (c + 1) per) -- an equal share of
-//     the whole work, whatever the block and tile counts; a query block's
-//     lists go to consecutive slots, one per CTA that touches it.
+//     the whole work, whatever the block and tile counts.  Going from unit to
+//     unit either the CTA or the query block (or both) moves on, so CTA c's
+//     list of query row q is row q + c BQ of `partial`: one list per row and BQ
+//     more per CTA.  (A place in every row for each CTA that may meet its block
+//     was two lists per row: 100,000 rows, k = 128, 201 MB and now 122.  The
+//     search takes as long either way: 20,011 x 20,011 x 100, k = 15, 3,188 and
+//     3,120 us; 10,000 x 60,000 x 256, k = 10, 10.76 and 10.73 ms; 100,000 x
+//     3,000 x 8, k = 128, 10.06 and 9.99 ms.)
 //   splits > 0: CTA c takes split c % splits (tiles_per tiles) of query block
-//     c / splits.
+//     c / splits; its list of row q is list c % splits of the row's `slots`.
 struct K1Walk {
   int64_t total, per;
   int tiles, splits, tiles_per;
-  int slots;  // lists per query row
+  int slots;  // lists per query row (splits == 0: at most)
+  int step;      // lists from a CTA's first to the next one's (splits == 0; 0: one list per row)
+  int stride;    // ... from a row's first to the next row's
+  int64_t rows;  // lists in all
 };
 
 template <int METRIC, int BQ, int KW, bool VEC>
@@ -481,10 +490,11 @@ __global__ void __launch_bounds__(K1_THREADS, k1_ctas<BQ, KW>())
     const int64_t qb = u / w.tiles;
     const int t0 = (int)(u - qb * w.tiles);
     const int t1 = (int)min((int64_t)w.tiles, t0 + (uend - u));
-    const int slot = w.splits > 0 ? (int)(blockIdx.x % w.splits)
-                                  : (int)((int64_t)blockIdx.x - qb * w.tiles / w.per);
+    // (the CTA as the unit's: with blockIdx.x here the compiler schedules the tile
+    // phase differently, 10.73 -> 10.92 ms at 10,000 x 60,000 x 256)
+    const int first = w.splits > 0 ? (int)(blockIdx.x % w.splits) : (int)(u / w.per) * w.step;
     k1_body<METRIC, BQ, KW, VEC>(base, (int64_t)t0 * K1_BN, min(n, (int64_t)t1 * K1_BN), qs, qrows, qb * BQ, nq, d,
-                                 qnorm, bnorm, k, partial + (int64_t)slot * k, (int64_t)w.slots * k, k1_smem);
+                                 qnorm, bnorm, k, partial + (int64_t)first * k, (int64_t)w.stride * k, k1_smem);
     u += t1 - t0;
     __syncthreads();  // the next block's set-up overwrites the lists
   }
@@ -1071,22 +1081,25 @@ mann_status run_few(int metric, int grid, const float* base, int64_t n, const fl
 }
 
 // Merge up to `slots` sorted lists of k keys per query into one sorted list
-// of k.  One warp per query; lane s walks list s (and s+32, ...).  A balanced
-// walk of the tile kernel (w.per > 0, bq rows per block) wrote only the slots
-// of the CTAs that its query block met.  With o.ids the results are written as
-// finish_kernel writes them, without a launch of its own.  `shared`: several
-// lists may hold the same key (inverted lists with points in common); it counts
-// once.
+// of k.  One warp per query; lane s walks list s (and s+32, ...).  After a
+// balanced walk of the tile kernel (per > 0, bq rows per block) a row has one
+// list for every CTA that its query block met, placed as K1Walk says.  With
+// o.ids the results are written as finish_kernel writes them, without a launch
+// of its own.  `shared`: several lists may hold the same key (inverted lists
+// with points in common); it counts once.
 __global__ void merge_lists_kernel(const uint64_t* __restrict__ partial, int64_t nq, int slots,
                                    int k, FewOut o, int64_t tiles, int64_t per, int bq, bool shared) {
   const int lane = threadIdx.x & 31;
   const int64_t q = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (q >= nq) return;
   const uint64_t* src = partial + q * (int64_t)slots * k;
+  int64_t next = k;  // from a list of the row to the next
   int nsplit = slots;
   if (per > 0) {
-    const int64_t qb = q / bq;
-    nsplit = (int)(((qb + 1) * tiles - 1) / per - qb * tiles / per) + 1;
+    const int64_t qb = q / bq, c0 = qb * tiles / per;
+    nsplit = (int)(((qb + 1) * tiles - 1) / per - c0) + 1;
+    src = partial + (q + c0 * bq) * k;
+    next = (int64_t)bq * k;
   }
   // Short lists of few splits, one entry per lane, merge in bitonic steps (about
   // 55 instructions a list); many splits take the head-by-head form below
@@ -1096,7 +1109,7 @@ __global__ void merge_lists_kernel(const uint64_t* __restrict__ partial, int64_t
     for (int g = 1; g < nsplit; g += 4) {
       uint64_t v[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) v[u] = g + u < nsplit && lane < k ? src[(int64_t)(g + u) * k + lane] : KEY_NONE;
+      for (int u = 0; u < 4; ++u) v[u] = g + u < nsplit && lane < k ? src[(g + u) * next + lane] : KEY_NONE;
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         if (g + u >= nsplit) break;  // uniform
@@ -1120,7 +1133,7 @@ __global__ void merge_lists_kernel(const uint64_t* __restrict__ partial, int64_t
   for (int t = 0; t < MAXL; ++t) {
     const int s = lane + 32 * t;
     head[t] = 0;
-    cur[t] = (s < nsplit) ? src[(int64_t)s * k] : KEY_NONE;
+    cur[t] = (s < nsplit) ? src[s * next] : KEY_NONE;
   }
   int found = 0;
   for (int e = 0; e < k; ++e) {
@@ -1144,7 +1157,7 @@ __global__ void merge_lists_kernel(const uint64_t* __restrict__ partial, int64_t
       if (cur[t] == m) {  // one owner, or every list that shares the key
         const int s = lane + 32 * t;
         ++head[t];
-        cur[t] = head[t] < k ? src[(int64_t)s * k + head[t]] : KEY_NONE;
+        cur[t] = head[t] < k ? src[s * next + head[t]] : KEY_NONE;
       }
     }
   }
@@ -1220,10 +1233,15 @@ K1Walk k1_walk(int num_sms, int64_t n, int64_t nq, int k, int splits) {
     w.tiles_per = (int)ceil_div(w.tiles, splits);
     w.splits = (int)ceil_div(w.tiles, w.tiles_per);
     w.slots = w.splits;
+    w.stride = w.slots;
+    w.rows = nq * w.slots;
     return w;
   }
   w.per = std::max(ceil_div(w.total, places), ceil_div(w.tiles, 96));  // at most 97 lists per row
   w.slots = w.per % w.tiles == 0 ? 1 : (w.tiles % w.per == 0 ? (int)(w.tiles / w.per) : (int)((w.tiles - 2) / w.per) + 2);
+  w.step = w.slots > 1 ? bq : 0;
+  w.stride = 1;
+  w.rows = nq + (ceil_div(w.total, w.per) - 1) * w.step;
   return w;
 }
 
@@ -1380,7 +1398,7 @@ static mann_status fp32_search(Context* ctx, cudaStream_t s, const float* base, 
   const int slots = few ? grid : w.slots;
   const bool fused = few && few_fused((int)nq, d, kk, ctx->few_ticket);
   uint64_t* partial = nullptr;
-  MANN_TRY(ctx->scratch_t(slot_partial, (size_t)nq * slots * kk, &partial));
+  MANN_TRY(ctx->scratch_t(slot_partial, (size_t)(few ? nq * slots : w.rows) * kk, &partial));
   if (!o.ids && (fused || slots > 1)) MANN_TRY(ctx->scratch_t(slot_keys, (size_t)nq * kk, &o.keys));
   if (few) {
     ctx->time_begin(s);
