@@ -74,11 +74,12 @@ mann_status fp32_then_resolve(Context* ctx, cudaStream_t s, const float* base, c
                               const uint64_t* fkeys, const float* qn, const float* bn,
                               uint64_t** out_keys, mann_knn_report* rep);
 
-// Rows listed in unres_rows (h_unres, device) re-resolved from their exact
-// FP32 top-min(n, KMAX_FUSED); the rows still unsettled are counted.
+// Rows listed in unres_rows (h_unres, device), whose exact lists held `entries`
+// keys (KMAX_FUSED: they start from certified candidates), re-resolved from their exact FP32 top-min(n, KMAX_FUSED); the rows still
+// unsettled are counted.
 mann_status widen_unresolved(Context* ctx, cudaStream_t s, const float* base, const float* qs,
                              int64_t n, int d, int metric, int kreq, const float* qn,
-                             const float* bn, const int32_t* unres_rows, int64_t h_unres,
+                             const float* bn, const int32_t* unres_rows, int64_t h_unres, int entries,
                              uint64_t* keys_out, int64_t* still_unresolved);
 
 // Plan and scratch-free variant of knn_fp32_keys (caller supplies `words`

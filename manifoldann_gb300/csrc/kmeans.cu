@@ -939,7 +939,10 @@ mann_status kmeans_assign_device(Context* ctx, cudaStream_t s, const float* X, i
   if (!dd) MANN_TRY(ctx->scratch_t(SLOT_KM_DIST, (size_t)n, &dd));
   // a point seldom has more than a few centroids within rounding of its
   // nearest, and every list entry costs insertions in each of the n rows: 8
-  // entries against 33 take 262,144 x 1,024 x 128 from 5.7 to 2.8 ms
+  // entries against 33 take 262,144 x 1,024 x 128 from 5.7 to 2.8 ms (host call
+  // 6.5 -> 3.6).  Points whose nearest centroid is repeated 8 to 32 times take
+  // both scans: 16.5 -> 19.2 ms with 9 of each, where 33 entries in the former
+  // tile kernel took 21.2
   return exact_search_device(ctx, s, &p, C, k, X, n, d, -1, 1, 1, assign, dd, nullptr, 7);
 }
 
