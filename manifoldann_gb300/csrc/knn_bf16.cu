@@ -2129,8 +2129,9 @@ __global__ void __launch_bounds__(32 * RR_WARPS) k2_rerank(RerankArgs a) {
 }
 
 // rows re-run by the FP32 scan: copy their sorted keys into the candidate table
+// (`whole`: kk is the number of points, none lies beyond the list)
 __global__ void k2_scatter_fallback(const uint64_t* __restrict__ keys, const int* __restrict__ rows,
-                                    const int* __restrict__ count, int kk, int L,
+                                    const int* __restrict__ count, int kk, bool whole, int L,
                                     uint64_t* __restrict__ cand, int* __restrict__ cand_count,
                                     float* __restrict__ floor_val) {
   const int cnt = *count;
@@ -2142,7 +2143,7 @@ __global__ void k2_scatter_fallback(const uint64_t* __restrict__ keys, const int
     while (c < kk && keys[(int64_t)i * kk + c] != KEY_NONE) ++c;
     cand_count[q] = c;
     // the kk-th FP32 distance bounds every point outside the list from below
-    floor_val[q] = (c == kk) ? key_dist(keys[(int64_t)i * kk + kk - 1]) : 3.0e38f;
+    floor_val[q] = (c == kk && !whole) ? key_dist(keys[(int64_t)i * kk + kk - 1]) : 3.0e38f;
   }
   }
 }
@@ -2707,8 +2708,9 @@ mann_status launch_resolve(Context* ctx, const float* base, const float* qs, int
 namespace {
 
 // candidate table from an exact FP32 top-kk list: counts and the floor (the
-// kk-th distance bounds every point outside the list from below)
-__global__ void fp32_lists_to_cand_kernel(const uint64_t* __restrict__ keys, int64_t nq, int kk,
+// kk-th distance bounds every point outside the list from below; `whole`: kk is
+// the number of points, none is outside)
+__global__ void fp32_lists_to_cand_kernel(const uint64_t* __restrict__ keys, int64_t nq, int kk, bool whole,
                                           int* __restrict__ cand_count, float* __restrict__ floor_val) {
   const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= nq) return;
@@ -2716,7 +2718,7 @@ __global__ void fp32_lists_to_cand_kernel(const uint64_t* __restrict__ keys, int
   int c = 0;
   while (c < kk && r[c] != KEY_NONE) ++c;
   cand_count[q] = c;
-  floor_val[q] = (c == kk) ? key_dist(r[kk - 1]) : 3.0e38f;
+  floor_val[q] = (c == kk && !whole) ? key_dist(r[kk - 1]) : 3.0e38f;
 }
 
 }  // namespace
@@ -2763,7 +2765,7 @@ mann_status widen_unresolved(Context* ctx, cudaStream_t s, const float* base, co
       uint64_t* fkeys = nullptr;
       MANN_TRY(knn_fp32_keys(ctx, s, base, n, qs, nr, d, metric, kk, rows + r0, qn, bn, &fkeys,
                              SLOT_TIES_PARTIAL, SLOT_TIES_KEYS));
-      fp32_lists_to_cand_kernel<<<(unsigned)ceil_div(nr, 128), 128, 0, s>>>(fkeys, nr, kk, cand_count + r0,
+      fp32_lists_to_cand_kernel<<<(unsigned)ceil_div(nr, 128), 128, 0, s>>>(fkeys, nr, kk, kk >= n, cand_count + r0,
                                                                            floor_val + r0);
       MANN_CHECK_LAUNCH();
       MANN_TRY(launch_resolve(ctx, base, qs, d, metric, nr, kk, kreq, 1, fkeys, cand_count + r0, floor_val + r0,
@@ -2794,7 +2796,7 @@ mann_status fp32_then_resolve(Context* ctx, cudaStream_t s, const float* base, c
   MANN_TRY(ctx->scratch_t(SLOT_OUT_KEYS_BF16, (size_t)nq * kreq, &keys));
   MANN_TRY(ctx->scratch_t(SLOT_TIES_ROWS, (size_t)nq, &unres));
   MANN_CUDA_TRY(cudaMemsetAsync(counters, 0, 64 * sizeof(unsigned long long), s));
-  fp32_lists_to_cand_kernel<<<(unsigned)ceil_div(nq, 128), 128, 0, s>>>(fkeys, nq, kk, cand_count,
+  fp32_lists_to_cand_kernel<<<(unsigned)ceil_div(nq, 128), 128, 0, s>>>(fkeys, nq, kk, kk >= n, cand_count,
                                                                        floor_val);
   MANN_CHECK_LAUNCH();
   MANN_TRY(launch_resolve(ctx, base, qs, d, metric, nq, kk, kreq, 1, fkeys, cand_count, floor_val, keys,
@@ -3559,7 +3561,8 @@ mann_status knn_bf16_keys(Context* ctx, cudaStream_t s, const float* base, int64
     const float* no_norm = nullptr;
     MANN_TRY(knn_fp32_keys(ctx, s, base, n, qs, h_fb, d, metric, kk, fb_rows, cosine ? cos_qn : no_norm,
                            cosine ? cos_bn : no_norm, &fkeys, SLOT_FALLBACK_KEYS, SLOT_MISC2));
-    k2_scatter_fallback<<<h_fb, 64, 0, s>>>(fkeys, fb_rows, fb_count, kk, L, cand, cand_count, floor_val);
+    k2_scatter_fallback<<<h_fb, 64, 0, s>>>(fkeys, fb_rows, fb_count, kk, kk >= n, L, cand, cand_count,
+                                                floor_val);
     MANN_CHECK_LAUNCH();
   }
 
