@@ -98,8 +98,8 @@ enum ScratchSlot : int {
   SLOT_CSR_ROWS,      // host-pointer union graph: row offsets
   SLOT_FP64_ERR,      // maximum FP64 error of the returned distances
   SLOT_TIES_ROWS,     // FP64 ties: rows whose boundary tie reached past the candidates
-  SLOT_TIES_ROWS2,    // FP64 ties: rows still unsettled after the first and the third widening
-  SLOT_TIES_ROWS3,    // FP64 ties: rows still unsettled after the top-64 widening
+  SLOT_TIES_ROWS2,    // FP64 ties: rows still unsettled after the first and the third wider scan
+  SLOT_TIES_ROWS3,    // FP64 ties: rows still unsettled after the second
   SLOT_TIES_PARTIAL,  // FP64 ties: their wider FP32 lists (per split)
   SLOT_TIES_KEYS,     // FP64 ties: their wider FP32 lists (merged)
   SLOT_TIES_CNT,      // FP64 ties: candidate counts of the wider lists

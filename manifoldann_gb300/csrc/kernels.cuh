@@ -75,7 +75,7 @@ mann_status fp32_then_resolve(Context* ctx, cudaStream_t s, const float* base, c
                               uint64_t** out_keys, mann_knn_report* rep);
 
 // Rows listed in unres_rows (h_unres, device), whose exact lists held `entries`
-// keys (KMAX_FUSED: they start from certified candidates), re-resolved from their exact FP32 top-min(n, KMAX_FUSED); the rows still
+// keys (0: they start from certified candidates), re-resolved from their exact FP32 top-min(n, KMAX_FUSED); the rows still
 // unsettled are counted.
 mann_status widen_unresolved(Context* ctx, cudaStream_t s, const float* base, const float* qs,
                              int64_t n, int d, int metric, int kreq, const float* qn,

@@ -2726,27 +2726,26 @@ __global__ void fp32_lists_to_cand_kernel(const uint64_t* __restrict__ keys, int
 // Rows whose boundary tie cluster reached past their candidates (listed in
 // unres_rows, h_unres of them): their exact FP32 top-64, then the FP64
 // near-tie order again, written over those rows of keys_out; rows whose
-// cluster is longer still get their exact top-min(n, KMAX_FUSED).  Exact
-// lists of fewer than kreq + TIE_ENTRIES entries grow to that first: a row's 33
-// nearest cost three quarters of its 64 nearest (60,000 x 64 points, 256
-// centroids of 9 equal ones each: 3.43 -> 2.92 ms for the assignment).  Rows left
-// unsettled after that (a tie cluster longer than the list) are returned in
-// *still_unresolved; they keep the FP32 (distance, id) order.
+// cluster is longer still get their exact top-min(n, KMAX_FUSED).  `entries`:
+// the length of the exact lists they come from (0: certified candidates); a
+// list is only replaced by a longer one.  Exact lists of fewer than kreq +
+// TIE_ENTRIES entries grow to that first: a row's 33 nearest cost three quarters
+// of its 64 nearest (60,000 x 64 points, 256 centroids of 9 equal ones each:
+// 3.43 -> 2.92 ms for the assignment).  Rows left unsettled after that (a tie
+// cluster longer than the list) are returned in *still_unresolved; they keep
+// the FP32 (distance, id) order.
 mann_status widen_unresolved(Context* ctx, cudaStream_t s, const float* base, const float* qs,
                              int64_t n, int d, int metric, int kreq, const float* qn,
                              const float* bn, const int32_t* unres_rows, int64_t h_unres, int entries,
                              uint64_t* keys_out, int64_t* still_unresolved) {
-  *still_unresolved = 0;
+  *still_unresolved = h_unres;
   const int32_t* rows = unres_rows;
-  const int sizes[3] = {std::min(kreq + TIE_ENTRIES, KMAX_FUSED), 64, KMAX_FUSED};
-  int before = 0;
-  for (int stage = entries < sizes[0] ? 0 : 1; stage < 3 && h_unres > 0; ++stage) {
+  const int sizes[3] = {entries > 0 ? std::min(kreq + TIE_ENTRIES, KMAX_FUSED) : 0, 64, KMAX_FUSED};
+  int scans = 0;
+  for (int stage = 0; stage < 3 && h_unres > 0; ++stage) {
     const int kk = (int)std::min<int64_t>(n, sizes[stage]);
-    if (kk <= kreq || kk <= before) {  // every point is already a candidate
-      *still_unresolved = 0;
-      return MANN_OK;
-    }
-    before = kk;
+    if (kk <= std::max(kreq, entries)) continue;
+    entries = kk;
     int* cand_count = nullptr;
     float* floor_val = nullptr;
     unsigned long long* counters = nullptr;
@@ -2754,7 +2753,7 @@ mann_status widen_unresolved(Context* ctx, cudaStream_t s, const float* base, co
     MANN_TRY(ctx->scratch_t(SLOT_TIES_CNT, (size_t)h_unres, &cand_count));
     MANN_TRY(ctx->scratch_t(SLOT_TIES_FLOOR, (size_t)h_unres, &floor_val));
     MANN_TRY(ctx->scratch_t(SLOT_TIES_COUNTERS, 4, &counters));
-    MANN_TRY(ctx->scratch_t(stage == 1 ? SLOT_TIES_ROWS3 : SLOT_TIES_ROWS2, (size_t)h_unres, &next_rows));
+    MANN_TRY(ctx->scratch_t(scans++ & 1 ? SLOT_TIES_ROWS3 : SLOT_TIES_ROWS2, (size_t)h_unres, &next_rows));
     MANN_CUDA_TRY(cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned long long), s));
     // up to a few batches of 32 rows take the few-row scan (one point per thread
     // across the GPU) when the list fits it; more rows, or a wider list, scan
@@ -3580,7 +3579,7 @@ mann_status knn_bf16_keys(Context* ctx, cudaStream_t s, const float* base, int64
     int64_t left = 0;
     if (fp64)
       MANN_TRY(widen_unresolved(ctx, s, base, qs, n, d, metric, kreq, cosine ? cos_qn : nullptr,
-                                cosine ? cos_bn : nullptr, unres, (int64_t)h[5], KMAX_FUSED, keys, &left));
+                                cosine ? cos_bn : nullptr, unres, (int64_t)h[5], 0, keys, &left));
     if (rep) {
       rep->rows_fallback = h_fb;
       rep->candidates = (int64_t)h[2];
