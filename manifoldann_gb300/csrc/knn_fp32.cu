@@ -1113,11 +1113,16 @@ __global__ void merge_lists_kernel(const uint64_t* __restrict__ partial, int64_t
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         if (g + u >= nsplit) break;  // uniform
-        if (shared) {  // entries that B holds already leave the list first
-          const bool twice = wl::contains32(B, v[u], lane);
-          if (__any_sync(FULL, twice)) v[u] = sort32(twice ? KEY_NONE : v[u], lane);
+        uint64_t M = merge32(B, v[u], lane);
+        if (shared) {
+          // equal keys stand side by side: entries that B holds already leave the list first
+          const uint64_t left = __shfl_up_sync(FULL, (unsigned long long)M, 1);
+          if (__any_sync(FULL, lane > 0 && left == M && M != KEY_NONE)) {
+            const bool twice = wl::contains32(B, v[u], lane);
+            M = merge32(B, sort32(twice ? KEY_NONE : v[u], lane), lane);
+          }
         }
-        B = merge32(B, v[u], lane);
+        B = M;
       }
     }
     if (o.ids)
