@@ -249,11 +249,14 @@ __global__ void __launch_bounds__(256)
     }
     mx = fmaxf(mx, __shfl_xor_sync(FULL, mx, s));
   }
-  if (lane == 0) {
+  float r = 0.0f, c = 0.0f;  // lane i: candidate i's
 #pragma unroll
-    for (int i = 0; i < NUM_SCALES; ++i) wsum[w][i] = cc[i] > 0.0f ? (double)rr[i] / (double)cc[i] : 0.0;
-    wmax[w] = mx < 3.0e38f ? mx : 0.0f;
+  for (int i = 0; i < NUM_SCALES; ++i) {
+    r = lane == i ? rr[i] : r;
+    c = lane == i ? cc[i] : c;
   }
+  if (lane < NUM_SCALES) wsum[w][lane] = c > 0.0f ? (double)r / (double)c : 0.0;
+  if (lane == 0) wmax[w] = mx < 3.0e38f ? mx : 0.0f;
   __syncthreads();
   if (threadIdx.x <= NUM_SCALES) {
     if (threadIdx.x < NUM_SCALES) {
