@@ -79,7 +79,10 @@ mann_status search_device_body(Context* ctx, cudaStream_t s, const mann_knn_para
     use_bf16 = true;
   } else if (p->precision == MANN_PREC_AUTO) {
     // between 2,048 and 4,096 points where the search is long enough for the
-    // preparation (10,000 x 2,048 x 256: 506 us in the FP32 form, 264 here)
+    // preparation.  FP32 and tensor-core form at the line's sides, k = 10, call
+    // by call: 1e9 multiply-adds 145 and 202 us (1,302 x 3,000 x 256), 195 and
+    // 248 (3,814 x 2,048 x 128), 189 and 219 (318 x 4,000 x 784); 2e9 259 and
+    // 253, 270 and 201, 259 and 218; 5e9 465 and 196, 501 and 289, 463 and 292
     use_bf16 = kreq <= 24 && d >= 128 && (n >= 4096 || (n >= 2048 && (double)nq * (double)n * d >= 2e9));
   }
   const int form_used = p->precision == MANN_PREC_AUTO ? FORM_AUTO16 : form;

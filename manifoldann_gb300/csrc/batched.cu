@@ -28,9 +28,9 @@
 namespace mann {
 namespace {
 
-__global__ void publish_queue_kernel(SegQueue* q, int count, const int* count_dev, unsigned epoch) {
+__global__ void publish_queue_kernel(SegQueue* q, int count, unsigned epoch) {
   q->head = 0;
-  q->count = count_dev ? *count_dev : count;
+  q->count = count;
   q->status = 0;
   __threadfence();
   q->epoch = epoch;
@@ -106,7 +106,7 @@ mann_status issue(int num_sms, const Shape& sh, const Plan& pl, const Bufs& b, u
                   long long wait_cycles, cudaStream_t s) {
   const int nitems = (int)pl.items.size();
   if (pl.S > 1) MANN_CUDA_TRY(cudaMemsetAsync(b.partial, 0xFF, sizeof(uint64_t) * sh.N * pl.S * sh.kk, s));
-  if (publish) MANN_TRY(launch_publish_queue(b.queue, nitems, nullptr, epoch, s));
+  if (publish) MANN_TRY(launch_publish_queue(b.queue, nitems, epoch, s));
   MANN_TRY(launch_k1_persistent(num_sms, sh.data, b.items, b.queue, epoch, wait_cycles, sh.d, sh.metric, pl.bq,
                                 sh.kk, pl.S, pl.S > 1 ? b.partial : b.keys, s));
   if (pl.S > 1) MANN_TRY(launch_merge_lists(b.partial, sh.N, pl.S, sh.kk, b.keys, s));
@@ -230,8 +230,8 @@ mann_status check_queue(const Bufs& b, cudaStream_t s) {
 
 }  // namespace
 
-mann_status launch_publish_queue(SegQueue* q, int count, const int* count_dev, unsigned epoch, cudaStream_t s) {
-  publish_queue_kernel<<<1, 1, 0, s>>>(q, count, count_dev, epoch);
+mann_status launch_publish_queue(SegQueue* q, int count, unsigned epoch, cudaStream_t s) {
+  publish_queue_kernel<<<1, 1, 0, s>>>(q, count, epoch);
   MANN_CHECK_LAUNCH();
   return MANN_OK;
 }
@@ -284,7 +284,7 @@ mann_status knn_graph_batched_device(Context* ctx, cudaStream_t s, const mann_kn
       // loaded first, on an empty queue: the first launch of a kernel takes about
       // a millisecond, which made two splits (23.6 ms at 338,792 rows x 32) win
       // over none (22.7)
-      MANN_TRY(launch_publish_queue(b.queue, 0, nullptr, ++st.epoch, s));
+      MANN_TRY(launch_publish_queue(b.queue, 0, ++st.epoch, s));
       MANN_TRY(launch_k1_persistent(ctx->num_sms, sh.data, b.items, b.queue, st.epoch, QUEUE_WAIT_CYCLES, sh.d,
                                     sh.metric, pl.bq, sh.kk, pl.S, pl.S > 1 ? b.partial : b.keys, s));
       cudaEventRecord(e0, s);

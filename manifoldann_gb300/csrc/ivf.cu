@@ -9,9 +9,10 @@
 //
 // The scan runs "inverted" like the reference's batched multi-level query
 // (src/indices/multilevel/query.jl:363-396): queries are grouped by the list
-// they probe, the data is gathered into list order once per call, and one
-// CTA scans one list for up to 32 of its queries, every distance in the FP32
-// form's sequential arithmetic, keeping each query's top-k.  Order: (distance,
+// they probe, and one CTA scans one list, or a part of a long one, for up to 16
+// of its queries, the points read in place through the list's ids, every
+// distance in the FP32 form's sequential arithmetic, keeping each query's
+// top-k.  Order: (distance,
 // id); the reference's heap keeps an arbitrary member of an exact tie at the
 // k-th place, this keeps the lower id.
 #include <algorithm>
@@ -50,7 +51,7 @@ __global__ void probe_count_kernel(const int32_t* __restrict__ probes, int64_t n
   if (l >= 0 && l < nlist) atomicAdd(&cnt[l], 1u);
 }
 
-// Exclusive prefix sums of the per-list query counts and of their 32-query
+// Exclusive prefix sums of the per-list query counts and of their qc-query
 // chunks; one block of 1024 threads, each owning a contiguous run of lists.
 __global__ void __launch_bounds__(1024) probe_scan_kernel(const unsigned* __restrict__ cnt, int nlist, int qc,
                                                           int64_t* __restrict__ qoff,
@@ -209,9 +210,14 @@ struct ScanSmem {
 // A warp brings in its 64 rows a 16-dimension slice at a time, four lanes to a
 // row (cp.async), and each thread reads its own rows back from shared memory;
 // the slices are the warp's own, so no block barrier falls inside the
-// arithmetic, and six CTAs per SM cover each other's loads.  What bounds it is shared-memory reads of the
-// queries, one 16-byte broadcast per four queries and dimension: two points
-// per thread halve them.
+// arithmetic (past 128 dimensions two per 128, where the queries are staged
+// anew), and six CTAs per SM cover each other's loads.  A pair of points per
+// thread halves the reads of the queries, one 16-byte broadcast per four queries
+// and dimension.  What bounds it is waiting: at 10,000 queries in 4 of 4,096
+// lists of 1M x 128 (338 us) issue slots are 52 % busy, the FMA pipe 31 %, shared
+// memory 24 % and DRAM 20 %; of the 8 warps waiting per issue 2.7 stand at the
+// barriers around the selection, 1.8 on fixed latencies, 1.5 on shared memory and
+// 1.3 on rows.
 template <int METRIC, int KW, bool VEC>
 __global__ void __launch_bounds__(SCAN_T, 6)
     ivf_scan_kernel(const float* __restrict__ data, const int64_t* __restrict__ loff,
@@ -519,7 +525,10 @@ mann_status ivf_route_device(Context* ctx, cudaStream_t s, const float* centroid
   p.metric = centroid_metric;
   p.k = nprobe;
   // a short search is over in the FP32 form before the tensor-core form's
-  // dozen launches are (100 queries x 4,096 x 128)
+  // dozen launches are.  FP32 and AUTO at the line's sides, 4 probes, call by
+  // call: 5e8 multiply-adds 100 and 174 us (953 queries x 4,096 x 128), 98 and
+  // 183 (476 x 4,096 x 256), 127 and 215 (77 x 8,192 x 784); 1e9 181 and 235,
+  // 142 and 185, 184 and 219; 2e9 262 and 179, 275 and 236, 257 and 220
   p.precision = (double)nq * nlist * d < 1e9 ? MANN_PREC_FP32 : MANN_PREC_AUTO;
   float* dd = nullptr;
   MANN_TRY(ctx->scratch_t(SLOT_IVF_ROUTE_D, (size_t)nq * nprobe, &dd));

@@ -127,8 +127,7 @@ mann_status launch_k1_persistent(int num_sms, const float* data, const SegItem* 
 mann_status launch_seg_rows(const float* data, const int32_t* rows, int cnt, const int64_t* offs, int nsets, int nsplit,
                             int64_t chunk, int d, int metric, uint64_t* partial, cudaStream_t s);
 // Publishes a work queue of `count` items (head 0, status 0, then the epoch).
-// count_dev (optional) supplies the count from device memory instead.
-mann_status launch_publish_queue(SegQueue* q, int count, const int* count_dev, unsigned epoch, cudaStream_t s);
+mann_status launch_publish_queue(SegQueue* q, int count, unsigned epoch, cudaStream_t s);
 mann_status knn_graph_batched_device(Context* ctx, cudaStream_t s, const mann_knn_params* p, const float* data,
                                      const int64_t* offs, int nsets, int d, int include_self, int32_t* ids,
                                      float* dists, mann_knn_report* rep);

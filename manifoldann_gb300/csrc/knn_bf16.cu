@@ -100,7 +100,7 @@ constexpr bool K2_USE_PAIRS = false;
 enum : int { ERR_TIMEOUT_PRODUCER = 1, ERR_TIMEOUT_MMA = 2, ERR_TIMEOUT_EPI = 3 };
 
 struct RowInfo {
-  float nrm;    // ||x~||^2 (FP64 sum rounded to nearest)
+  float nrm;    // ||x~||^2 (an FP32 sum; the certificate is charged with its rounding)
   float xn_up;  // ||x~|| rounded up
   float r_up;   // bound on ||(x - mu) - x~|| (includes the FP32 rounding of x - mu)
   float lo_up;  // split form: ||x_lo|| rounded up (0 otherwise)
@@ -3702,8 +3702,8 @@ void build_seg_tables(const int64_t* offs, int nsets, int ctas, SegTables* T) {
 // the BF16 form: one operand preparation over all rows, one segmented k2_main
 // pass over every (set, 128-row block, 256-point tile) item, the certificate
 // and exact FP32 rerank per row, uncertified rows re-scanned exactly over
-// their own set on the device (work queue published by a kernel, so the host
-// never waits for their count), and the (distance, id) truncation to kreq.
+// their own set (the host reads their count and sizes that launch by it), and
+// the (distance, id) truncation to kreq.
 // Result: keys [N][kreq] with global ids (the row itself included).
 mann_status knn_bf16_batched_keys(Context* ctx, cudaStream_t s, const float* data, const int64_t* offs_host,
                                   const int64_t* offs_dev, int nsets, int d, int metric, int kreq, int margin,

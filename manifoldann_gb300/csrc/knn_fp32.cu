@@ -65,13 +65,10 @@ __global__ void __launch_bounds__(256) row_sqnorm_kernel(const float* __restrict
   if (lane < nr) out[r0 + lane] = s;
 }
 
-// Thread-tile row/column maps.  TQ rows per thread: 8 -> {ty*4+i, 64+ty*4+i},
-// 4 -> ty*4+i, 2 -> ty*2+i.  Eight columns per thread: {tx*4+j, 64+tx*4+j}.
+// Thread-tile row/column maps.  TQ rows per thread, 4 or 2: ty*TQ+i.  Eight columns per thread: {tx*4+j, 64+tx*4+j}.
 template <int TQ>
 __device__ __forceinline__ int tile_row(int ty, int i) {
-  if constexpr (TQ == 8) return (i < 4) ? ty * 4 + i : 64 + ty * 4 + (i - 4);
-  else if constexpr (TQ == 4) return ty * 4 + i;
-  else return ty * 2 + i;
+  return ty * TQ + i;
 }
 __device__ __forceinline__ int tile_col(int tx, int j) {
   return (j < 4) ? tx * 4 + j : 64 + tx * 4 + (j - 4);
@@ -79,12 +76,7 @@ __device__ __forceinline__ int tile_col(int tx, int j) {
 
 template <int TQ>
 __device__ __forceinline__ void load_q_frag(const float* p, int ty, float (&v)[TQ]) {
-  if constexpr (TQ == 8) {
-    float4 a = *reinterpret_cast<const float4*>(p + ty * 4);
-    float4 b = *reinterpret_cast<const float4*>(p + 64 + ty * 4);
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-  } else if constexpr (TQ == 4) {
+  if constexpr (TQ == 4) {
     float4 a = *reinterpret_cast<const float4*>(p + ty * 4);
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
   } else {
@@ -239,9 +231,11 @@ __device__ __forceinline__ void k1_drain_row(uint64_t* __restrict__ list, const 
 // One CTA's work: queries [q0, min(q0 + BQ, nq)) against points [nb0, nb1);
 // the sorted list of query row gq goes to dst + gq * dst_stride.
 //
-// Tile phase: BQ x 128 distances in registers, TQ x 8 per thread, bound by
-// the FP32 pipe (one sub and one fma per dimension and pair, two pairs per
-// f32x2 instruction).  The global loads of the next 16-dimension slice -- of
+// Tile phase: BQ x 128 distances in registers, TQ x 8 per thread, one sub and
+// one fma per dimension and pair, two pairs per f32x2 instruction.  Bound by the
+// FP32 pipe and the reads of its operands from shared memory (20,011 x 100: 25 of
+// the 33.8 T lane-operations/s of that mix; issue slots 57 % busy, shared memory
+// 53 %; per issue 2.1 warps wait for operands, 1.3 for the pipe).  The global loads of the next 16-dimension slice -- of
 // the next tile after a tile's last -- are in flight during the current one.
 //
 // Fold: distances are never staged.  Every distance is compared in its
@@ -1449,7 +1443,11 @@ namespace mann {
 // Plan of the FP32 form for (n, nq, kk) on a device with num_sms SMs, as
 // knn_fp32_keys_on makes it: a few rows (nq <= FEW_Q, kk <= 64) go to the
 // few-row kernel with `*nsplit_out` = its grid of point slices; otherwise the
-// tile kernel with `*nsplit_out` point splits.  `*words_out` = the uint64
+// tile kernel with `*nsplit_out` point splits: one CTA per SM if its blocks had
+// 128 rows, so two of the three that an SM holds with the 64 rows they have (k <=
+// 64).  More splits would fill those places but take more scratch, of which the
+// entry point has a fixed amount: a search that fits must go on fitting.
+// `*words_out` = the uint64
 // words of scratch (per-split lists, then merged lists when there is more
 // than one split).
 void knn_fp32_plan(int num_sms, int64_t n, int64_t nq, int kk, int* nsplit_out,

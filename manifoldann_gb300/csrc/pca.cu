@@ -205,8 +205,9 @@ __global__ void __launch_bounds__(PCA_WARPS * 32)
 // lane fetches its partner's column by shuffles.  No shared memory, no warp
 // barriers.
 //
-// The kernel is bound by issued instructions, ~15 rounds x ~8 sweeps per
-// centre: per round one shuffle and one multiply-add (the pair's inner
+// The kernel is bound by issued instructions (issue slots 69 % busy) and the
+// latencies between them (2.9 of the 5 warps waiting per issue), ~15 rounds x ~8
+// sweeps per centre: per round one shuffle and one multiply-add (the pair's inner
 // product) per dimension, and after a rotation another multiply-add (the
 // column's own norm, which its partner gets by one shuffle instead of summing
 // it again -- the same sum in the same order) and three paired operations per
